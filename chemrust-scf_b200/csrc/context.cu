@@ -14,6 +14,7 @@
 #include "chfsi.h"
 #include "dense.hpp"
 #include "gemm.hpp"
+#include "scratch.hpp"
 #include "gemm_tc.hpp"
 #include "fft_plan.hpp"
 #include "kernels.hpp"
@@ -376,13 +377,20 @@ void digit_reversal(const AxisPlan& P, std::vector<int>& pos) {
 // Test hook (chfsi_test_inject): device allocations left before one fails
 // with cudaErrorMemoryAllocation; negative = no failure planned.
 std::atomic<long long> g_alloc_fail_in{-1};
+std::atomic<int> g_contexts{0};  // live contexts
 
 template <typename T> cudaError_t dalloc(T** p, size_t n) {
     *p = nullptr;
     if (n == 0) return cudaSuccess;
     if (g_alloc_fail_in.load() >= 0 && g_alloc_fail_in.fetch_sub(1) == 0)
         return cudaErrorMemoryAllocation;
-    return cudaMalloc((void**)p, n * sizeof(T));
+    cudaError_t e = cudaMalloc((void**)p, n * sizeof(T));
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        scratch_trim();  // the scratch kept between calls may be what is missing
+        e = cudaMalloc((void**)p, n * sizeof(T));
+    }
+    return e;
 }
 
 // The context stream is non-blocking, so a legacy-stream cudaMemcpy or
@@ -2103,6 +2111,7 @@ chfsi_status chfsi_create(const chfsi_dims* dims, const chfsi_config* cfg, chfsi
             return bail(CHFSI_ERR_CUDA);
     }
     *out = ctx;
+    g_contexts.fetch_add(1);
     return CHFSI_OK;
 }
 
@@ -2112,6 +2121,7 @@ void chfsi_destroy(chfsi_ctx* ctx) {
     if (ctx->st) cudaStreamSynchronize(ctx->st);
     free_all(ctx);
     delete ctx;
+    if (g_contexts.fetch_sub(1) == 1) scratch_trim();
 }
 
 chfsi_status chfsi_set_basis(chfsi_ctx* ctx, const int32_t* miller, const double* kinetic,
@@ -3695,7 +3705,7 @@ constexpr int kGemmMaxK = 1 << 30;
 // leading dimensions lda, ldb; C dense m x n) — the op::C ZGEMM of the
 // reference's BlasHandle::gemm_c64 (src/device/blas.rs:79-102) as used for
 // beta^H psi and the subspace matrices.  Split-K partials go to stream-
-// ordered scratch (cudaMallocAsync / cudaFreeAsync on `stream`).
+// ordered scratch (scratch.hpp).
 extern "C" chfsi_status chfsi_zgemm_cn(const chfsi_c128* a_dev, int lda, const chfsi_c128* b_dev,
                                        int ldb, int m, int n, int k, chfsi_c128* c_dev,
                                        void* stream) {
@@ -3707,12 +3717,12 @@ extern "C" chfsi_status chfsi_zgemm_cn(const chfsi_c128* a_dev, int lda, const c
     cudaStream_t st = (cudaStream_t)stream;
     double2* part = nullptr;
     const size_t pe = splitk_partial_elems(m, n, k);
-    cudaError_t e = cudaMallocAsync((void**)&part, pe * sizeof(double2), st);
-    if (e != cudaSuccess) return cuda_fail(e, "cudaMallocAsync", __FILE__, __LINE__);
+    cudaError_t e = scratch_alloc((void**)&part, pe * sizeof(double2), st);
+    if (e != cudaSuccess) return cuda_fail(e, "scratch_alloc", __FILE__, __LINE__);
     gemm_cn(reinterpret_cast<const double2*>(a_dev), lda, reinterpret_cast<const double2*>(b_dev),
             ldb, m, n, k, part, reinterpret_cast<double2*>(c_dev), st);
     e = cudaGetLastError();
-    cudaFreeAsync(part, st);
+    scratch_free(part, st);
     if (e != cudaSuccess) return cuda_fail(e, "gemm_cn", __FILE__, __LINE__);
     e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_fail(e, "cudaStreamSynchronize", __FILE__, __LINE__);
@@ -3750,8 +3760,8 @@ extern "C" chfsi_status chfsi_zgemm_cn_bf16x3_shape(const chfsi_c128* a_dev, int
     char* buf = nullptr;
     const size_t part_f = tc_partial_floats(m, n, k);
     const size_t bytes = 3 * (na + nbe) * 2 + part_f * 4 + 256;
-    cudaError_t e = cudaMallocAsync((void**)&buf, bytes, st);
-    if (e != cudaSuccess) return cuda_fail(e, "cudaMallocAsync", __FILE__, __LINE__);
+    cudaError_t e = scratch_alloc((void**)&buf, bytes, st);
+    if (e != cudaSuccess) return cuda_fail(e, "scratch_alloc", __FILE__, __LINE__);
     cudaMemsetAsync(buf, 0, 3 * (na + nbe) * 2 + 256, st);
     for (int i = 0; i < 3; ++i) {
         pa.p[i] = buf + (size_t)i * na * 2;
@@ -3764,7 +3774,7 @@ extern "C" chfsi_status chfsi_zgemm_cn_bf16x3_shape(const chfsi_c128* a_dev, int
     e = tc_gemm(pa, pb, m, n, k, kTcOutPartial, c_dev, n, part, err, st, shape);
     int herr = 0;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, st);
-    cudaFreeAsync(buf, st);
+    scratch_free(buf, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_fail(e, "tc_gemm", __FILE__, __LINE__);
     if (herr) {
@@ -3814,8 +3824,8 @@ extern "C" chfsi_status chfsi_hegv_dev(const chfsi_c128* h_dev, const chfsi_c128
     const size_t jac = jacobi_scratch_doubles(n, max_sweeps);
     char* buf = nullptr;
     const size_t bytes = 5 * nn * sizeof(double2) + (jac + n) * sizeof(double) + 64;
-    cudaError_t e = cudaMallocAsync((void**)&buf, bytes, st);
-    if (e != cudaSuccess) return cuda_fail(e, "cudaMallocAsync", __FILE__, __LINE__);
+    cudaError_t e = scratch_alloc((void**)&buf, bytes, st);
+    if (e != cudaSuccess) return cuda_fail(e, "scratch_alloc", __FILE__, __LINE__);
     double2* H = (double2*)buf;
     double2* S = H + nn;
     double2* T1 = S + nn;
@@ -3841,7 +3851,7 @@ extern "C" chfsi_status chfsi_hegv_dev(const chfsi_c128* h_dev, const chfsi_c128
     int fl[4] = {0, 0, 0, 0};
     if (e == cudaSuccess) e = cudaMemcpyAsync(w_host, w, sizeof(double) * n, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(fl, flags, sizeof(fl), cudaMemcpyDeviceToHost, st);
-    cudaFreeAsync(buf, st);
+    scratch_free(buf, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_fail(e, "chfsi_hegv_dev", __FILE__, __LINE__);
     if (fl[0] != 0) {

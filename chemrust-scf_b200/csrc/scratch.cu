@@ -1,0 +1,63 @@
+// One memory pool per device.  The device's default pool returns its memory at
+// every synchronisation, so that a call that allocates, launches and waits paid
+// the mapping of its scratch each time (about 10 us per MB: 420 of the 660 us of
+// a 261 x 77 x 23,847 projection, 1.4 ms of a 1,728 x 576 x 173,925 one); this
+// pool keeps up to kScratchKeep bytes between calls.  Pool allocations are
+// stream-ordered and may be made from any thread.
+#include "scratch.hpp"
+
+#include <mutex>
+
+namespace chfsi {
+
+namespace {
+std::mutex g_pool_mu;
+cudaMemPool_t g_pools[64] = {};
+
+cudaError_t pool_of(int dev, cudaMemPool_t* out) {
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    if (!g_pools[dev]) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.handleTypes = cudaMemHandleTypeNone;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t pool = nullptr;
+        cudaError_t e = cudaMemPoolCreate(&pool, &props);
+        if (e != cudaSuccess) return e;
+        unsigned long long keep = kScratchKeep;
+        e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        if (e != cudaSuccess) {
+            cudaMemPoolDestroy(pool);
+            return e;
+        }
+        g_pools[dev] = pool;
+    }
+    *out = g_pools[dev];
+    return cudaSuccess;
+}
+}  // namespace
+
+cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t st) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= 64) return cudaMallocAsync(p, bytes, st);
+    cudaMemPool_t pool = nullptr;
+    e = pool_of(dev, &pool);
+    if (e != cudaSuccess) return e;
+    return cudaMallocFromPoolAsync(p, bytes, pool, st);
+}
+
+void scratch_free(void* p, cudaStream_t st) {
+    if (p) cudaFreeAsync(p, st);
+}
+
+void scratch_trim() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    if (g_pools[dev]) cudaMemPoolTrimTo(g_pools[dev], 0);
+}
+
+}  // namespace chfsi
