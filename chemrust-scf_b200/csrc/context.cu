@@ -14,6 +14,7 @@
 #include "chfsi.h"
 #include "dense.hpp"
 #include "gemm.hpp"
+#include "gemm_i8.hpp"
 #include "scratch.hpp"
 #include "gemm_tc.hpp"
 #include "fft_plan.hpp"
@@ -511,6 +512,13 @@ struct chfsi_ctx {
     void* d_planes = nullptr;    // all bf16 plane storage
     TcPlanes tp_beta_a, tp_betaT_b, tp_psi_b, tp_small_a;
     float* d_tc_part = nullptr; int* d_tc_err = nullptr;
+    // FP64 products on the INT8 tensor cores: digits of beta for the
+    // projections (rows of beta) and the expansions (rows of beta^T), cut once
+    // per projector set; scratch for the other operands; error word in mapped
+    // host memory, read after each synchronisation
+    I8Operand i8_beta, i8_betaT;
+    void* d_i8_beta = nullptr; void* d_i8 = nullptr; size_t i8_bytes = 0;
+    int* h_i8_err = nullptr;
     bool beta_planes_ready = false;
     // tcgen05 launch shapes of the projection and the expansion (-1: time
     // them at the first mixed filter)
@@ -588,6 +596,90 @@ chfsi_status ensure_pinned(chfsi_ctx* ctx, size_t n) {
     return CHFSI_OK;
 }
 
+// ---------------------------------------------------------------- GEMMs
+// out = conj(A) B^T and O = alpha W^T X + beta O of the FP64 path, on the INT8
+// tensor cores where that is the faster way (i8_cn_pays, i8_tn_pays) and its
+// scratch is there, else on the FP64 tensor path.  pre: digits of A or X.
+void cn_product(chfsi_ctx* ctx, const double2* A, const I8Operand* pre, const double2* B, int M,
+                int N, int K, double2* out, bool herm = false) {
+    const bool cut = pre && pre->ready();
+    if (ctx->d_i8 && i8_cn_pays(M, N, K, herm, cut) &&
+        gemm_cn_i8(A, K, cut ? pre : nullptr, B, K, M, N, K, herm, ctx->d_i8, ctx->i8_bytes, out,
+                   ctx->h_i8_err, ctx->st))
+        return;
+    if (herm) gemm_cn_herm(A, K, B, K, N, K, ctx->d_part, out, ctx->st);
+    else gemm_cn(A, K, B, K, M, N, K, ctx->d_part, out, ctx->st);
+}
+void tn_product(chfsi_ctx* ctx, const double2* W, int ldw, const double2* X, const I8Operand* pre,
+                double2* O, int M, int N, int K, double alpha = 1.0, double beta = 0.0) {
+    const bool cut = pre && pre->ready();
+    if (ctx->d_i8 && i8_tn_pays(M, N, K, cut) &&
+        gemm_tn_i8(W, ldw, X, N, cut ? pre : nullptr, O, N, M, N, K, alpha, beta, ctx->d_i8,
+                   ctx->i8_bytes, ctx->h_i8_err, ctx->st))
+        return;
+    gemm_tn(W, ldw, X, N, O, N, M, N, K, alpha, beta, ctx->st);
+}
+
+// a bounded wait of the INT8 products that ran out (after a synchronisation)
+chfsi_status i8_status(chfsi_ctx* ctx) {
+    if (!ctx->h_i8_err || *(volatile int*)ctx->h_i8_err == 0) return CHFSI_OK;
+    *(volatile int*)ctx->h_i8_err = 0;
+    return ctx->fail(CHFSI_ERR_TIMEOUT, "tensor-core GEMM pipeline wait timed out");
+}
+
+// Scratch for the INT8 products of this context's sizes, at most kI8Scratch
+// bytes (longer products run in groups).  Without it, as when the device is
+// short of memory, the FP64 tensor path computes the same products.
+constexpr size_t kI8Scratch = (size_t)1 << 30;
+void alloc_i8(chfsi_ctx* ctx) {
+    const int nb = ctx->nb + 1, np = ctx->np, npw = ctx->n_pw;
+    size_t need = 0;
+    if (i8_cn_pays(nb, nb, npw, true, false)) need = std::max(need, i8_cn_scratch_bytes(nb, nb, npw, false));
+    if (i8_tn_pays(nb, npw, nb, false)) need = std::max(need, i8_tn_scratch_bytes(nb, npw, nb, false));
+    if (np > 0 && i8_cn_pays(np, nb, npw, false, true))
+        need = std::max(need, i8_cn_scratch_bytes(np, nb, npw, true));
+    if (np > 0 && i8_tn_pays(nb, npw, np, true)) need = std::max(need, i8_tn_scratch_bytes(nb, npw, np, true));
+    if (np > 0 && i8_tn_pays(np, nb, np, false)) need = std::max(need, i8_tn_scratch_bytes(np, nb, np, false));
+    if (need == 0) return;
+    need = std::min(need, kI8Scratch);
+    if (cudaHostAlloc((void**)&ctx->h_i8_err, sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
+        cudaMalloc(&ctx->d_i8, need) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->d_i8 = nullptr;
+        return;
+    }
+    *ctx->h_i8_err = 0;
+    ctx->i8_bytes = need;
+}
+
+// Digits of beta (24 bytes per element and layout beside its 16), where the
+// projector products use them and the memory is there.
+void cut_beta(chfsi_ctx* ctx) {
+    if (ctx->d_i8_beta) cudaFree(ctx->d_i8_beta);
+    ctx->d_i8_beta = nullptr;
+    ctx->i8_beta = ctx->i8_betaT = I8Operand{};
+    const int np = ctx->np, nb = ctx->nb, npw = ctx->n_pw;
+    if (!ctx->d_i8) return;
+    const bool rows = i8_cn_pays(np, nb, npw, false, true), cols = i8_tn_pays(nb, npw, np, true);
+    const int spc = i8_cn_chunk_slabs(np, nb, npw), spcT = (np + 31) / 32;
+    const size_t ba = rows ? i8_operand_bytes(np, kI8RowTile, npw, spc) : 0;
+    const size_t bt = cols ? i8_operand_bytes(npw, kI8RowTile, np, spcT) : 0;
+    if (ba + bt == 0) return;
+    if (cudaMalloc(&ctx->d_i8_beta, ba + bt) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->d_i8_beta = nullptr;
+        return;
+    }
+    if (rows) {
+        i8_operand_place(ctx->i8_beta, ctx->d_i8_beta, np, kI8RowTile, npw, spc);
+        i8_slice(ctx->d_beta, npw, false, -1, ctx->i8_beta, ctx->st);
+    }
+    if (cols) {
+        i8_operand_place(ctx->i8_betaT, (char*)ctx->d_i8_beta + ba, npw, kI8RowTile, np, spcT);
+        i8_slice(ctx->d_beta, npw, true, 1, ctx->i8_betaT, ctx->st);
+    }
+}
+
 // ---------------------------------------------------------------- H|psi>
 // out = epilogue(H psi) for nb bands of psi (ld n_pw, context PW order).
 // Coefficients of one residual (R-ChFSI) step for the kEpiResid epilogue.
@@ -612,14 +704,13 @@ chfsi_status apply_h_dev(chfsi_ctx* ctx, const double2* psi, double2* out, int n
     e.inv_n = 1.0 / (double)ctx->ng;
     if (ctx->np > 0 && with_nl) {
         // C = beta^H psi, C <- D C, nl = beta C  (chebyshev.rs:416-500)
-        gemm_cn(ctx->d_beta, ctx->n_pw, psi, ctx->n_pw, ctx->np, nb, ctx->n_pw, ctx->d_part,
-                ctx->d_cp, ctx->st);
+        cn_product(ctx, ctx->d_beta, &ctx->i8_beta, psi, ctx->np, nb, ctx->n_pw, ctx->d_cp);
         count_launch();
         k_apply_dmat<<<grid_for((size_t)ctx->np * nb), 256, 0, ctx->st>>>(
             ctx->d_cp, ctx->d_cd, ctx->np, nb, ctx->d_proj_ion, ctx->d_poff, ctx->d_doff,
             ctx->d_dmat);
-        gemm_tn(ctx->d_cd, nb, ctx->d_beta, ctx->n_pw, ctx->d_nl, ctx->n_pw, nb, ctx->n_pw,
-                ctx->np, 1.0, 0.0, ctx->st);
+        tn_product(ctx, ctx->d_cd, nb, ctx->d_beta, &ctx->i8_betaT, ctx->d_nl, nb, ctx->n_pw,
+                   ctx->np);
         e.nl = ctx->d_nl;
     }
     launch_zsticks_inverse<double2>(psi, ctx->n_pw, ctx->d_work, nb, ctx->geo, ctx->st);
@@ -641,19 +732,19 @@ chfsi_status apply_h_dev(chfsi_ctx* ctx, const double2* psi, double2* out, int n
 chfsi_status sinv_h_parts(chfsi_ctx* ctx, const double2* x, int ncols, int nout) {
     cudaStream_t st = ctx->st;
     const int np = ctx->np, npw = ctx->n_pw;
-    gemm_cn(ctx->d_beta, npw, x, npw, np, ncols, npw, ctx->d_part, ctx->d_cp, st);
+    cn_product(ctx, ctx->d_beta, &ctx->i8_beta, x, np, ncols, npw, ctx->d_cp);
     count_launch();
     k_apply_dmat<<<grid_for((size_t)np * ncols), 256, 0, st>>>(
         ctx->d_cp, ctx->d_cd, np, ncols, ctx->d_proj_ion, ctx->d_poff, ctx->d_doff, ctx->d_dmat);
     chfsi_status s = apply_h_dev(ctx, x, ctx->d_hpsi, ncols, kEpiApply, nullptr, -1, nullptr,
                                  nullptr, false);
     if (s) return s;
-    gemm_cn(ctx->d_beta, npw, ctx->d_hpsi, npw, np, ncols, npw, ctx->d_part, ctx->d_cp, st);
-    gemm_tn(ctx->d_bmatT, np, ctx->d_cd, ncols, ctx->d_cp, ncols, np, ncols, np, 1.0, 1.0, st);
+    cn_product(ctx, ctx->d_beta, &ctx->i8_beta, ctx->d_hpsi, np, ncols, npw, ctx->d_cp);
+    tn_product(ctx, ctx->d_bmatT, np, ctx->d_cd, nullptr, ctx->d_cp, np, ncols, np, 1.0, 1.0);
     CK(cudaMemcpyAsync(ctx->d_cq, ctx->d_cd, sizeof(double2) * (size_t)np * ncols,
                        cudaMemcpyDeviceToDevice, st));
-    gemm_tn(ctx->d_sinvT, np, ctx->d_cp, ncols, ctx->d_cq, ncols, np, ncols, np, 1.0, -1.0, st);
-    gemm_tn(ctx->d_cq, ncols, ctx->d_beta, npw, ctx->d_sx, npw, nout, npw, np, 1.0, 0.0, st);
+    tn_product(ctx, ctx->d_sinvT, np, ctx->d_cp, nullptr, ctx->d_cq, np, ncols, np, 1.0, -1.0);
+    tn_product(ctx, ctx->d_cq, ncols, ctx->d_beta, &ctx->i8_betaT, ctx->d_sx, nout, npw, np);
     CK(cudaGetLastError());
     return CHFSI_OK;
 }
@@ -678,8 +769,8 @@ chfsi_status apply_op_dev(chfsi_ctx* ctx, const double2* x, double2* out, int nb
         // H v = H_loc v + beta G_v
         CK(cudaMemcpyAsync(ctx->d_lz_f, ctx->d_hpsi + (size_t)nb * ctx->n_pw,
                            sizeof(double2) * ctx->n_pw, cudaMemcpyDeviceToDevice, st));
-        gemm_tn(ctx->d_cd + nb, ncols, ctx->d_beta, ctx->n_pw, ctx->d_lz_f, ctx->n_pw, 1,
-                ctx->n_pw, ctx->np, 1.0, 1.0, st);
+        tn_product(ctx, ctx->d_cd + nb, ncols, ctx->d_beta, &ctx->i8_betaT, ctx->d_lz_f, 1,
+                   ctx->n_pw, ctx->np, 1.0, 1.0);
     }
     const size_t n = (size_t)nb * ctx->n_pw;
     count_launch();
@@ -818,28 +909,27 @@ chfsi_status rr_dev(chfsi_ctx* ctx, bool fp32_block) {
     const bool aug_s = ctx->uspp && np > 0;
     if (nl_sub || aug_s) {
         // C = beta^H psi and its conjugate
-        gemm_cn(ctx->d_beta, ctx->n_pw, ctx->d_psi, ctx->n_pw, np, n, ctx->n_pw, ctx->d_part,
-                ctx->d_cp, st);
+        cn_product(ctx, ctx->d_beta, &ctx->i8_beta, ctx->d_psi, np, n, ctx->n_pw, ctx->d_cp);
         count_launch();
         k_conj<<<grid_for((size_t)np * n), 256, 0, st>>>(ctx->d_cp, ctx->d_cq, (size_t)np * n);
     }
     // psi^H H psi and psi^H psi are Hermitian: upper tiles only
-    gemm_cn_herm(ctx->d_psi, ctx->n_pw, ctx->d_hpsi, ctx->n_pw, n, ctx->n_pw, ctx->d_part, ctx->d_T1, st);
+    cn_product(ctx, ctx->d_psi, nullptr, ctx->d_hpsi, n, n, ctx->n_pw, ctx->d_T1, true);
     if (nl_sub) {
         // H_sub += C^H D C
         count_launch();
         k_apply_dmat<<<grid_for((size_t)np * n), 256, 0, st>>>(
             ctx->d_cp, ctx->d_cd, np, n, ctx->d_proj_ion, ctx->d_poff, ctx->d_doff, ctx->d_dmat);
-        gemm_tn(ctx->d_cq, n, ctx->d_cd, n, ctx->d_T1, n, n, n, np, 1.0, 1.0, st);
+        tn_product(ctx, ctx->d_cq, n, ctx->d_cd, nullptr, ctx->d_T1, n, n, np, 1.0, 1.0);
     }
     symmetrize(ctx->d_T1, ctx->d_H, n, st);
-    gemm_cn_herm(ctx->d_psi, ctx->n_pw, ctx->d_psi, ctx->n_pw, n, ctx->n_pw, ctx->d_part, ctx->d_T1, st);
+    cn_product(ctx, ctx->d_psi, nullptr, ctx->d_psi, n, n, ctx->n_pw, ctx->d_T1, true);
     if (aug_s) {
         // S_sub = psi^H psi + C^H q C
         count_launch();
         k_apply_dmat<<<grid_for((size_t)np * n), 256, 0, st>>>(
             ctx->d_cp, ctx->d_cd, np, n, ctx->d_proj_ion, ctx->d_poff, ctx->d_doff, ctx->d_qmat);
-        gemm_tn(ctx->d_cq, n, ctx->d_cd, n, ctx->d_T1, n, n, n, np, 1.0, 1.0, st);
+        tn_product(ctx, ctx->d_cq, n, ctx->d_cd, nullptr, ctx->d_T1, n, n, np, 1.0, 1.0);
     }
     symmetrize(ctx->d_T1, ctx->d_S, n, st);
     cholesky(ctx->d_S, n, ctx->d_flags + 0, st);                   // S -> L
@@ -850,7 +940,7 @@ chfsi_status rr_dev(chfsi_ctx* ctx, bool fp32_block) {
     CK(jacobi(ctx->d_T2, ctx->d_V, n, ctx->jac_max_sweeps, 1e-26, ctx->d_jac, ctx->d_flags + 2, st));
     sort_eig(ctx->d_T2, ctx->d_V, n, ctx->d_eig, ctx->d_H, st);     // H = U (sorted)
     small_gemm(1, 0, ctx->d_T1, ctx->d_H, ctx->d_T2, n, st);        // T2 = Li^H U
-    gemm_tn(ctx->d_T2, n, ctx->d_psi, ctx->n_pw, ctx->d_psi2, ctx->n_pw, n, ctx->n_pw, n, 1.0, 0.0, st);
+    tn_product(ctx, ctx->d_T2, n, ctx->d_psi, nullptr, ctx->d_psi2, n, ctx->n_pw, n);
     if (fp32_block) {
         // copy back instead of swapping the pointers: a mixed pass captured
         // into a CUDA graph (chfsi_batch_capture) replays on fixed buffers
@@ -1214,17 +1304,17 @@ chfsi_status filter_rchfsi(chfsi_ctx* ctx, int ndeg, const double* eig_dev, int 
     if ((s = apply_h_dev(ctx, ctx->d_psi, ctx->d_rc_hx, nb, kEpiApply, nullptr))) return s;
     if (ctx->uspp) {
         // S X - X = beta q beta^H X, then Y = S^-1 (H X - S X Lam)
-        gemm_cn(ctx->d_beta, npw, ctx->d_psi, npw, np, nb, npw, ctx->d_part, ctx->d_cp, st);
+        cn_product(ctx, ctx->d_beta, &ctx->i8_beta, ctx->d_psi, np, nb, npw, ctx->d_cp);
         count_launch();
         k_apply_dmat<<<grid_for((size_t)np * nb), 256, 0, st>>>(
             ctx->d_cp, ctx->d_cd, np, nb, ctx->d_proj_ion, ctx->d_poff, ctx->d_doff, ctx->d_qmat);
-        gemm_tn(ctx->d_cd, nb, ctx->d_beta, npw, ctx->d_sx, npw, nb, npw, np, 1.0, 0.0, st);
+        tn_product(ctx, ctx->d_cd, nb, ctx->d_beta, &ctx->i8_betaT, ctx->d_sx, nb, npw, np);
         count_launch();
         k_rc_resid<<<grid_for(n), 256, 0, st>>>(ctx->d_rc_hx, ctx->d_psi, ctx->d_sx, eig_dev, npw, n,
                                                 ctx->d_rc_y);
-        gemm_cn(ctx->d_beta, npw, ctx->d_rc_y, npw, np, nb, npw, ctx->d_part, ctx->d_cp, st);
-        gemm_tn(ctx->d_sinvT, np, ctx->d_cp, nb, ctx->d_cq, nb, np, nb, np, 1.0, 0.0, st);
-        gemm_tn(ctx->d_cq, nb, ctx->d_beta, npw, ctx->d_sx, npw, nb, npw, np, 1.0, 0.0, st);
+        cn_product(ctx, ctx->d_beta, &ctx->i8_beta, ctx->d_rc_y, np, nb, npw, ctx->d_cp);
+        tn_product(ctx, ctx->d_sinvT, np, ctx->d_cp, nullptr, ctx->d_cq, np, nb, np);
+        tn_product(ctx, ctx->d_cq, nb, ctx->d_beta, &ctx->i8_betaT, ctx->d_sx, nb, npw, np);
         count_launch();
         k_cheb_combine<double2><<<grid_for(n), 256, 0, st>>>(ctx->d_rc_y, ctx->d_sx, ctx->d_rc_y,
                                                              ctx->d_rc_y, n, ctx->d_coef, 0, nullptr);
@@ -1316,6 +1406,7 @@ chfsi_status finish_diag(chfsi_ctx* ctx, double* eig_out, bool have_rr) {
     if (ctx->d_tc_err)
         CK(cudaMemcpyAsync(&tc_err, ctx->d_tc_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
+    if (chfsi_status e = i8_status(ctx)) return e;
     if (tc_err) {
         CK(cudaMemsetAsync(ctx->d_tc_err, 0, sizeof(int), ctx->st));
         return ctx->fail(CHFSI_ERR_TIMEOUT, "tensor-core GEMM pipeline wait timed out");
@@ -1476,8 +1567,7 @@ chfsi_status density_dev(chfsi_ctx* ctx, double* rho) {
     }
     if (ctx->aug && nocc > 0) {
         // c_I = sum_n f_n C_n^H q C_n with C = beta^H psi
-        gemm_cn(ctx->d_beta, ctx->n_pw, ctx->d_psi, ctx->n_pw, ctx->np, ctx->nb, ctx->n_pw,
-                ctx->d_part, ctx->d_cp, st);
+        cn_product(ctx, ctx->d_beta, &ctx->i8_beta, ctx->d_psi, ctx->np, ctx->nb, ctx->n_pw, ctx->d_cp);
         count_launch();
         k_apply_dmat<<<grid_for((size_t)ctx->np * ctx->nb), 256, 0, st>>>(
             ctx->d_cp, ctx->d_cd, ctx->np, ctx->nb, ctx->d_proj_ion, ctx->d_poff, ctx->d_doff,
@@ -1680,6 +1770,7 @@ chfsi_status alloc_all(chfsi_ctx* ctx) {
     }
     ctx->occ.assign(ctx->nb, 0.0);
     CK(cudaMemsetAsync(ctx->d_occ, 0, sizeof(double) * ctx->nb, ctx->st));
+    alloc_i8(ctx);
     return alloc_density(ctx);
 }
 
@@ -1705,10 +1796,12 @@ void free_all(chfsi_ctx* ctx) {
                   ctx->d_cgv, ctx->d_cgc, ctx->d_cgov, ctx->d_cgpart, ctx->d_cgdot, ctx->d_cgG,
                   ctx->d_psi_save, ctx->d_rc_hx, ctx->d_rc_y, ctx->d_rc_r0, ctx->d_rc_r1,
                   ctx->d_rc_y32, ctx->d_rc_coef, ctx->d_rc_lam, ctx->d_gga, ctx->d_gga_v1,
-                  ctx->d_ion, ctx->d_qvec, ctx->d_atom_of_ion, ctx->d_colidx, ctx->d_bmatT};
+                  ctx->d_ion, ctx->d_qvec, ctx->d_atom_of_ion, ctx->d_colidx, ctx->d_bmatT,
+                  ctx->d_i8, ctx->d_i8_beta};
     for (void* p : mp)
         if (p) cudaFree(p);
     if (ctx->h_pin) cudaFreeHost(ctx->h_pin);
+    if (ctx->h_i8_err) cudaFreeHost(ctx->h_i8_err);
     if (ctx->st) cudaStreamDestroy(ctx->st);
 }
 
@@ -2306,6 +2399,7 @@ chfsi_status chfsi_set_projectors(chfsi_ctx* ctx, const chfsi_c128* beta,
     }
     ctx->proj_set = true;
     ctx->beta_planes_ready = false;
+    cut_beta(ctx);
     return pack_beta_planes(ctx);
 }
 
@@ -2488,7 +2582,7 @@ chfsi_status chfsi_apply_sinv_h(chfsi_ctx* ctx, const chfsi_c128* psi_dev, chfsi
     }
     if (s) return s;
     CK(cudaStreamSynchronize(ctx->st));
-    return CHFSI_OK;
+    return i8_status(ctx);
 }
 
 chfsi_status chfsi_apply_h(chfsi_ctx* ctx, const chfsi_c128* psi_dev, chfsi_c128* hpsi_dev, int nb) {
@@ -2499,7 +2593,7 @@ chfsi_status chfsi_apply_h(chfsi_ctx* ctx, const chfsi_c128* psi_dev, chfsi_c128
                     reinterpret_cast<double2*>(hpsi_dev), nb, kEpiApply, nullptr);
     if (s) return s;
     CK(cudaStreamSynchronize(ctx->st));
-    return CHFSI_OK;
+    return i8_status(ctx);
 }
 
 static chfsi_status upload_eig(chfsi_ctx* ctx, const double* eig_prev, int n_eig,
@@ -2710,7 +2804,7 @@ chfsi_status chfsi_construct_density(chfsi_ctx* ctx, double* rho_out) {
         CK(cudaMemcpyAsync(rho_out, ctx->d_rho_out, sizeof(double) * ctx->fng, cudaMemcpyDeviceToHost, ctx->st));
     }
     CK(cudaStreamSynchronize(ctx->st));
-    return CHFSI_OK;
+    return i8_status(ctx);
 }
 
 chfsi_status chfsi_build_veff(chfsi_ctx* ctx, const double* rho, double* e2) {
@@ -3311,10 +3405,10 @@ extern "C" chfsi_status chfsi_forces(chfsi_ctx* ctx, double* forces) {
             CK(dalloc(&ctx->d_qvec, q.size()));
             CK(copy_sync(ctx->d_qvec, q.data(), sizeof(double) * q.size(), cudaMemcpyHostToDevice, st));
         }
-        gemm_cn(ctx->d_beta, npw, ctx->d_psi, npw, np, nb, npw, ctx->d_part, ctx->d_cp, st);
+        cn_product(ctx, ctx->d_beta, &ctx->i8_beta, ctx->d_psi, np, nb, npw, ctx->d_cp);
         for (int a = 0; a < 3; ++a) {
             launch_scale_pw(ctx->d_psi, ctx->d_qvec + (size_t)a * npw, npw, nb, ctx->d_hpsi, st);
-            gemm_cn(ctx->d_beta, npw, ctx->d_hpsi, npw, np, nb, npw, ctx->d_part, ctx->d_cd, st);
+            cn_product(ctx, ctx->d_beta, &ctx->i8_beta, ctx->d_hpsi, np, nb, npw, ctx->d_cd);
             launch_force_nl(ctx->d_cp, ctx->d_cd, nb, ctx->d_occ, ctx->d_poff, ctx->d_doff,
                             ctx->d_dmat, ctx->nions, a, ctx->d_atom_of_ion, d_f, st);
         }
@@ -3322,6 +3416,7 @@ extern "C" chfsi_status chfsi_forces(chfsi_ctx* ctx, double* forces) {
     CK(cudaGetLastError());
     std::vector<double> f(3 * (size_t)na);
     CK(copy_sync(f.data(), d_f, sizeof(double) * f.size(), cudaMemcpyDeviceToHost, st));
+    if (chfsi_status e = i8_status(ctx)) return e;
     // ion-ion part
     double lat[9];
     for (int i = 0; i < 9; ++i) lat[i] = ctx->lattice[i];
@@ -3701,6 +3796,33 @@ extern "C" chfsi_status chfsi_mixer_samples(chfsi_ctx* ctx, const double* rho_in
 // Largest K of the GEMM entry points: the split-K chunk arithmetic is 32-bit.
 constexpr int kGemmMaxK = 1 << 30;
 
+// Runs an INT8-path product with scratch of its own on `st` and waits for it.
+// *done stays false, with nothing launched, where the scratch is not to be had
+// or too small: the caller then takes the FP64 tensor path.
+template <typename F>
+static chfsi_status with_i8_scratch(size_t want, cudaStream_t st, bool* done, F&& product) {
+    const size_t bytes = std::min(want, kScratchKeep - 256);
+    char* buf = nullptr;
+    if (scratch_alloc((void**)&buf, bytes + 256, st) != cudaSuccess) {
+        cudaGetLastError();
+        return CHFSI_OK;
+    }
+    int* err = (int*)(buf + bytes);
+    int herr = 0;
+    cudaError_t e = cudaMemsetAsync(err, 0, sizeof(int), st);
+    if (e == cudaSuccess) *done = product(buf, bytes, err);
+    if (*done) e = cudaGetLastError();
+    if (*done && e == cudaSuccess) e = cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, st);
+    scratch_free(buf, st);
+    if (*done && e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return cuda_fail(e, "INT8-path product", __FILE__, __LINE__);
+    if (herr) {
+        g_last_error = "tensor-core GEMM pipeline wait timed out";
+        return CHFSI_ERR_TIMEOUT;
+    }
+    return CHFSI_OK;
+}
+
 // C[m][n] = sum_k conj(A[m][k]) B[n][k] on device pointers (row-major,
 // leading dimensions lda, ldb; C dense m x n) — the op::C ZGEMM of the
 // reference's BlasHandle::gemm_c64 (src/device/blas.rs:79-102) as used for
@@ -3715,12 +3837,21 @@ extern "C" chfsi_status chfsi_zgemm_cn(const chfsi_c128* a_dev, int lda, const c
         return CHFSI_ERR_BAD_INPUT;
     }
     cudaStream_t st = (cudaStream_t)stream;
+    const double2* a = reinterpret_cast<const double2*>(a_dev);
+    const double2* b = reinterpret_cast<const double2*>(b_dev);
+    double2* c = reinterpret_cast<double2*>(c_dev);
+    if (i8_cn_pays(m, n, k, false, false)) {
+        bool done = false;
+        chfsi_status s = with_i8_scratch(i8_cn_scratch_bytes(m, n, k, false), st, &done,
+                                         [&](void* buf, size_t bytes, int* err) {
+            return gemm_cn_i8(a, lda, nullptr, b, ldb, m, n, k, false, buf, bytes, c, err, st);
+        });
+        if (s || done) return s;
+    }
     double2* part = nullptr;
-    const size_t pe = splitk_partial_elems(m, n, k);
-    cudaError_t e = scratch_alloc((void**)&part, pe * sizeof(double2), st);
+    cudaError_t e = scratch_alloc((void**)&part, splitk_partial_elems(m, n, k) * sizeof(double2), st);
     if (e != cudaSuccess) return cuda_fail(e, "scratch_alloc", __FILE__, __LINE__);
-    gemm_cn(reinterpret_cast<const double2*>(a_dev), lda, reinterpret_cast<const double2*>(b_dev),
-            ldb, m, n, k, part, reinterpret_cast<double2*>(c_dev), st);
+    gemm_cn(a, lda, b, ldb, m, n, k, part, c, st);
     e = cudaGetLastError();
     scratch_free(part, st);
     if (e != cudaSuccess) return cuda_fail(e, "gemm_cn", __FILE__, __LINE__);
@@ -3796,8 +3927,18 @@ extern "C" chfsi_status chfsi_zgemm_tn(const chfsi_c128* w_dev, int ldw, const c
         return CHFSI_ERR_BAD_INPUT;
     }
     cudaStream_t st = (cudaStream_t)stream;
-    gemm_tn(reinterpret_cast<const double2*>(w_dev), ldw, reinterpret_cast<const double2*>(x_dev),
-            ldx, reinterpret_cast<double2*>(o_dev), ldo, m, n, k, alpha, beta, st);
+    const double2* w = reinterpret_cast<const double2*>(w_dev);
+    const double2* x = reinterpret_cast<const double2*>(x_dev);
+    double2* o = reinterpret_cast<double2*>(o_dev);
+    if (i8_tn_pays(m, n, k, false)) {
+        bool done = false;
+        chfsi_status s = with_i8_scratch(i8_tn_scratch_bytes(m, n, k, false), st, &done,
+                                         [&](void* buf, size_t bytes, int* err) {
+            return gemm_tn_i8(w, ldw, x, ldx, nullptr, o, ldo, m, n, k, alpha, beta, buf, bytes, err, st);
+        });
+        if (s || done) return s;
+    }
+    gemm_tn(w, ldw, x, ldx, o, ldo, m, n, k, alpha, beta, st);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_fail(e, "gemm_tn", __FILE__, __LINE__);

@@ -11,7 +11,8 @@
 //             -> beta (D beta^H psi), psi V
 //
 // B200 FP64 has no tcgen05 kind; both run on the FP64 tensor path
-// (mma.sync m8n8k4 .f64).
+// (mma.sync m8n8k4 .f64): the sizes below i8_cn_pays / i8_tn_pays, and callers
+// without scratch for the INT8 digits (gemm_i8.cu).
 #include <algorithm>
 #include "gemm.hpp"
 #include "launch_count.hpp"

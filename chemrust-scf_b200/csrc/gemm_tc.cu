@@ -30,6 +30,7 @@
 // TMEM and returns, so the context stays usable and the host reads the error.
 #include "gemm_tc.hpp"
 #include "launch_count.hpp"
+#include "tcgen05.cuh"
 
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -54,55 +55,10 @@ template <int SK> struct TcStage {
     static constexpr int stages = SK == 32 ? 3 : 2;
 };
 constexpr int kThreads = 128;
-// hard cap on polls of one wait, whatever the clock says
-constexpr long long kSpinLimit = 1LL << 30;
-// time limit of one wait in normal operation (a whole GEMM takes milliseconds)
-constexpr unsigned long long kWaitNs = 4000000000ULL;
 // time limit while a test has switched the producer's loads off
 constexpr unsigned long long kInjectedWaitNs = 20000000ULL;
 
 std::atomic<int> g_inject_no_loads{0};
-
-__device__ __forceinline__ unsigned long long global_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-    return (uint32_t)__cvta_generic_to_shared(p);
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
-                 "r"(bytes)
-                 : "memory");
-}
-
-// Parity wait bounded by wait_ns of device time (and kSpinLimit polls);
-// returns false on timeout.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
-                                          unsigned long long wait_ns) {
-    const uint32_t a = smem_u32(bar);
-    const unsigned long long t0 = global_ns();
-    for (long long i = 0; i < kSpinLimit; ++i) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(a), "r"(parity)
-            : "memory");
-        if (ok) return true;
-        if ((i & 63) == 63 && global_ns() - t0 > wait_ns) return false;
-    }
-    return false;
-}
 
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, uint64_t* bar,
                                             int x, int y) {
@@ -140,12 +96,6 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t a, uint64_t 
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
         "l"(a), "l"(b), "r"(idesc), "r"(accumulate));
-}
-
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                     smem_u32(bar))
-                 : "memory");
 }
 
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
