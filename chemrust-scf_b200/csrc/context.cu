@@ -898,6 +898,40 @@ chfsi_status filter_dev(chfsi_ctx* ctx, int ndeg, const double* eig_dev, int n_e
 }
 
 // ---------------------------------------------------------------- Rayleigh-Ritz
+// B = Li H Li^H, B U = U diag(w), T2 = Li^H U for n x n matrices; H and S are
+// overwritten, V is scratch.  Past kSmallGemm rows the three products run on
+// the FP64 tensor path (576: 200 us together against 575), below it the plain
+// tiles start faster (160: 14 us each against 24); they take conj(Li) in S:
+//   gemm_cn(Li, H) = conj(Li H),  gemm_cn(conj Li, that) = Li H Li^H.
+constexpr int kSmallGemm = 256;
+cudaError_t subspace_ritz(const double2* Li, double2* H, double2* T2, double2* S, double2* V, double* w,
+                          int n, double* scratch, int max_sweeps, int* sweeps, double2* part,
+                          cudaStream_t st) {
+    const bool big = n > kSmallGemm;
+    if (big) {
+        count_launch();
+        k_conj<<<grid_for((size_t)n * n), 256, 0, st>>>(Li, S, (size_t)n * n);
+        gemm_cn(Li, n, H, n, n, n, n, part, T2, st);
+        gemm_cn(S, n, T2, n, n, n, n, part, H, st);
+    } else {
+        small_gemm(0, 0, Li, H, T2, n, st);
+        small_gemm(0, 1, T2, Li, H, n, st);
+    }
+    symmetrize(H, T2, n, st);
+    cudaError_t e;
+    if (heev_fits(n)) {
+        e = heev(T2, n, w, H, scratch, sweeps, st);  // H = U
+    } else {
+        e = jacobi(T2, V, n, max_sweeps, 1e-26, scratch, sweeps, st);
+        if (e == cudaSuccess) sort_eig(T2, V, n, w, H, st);
+    }
+    if (e != cudaSuccess) return e;
+    if (big) gemm_tn(S, n, H, n, T2, n, n, n, n, 1.0, 0.0, st);
+    else small_gemm(1, 0, Li, H, T2, n, st);
+    return cudaGetLastError();
+}
+size_t subspace_part_elems(int n) { return n > kSmallGemm ? splitk_partial_elems(n, n, n) : 0; }
+
 // fp32_block: the block comes from the FP32 filter, whose d_hpsi holds the
 // local part only; the non-local part enters the subspace matrix as C^H D C
 // (C = beta^H psi, shared with the ultrasoft overlap), which is how the
@@ -932,14 +966,9 @@ chfsi_status rr_dev(chfsi_ctx* ctx, bool fp32_block) {
         tn_product(ctx, ctx->d_cq, n, ctx->d_cd, nullptr, ctx->d_T1, n, n, np, 1.0, 1.0);
     }
     symmetrize(ctx->d_T1, ctx->d_S, n, st);
-    cholesky(ctx->d_S, n, ctx->d_flags + 0, st);                   // S -> L
-    tri_inv(ctx->d_S, ctx->d_T1, n, st);                            // T1 = L^-1
-    small_gemm(0, 0, ctx->d_T1, ctx->d_H, ctx->d_T2, n, st);        // T2 = Li H
-    small_gemm(0, 1, ctx->d_T2, ctx->d_T1, ctx->d_H, n, st);        // H = Li H Li^H
-    symmetrize(ctx->d_H, ctx->d_T2, n, st);                         // T2 = B
-    CK(jacobi(ctx->d_T2, ctx->d_V, n, ctx->jac_max_sweeps, 1e-26, ctx->d_jac, ctx->d_flags + 2, st));
-    sort_eig(ctx->d_T2, ctx->d_V, n, ctx->d_eig, ctx->d_H, st);     // H = U (sorted)
-    small_gemm(1, 0, ctx->d_T1, ctx->d_H, ctx->d_T2, n, st);        // T2 = Li^H U
+    CK(chol_inv(ctx->d_S, ctx->d_T1, n, ctx->d_flags + 0, st));     // T1 = L^-1
+    CK(subspace_ritz(ctx->d_T1, ctx->d_H, ctx->d_T2, ctx->d_S, ctx->d_V, ctx->d_eig, n, ctx->d_jac,
+                     ctx->jac_max_sweeps, ctx->d_flags + 2, ctx->d_part, st));  // T2 = Li^H U
     tn_product(ctx, ctx->d_T2, n, ctx->d_psi, nullptr, ctx->d_psi2, n, ctx->n_pw, n);
     if (fp32_block) {
         // copy back instead of swapping the pointers: a mixed pass captured
@@ -1730,7 +1759,8 @@ chfsi_status alloc_all(chfsi_ctx* ctx) {
     CK(dalloc(&ctx->d_H, nn)); CK(dalloc(&ctx->d_S, nn)); CK(dalloc(&ctx->d_T1, nn));
     CK(dalloc(&ctx->d_T2, nn)); CK(dalloc(&ctx->d_V, nn));
     CK(dalloc(&ctx->d_eig, ctx->nb)); CK(dalloc(&ctx->d_eig_prev, ctx->nb));
-    CK(dalloc(&ctx->d_jac, jacobi_scratch_doubles(ctx->nb, ctx->jac_max_sweeps)));
+    CK(dalloc(&ctx->d_jac, heev_fits(ctx->nb) ? heev_scratch_doubles(ctx->nb)
+                                              : jacobi_scratch_doubles(ctx->nb, ctx->jac_max_sweeps)));
     CK(dalloc(&ctx->d_flags, 8));
     CK(cudaMemsetAsync(ctx->d_flags, 0, 8 * sizeof(int), ctx->st));
     CK(dalloc(&ctx->d_coef, 8));
@@ -1746,6 +1776,7 @@ chfsi_status alloc_all(chfsi_ctx* ctx) {
     // (any band count 1..nb may reach the projector GEMM through chfsi_apply_h)
     size_t pe = std::max(splitk_partial_elems(ctx->nb, ctx->nb, ctx->n_pw),
                          splitk_partial_elems_herm(ctx->nb, ctx->n_pw));
+    pe = std::max(pe, subspace_part_elems(ctx->nb));
     if (ctx->np > 0)
         for (int n = 1; n <= nbx; ++n)
             pe = std::max(pe, splitk_partial_elems(ctx->np, n, ctx->n_pw));
@@ -3962,33 +3993,27 @@ extern "C" chfsi_status chfsi_hegv_dev(const chfsi_c128* h_dev, const chfsi_c128
     cudaStream_t st = (cudaStream_t)stream;
     const size_t nn = (size_t)n * n;
     const int max_sweeps = 60;
-    const size_t jac = jacobi_scratch_doubles(n, max_sweeps);
+    const size_t jac = heev_fits(n) ? heev_scratch_doubles(n) : jacobi_scratch_doubles(n, max_sweeps);
     char* buf = nullptr;
-    const size_t bytes = 5 * nn * sizeof(double2) + (jac + n) * sizeof(double) + 64;
+    const size_t pe = subspace_part_elems(n);
+    const size_t bytes = (4 * nn + pe) * sizeof(double2) + (jac + n) * sizeof(double) + 64;
     cudaError_t e = scratch_alloc((void**)&buf, bytes, st);
     if (e != cudaSuccess) return cuda_fail(e, "scratch_alloc", __FILE__, __LINE__);
     double2* H = (double2*)buf;
     double2* S = H + nn;
     double2* T1 = S + nn;
-    double2* T2 = T1 + nn;
-    double2* V = T2 + nn;
-    double* w = (double*)(V + nn);
+    double2* V = T1 + nn;
+    double2* part = V + nn;
+    double* w = (double*)(part + pe);
     double* js = w + n;
     int* flags = (int*)(js + jac);
     cudaMemsetAsync(flags, 0, 4 * sizeof(int), st);
     symmetrize(reinterpret_cast<const double2*>(h_dev), H, n, st);
     symmetrize(reinterpret_cast<const double2*>(s_dev), S, n, st);
-    cholesky(S, n, flags + 0, st);
-    tri_inv(S, T1, n, st);                       // T1 = L^-1
-    small_gemm(0, 0, T1, H, T2, n, st);          // T2 = L^-1 H
-    small_gemm(0, 1, T2, T1, H, n, st);          // H = L^-1 H L^-H
-    symmetrize(H, T2, n, st);
-    e = jacobi(T2, V, n, max_sweeps, 1e-26, js, flags + 2, st);
-    if (e == cudaSuccess) {
-        sort_eig(T2, V, n, w, H, st);            // H = U (sorted)
-        small_gemm(1, 0, T1, H, reinterpret_cast<double2*>(v_dev), n, st);  // V = L^-H U
-        e = cudaGetLastError();
-    }
+    e = chol_inv(S, T1, n, flags + 0, st);       // T1 = L^-1
+    if (e == cudaSuccess)                        // v = L^-H U
+        e = subspace_ritz(T1, H, reinterpret_cast<double2*>(v_dev), S, V, w, n, js, max_sweeps,
+                          flags + 2, part, st);
     int fl[4] = {0, 0, 0, 0};
     if (e == cudaSuccess) e = cudaMemcpyAsync(w_host, w, sizeof(double) * n, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(fl, flags, sizeof(fl), cudaMemcpyDeviceToHost, st);

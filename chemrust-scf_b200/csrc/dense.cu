@@ -4,21 +4,18 @@
 //
 // Rayleigh-Ritz follows the Cholesky reduction of the reference's CPU
 // path (src/eigensolver/subspace_diag.rs:229-391):
-//   S = L L^H (right-looking Cholesky, info = failing column as ZPOTRF),
-//   Li = L^-1, B = Li H Li^H (Hermitian-symmetrised),
-//   B U = U diag(w) by parallel cyclic Jacobi (cooperative launch,
-//   round-robin pair ordering, rows then columns per step),
+//   S = L L^H (info = failing column as ZPOTRF), Li = L^-1,
+//   B = Li H Li^H (Hermitian-symmetrised), B U = U diag(w),
 //   V = Li^H U; psi <- psi V (caller).
-// It replaces cuSOLVER ZHEGVD itype 1 (src/device/solver.rs:47-95).
+// It replaces cuSOLVER ZHEGVD itype 1 (src/device/solver.rs:47-95).  The factor
+// and the eigensolver are in heev.cu; a parallel cyclic Jacobi (round-robin pair
+// ordering, one cooperative launch) serves the sizes past those of heev().
 #include "dense.hpp"
 #include "launch_count.hpp"
 
 #include <cooperative_groups.h>
 
 namespace cg = cooperative_groups;
-
-// V row entries one lane keeps in registers in k_jacobi_cluster (n <= 32 x this)
-constexpr int kJacClusterMaxPerLane = 8;
 
 namespace chfsi {
 
@@ -50,110 +47,6 @@ __global__ void k_symmetrize(const double2* __restrict__ in, double2* __restrict
         const int i = (int)(t / n), j = (int)(t % n);
         const double2 a = in[(size_t)i * n + j], b = in[(size_t)j * n + i];
         out[t] = make_double2(0.5 * (a.x + b.x), 0.5 * (a.y - b.y));
-    }
-}
-
-// Right-looking Cholesky of a Hermitian positive-definite matrix in place
-// (lower triangle = L, upper zeroed).  info = 0 or the failing column + 1.
-// A pivot fails when it is not above n * 2^-52 times its column's original
-// diagonal entry: such a matrix is singular to working precision (e.g. two
-// equal columns, whose pivot is a rounding residue of either sign) and its
-// factor would only amplify rounding.  The original diagonal is kept in row
-// 0 of the upper triangle, which the factorisation does not touch.
-__global__ void __launch_bounds__(1024) k_cholesky(double2* A, int n, int* info) {
-    __shared__ double ljj;
-    __shared__ int fail;
-    if (threadIdx.x == 0) fail = 0;
-    for (int j = 1 + threadIdx.x; j < n; j += blockDim.x) A[j].x = A[(size_t)j * n + j].x;
-    __syncthreads();
-    const double rel = (double)n * 2.220446049250313e-16;
-    for (int j = 0; j < n; ++j) {
-        if (threadIdx.x == 0) {
-            const double d = A[(size_t)j * n + j].x;
-            const double d0 = j == 0 ? d : A[j].x;
-            if (!(d > 0.0) || !(d > rel * d0)) { fail = j + 1; }
-            else {
-                ljj = sqrt(d);
-                A[(size_t)j * n + j] = make_double2(ljj, 0.0);
-            }
-        }
-        __syncthreads();
-        if (fail) break;
-        const double inv = 1.0 / ljj;
-        for (int i = j + 1 + threadIdx.x; i < n; i += blockDim.x) {
-            double2& a = A[(size_t)i * n + j];
-            a = make_double2(a.x * inv, a.y * inv);
-        }
-        __syncthreads();
-        // trailing update of the lower triangle: A[i][k] -= L[i][j] conj(L[k][j]),
-        // j < k <= i; one warp per row, lanes along the row
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-        for (int i = j + 1 + warp; i < n; i += nw) {
-            const double2 lij = A[(size_t)i * n + j];
-            for (int k = j + 1 + lane; k <= i; k += 32) {
-                const double2 lkj = A[(size_t)k * n + j];
-                double2& a = A[(size_t)i * n + k];
-                a.x -= lij.x * lkj.x + lij.y * lkj.y;
-                a.y -= lij.y * lkj.x - lij.x * lkj.y;
-            }
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) *info = fail;
-    if (fail) return;
-    for (size_t t = threadIdx.x; t < (size_t)n * n; t += blockDim.x) {
-        const int i = (int)(t / n), k = (int)(t % n);
-        if (k > i) A[t] = make_double2(0.0, 0.0);
-    }
-}
-
-// X = L^-1 by forward substitution, one column per thread.
-// X = L^-1 by forward substitution, one warp per column c: row i of the
-// column needs sum_{c <= k < i} L[i][k] X[k][c] (lanes along k, the column
-// kept in shared memory), then X[i][c] = (delta_ic - sum) / L[i][i].
-__global__ void __launch_bounds__(256)
-k_tri_inv_w(const double2* __restrict__ L, double2* __restrict__ X, int n) {
-    extern __shared__ double2 tri_cols[];  // 8 warps x n
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int c = blockIdx.x * 8 + wib;
-    if (c >= n) return;  // whole warps only; no block barrier below
-    double2* xc = tri_cols + (size_t)wib * n;
-    for (int i = lane; i < c; i += 32) X[(size_t)i * n + c] = make_double2(0.0, 0.0);
-    for (int i = c; i < n; ++i) {
-        const double2* Li = L + (size_t)i * n;
-        double sr = 0.0, si = 0.0;
-        for (int k = c + lane; k < i; k += 32) {
-            const double2 l = Li[k], x = xc[k];
-            sr += l.x * x.x - l.y * x.y;
-            si += l.x * x.y + l.y * x.x;
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-            sr += __shfl_xor_sync(0xffffffffu, sr, o);
-            si += __shfl_xor_sync(0xffffffffu, si, o);
-        }
-        const double d = Li[i].x;  // real diagonal
-        const double2 v = make_double2(((i == c ? 1.0 : 0.0) - sr) / d, -si / d);
-        if (lane == 0) {
-            xc[i] = v;
-            X[(size_t)i * n + c] = v;
-        }
-        __syncwarp();
-    }
-}
-
-__global__ void k_tri_inv(const double2* __restrict__ L, double2* __restrict__ X, int n) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= n) return;
-    for (int i = 0; i < c; ++i) X[(size_t)i * n + c] = make_double2(0.0, 0.0);
-    for (int i = c; i < n; ++i) {
-        double2 s = make_double2(i == c ? 1.0 : 0.0, 0.0);
-        for (int k = c; k < i; ++k) {
-            const double2 l = L[(size_t)i * n + k], x = X[(size_t)k * n + c];
-            s.x -= l.x * x.x - l.y * x.y;
-            s.y -= l.x * x.y + l.y * x.x;
-        }
-        const double2 d = L[(size_t)i * n + i];  // real diagonal
-        X[(size_t)i * n + c] = make_double2(s.x / d.x, s.y / d.x);
     }
 }
 
@@ -344,364 +237,6 @@ k_jacobi2(double2* A, double2* V, double2* X, int n, int max_sweeps, double tol2
         converged = scratch[1 + sweep] <= tol2 * total;
     }
     if (gtid == 0) *sweeps_out = converged ? sweep : max_sweeps;
-}
-
-// Same rotation sequence as k_jacobi2 with the working rows kept on chip.
-// Warp w owns pair w at every step: the two A rows of that pair live in its
-// shared memory (phase 2 of step s builds exactly the rows the warp rotates
-// in phase 1 of step s + 1), and V rows 2w, 2w + 1 stay in shared memory for
-// the whole solve (V <- V G only mixes columns).  Per step the only global
-// traffic is the X rows of each pair and the rotation parameters: phase 1
-// writes them, one grid barrier, phase 2 reads them back.  Each pair has two
-// warps: the A warp rotates, writes the X rows and rebuilds the next pair's A
-// rows; the V warp updates the pair's two V rows in the same phase.
-// Requires every pair to have its resident warps (the host checks
-// co-residency).  Shared memory per pair (double2): A rows [2n], X staging
-// [2n], V rows [2n], V ping-pong [2n].
-__global__ void __launch_bounds__(512)
-k_jacobi3(double2* __restrict__ A, double2* __restrict__ V, double2* __restrict__ X, int n,
-          int max_sweeps, double tol2, double* scratch, double* rot, int* sweeps_out) {
-    cg::grid_group grid = cg::this_grid();
-    extern __shared__ double2 jsm[];
-    __shared__ double red[32];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, wpb = blockDim.x >> 6;
-    const int role = wib / wpb, pw = wib - role * wpb;
-    const int gw = blockIdx.x * wpb + pw;
-    const int m = n + (n & 1), npairs = m / 2, nsteps = m - 1;
-    double* rs_s = reinterpret_cast<double*>(jsm);  // 4 * npairs doubles
-    double2* wbase = jsm + 2 * (size_t)npairs + (size_t)pw * 8 * n;
-    double2* sA = wbase;          // rows p, q of this pair
-    double2* sX = wbase + 2 * n;  // staging for the X rows of the next pair
-    double2* sV = wbase + 4 * n;  // V rows 2w, 2w + 1 (ping-pong with sT)
-    double2* sT = wbase + 6 * n;
-    const bool activeA = gw < npairs && role == 0;
-    const bool activeV = gw < npairs && role == 1;
-    const int r0 = 2 * gw, r1 = 2 * gw + 1;
-    const size_t nn = (size_t)n * n;
-    const size_t gtid = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    const size_t gstride = (size_t)gridDim.x * blockDim.x;
-    double tot = 0.0;
-    for (size_t t = gtid; t < nn; t += gstride) tot += A[t].x * A[t].x + A[t].y * A[t].y;
-    tot = block_sum(tot, red);
-    if (threadIdx.x == 0) atomicAdd(&scratch[0], tot);
-    int p = 0, q = 0;
-    if (activeA) {
-        jac_pair(m, 0, gw, p, q);
-        for (int k = lane; k < n; k += 32) {
-            sA[k] = A[(size_t)p * n + k];
-            sA[n + k] = q < n ? A[(size_t)q * n + k] : make_double2(0.0, 0.0);
-        }
-    }
-    if (activeV) {
-        for (int k = lane; k < n; k += 32) {
-            sV[k] = make_double2(k == r0 ? 1.0 : 0.0, 0.0);
-            sV[n + k] = make_double2(k == r1 ? 1.0 : 0.0, 0.0);
-        }
-    }
-    grid.sync();
-    const double total = scratch[0];
-    int sweep = 0;
-    bool converged = false;
-    for (; sweep < max_sweeps && !converged; ++sweep) {
-        for (int s = 0; s < nsteps; ++s) {
-            double* rs = rot + 4 * (size_t)npairs * (s & 1);
-            // ---- phase 1: rotation of this warp's pair from its rows on chip
-            if (activeA) {
-                jac_pair(m, s, gw, p, q);
-                double c = 1.0, sn = 0.0, phr = 1.0, phi = 0.0;
-                if (q < n) {
-                    const double2 apq = sA[q];
-                    const double app = sA[p].x, aqq = sA[n + q].x;
-                    const double bm = hypot(apq.x, apq.y);
-                    if (bm > 1e-300 && bm > 1e-18 * sqrt(fabs(app * aqq))) {
-                        phr = apq.x / bm;
-                        phi = apq.y / bm;
-                        const double tau = (aqq - app) / (2.0 * bm);
-                        const double t = (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
-                        c = 1.0 / sqrt(1.0 + t * t);
-                        sn = t * c;
-                    }
-                    for (int k = lane; k < n; k += 32) {
-                        const double2 apk = sA[k], aqk = sA[n + k];
-                        const double2 pa = make_double2(phr * aqk.x - phi * aqk.y, phr * aqk.y + phi * aqk.x);
-                        X[(size_t)p * n + k] = make_double2(c * apk.x - sn * pa.x, c * apk.y - sn * pa.y);
-                        X[(size_t)q * n + k] = make_double2(sn * apk.x + c * pa.x, sn * apk.y + c * pa.y);
-                    }
-                } else {
-                    for (int k = lane; k < n; k += 32) X[(size_t)p * n + k] = sA[k];
-                }
-                if (lane == 0) {
-                    rs[4 * gw + 0] = c; rs[4 * gw + 1] = sn; rs[4 * gw + 2] = phr; rs[4 * gw + 3] = phi;
-                }
-            }
-            grid.sync();
-            // ---- phase 2: rows of the next pair, A[r] = X[r] G(s); V <- V G(s)
-            const int s2 = (s + 1) % nsteps;
-            int p2 = 0, q2 = 0;
-            if (activeA) {
-                jac_pair(m, s2, gw, p2, q2);
-                for (int k = lane; k < n; k += 32) {
-                    sX[k] = X[(size_t)p2 * n + k];
-                    if (q2 < n) sX[n + k] = X[(size_t)q2 * n + k];
-                }
-            }
-            for (int i = threadIdx.x; i < 4 * npairs; i += blockDim.x) rs_s[i] = rs[i];
-            __syncthreads();
-            if (activeA || activeV) {
-                auto mix = [&](const double2* src, int k) -> double2 {
-                    int pi, partner;
-                    jac_partner(m, s, k, pi, partner);
-                    const double2 xk = src[k];
-                    if (partner >= n) return xk;
-                    const double c = rs_s[4 * pi + 0], sn = rs_s[4 * pi + 1];
-                    const double phr = rs_s[4 * pi + 2], phi = rs_s[4 * pi + 3];
-                    const double2 xp = src[partner];
-                    if (k < partner) {
-                        const double2 qc = make_double2(phr * xp.x + phi * xp.y, phr * xp.y - phi * xp.x);
-                        return make_double2(c * xk.x - sn * qc.x, c * xk.y - sn * qc.y);
-                    }
-                    const double2 qc = make_double2(phr * xk.x + phi * xk.y, phr * xk.y - phi * xk.x);
-                    return make_double2(sn * xp.x + c * qc.x, sn * xp.y + c * qc.y);
-                };
-                __syncwarp();
-                if (activeA) {
-                    for (int k = lane; k < n; k += 32) {
-                        sA[k] = mix(sX, k);
-                        if (q2 < n) sA[n + k] = mix(sX + n, k);
-                    }
-                } else {
-                    for (int k = lane; k < n; k += 32) {
-                        if (r0 < n) sT[k] = mix(sV, k);
-                        if (r1 < n) sT[n + k] = mix(sV + n, k);
-                    }
-                    double2* t = sV; sV = sT; sT = t;
-                }
-                __syncwarp();
-            }
-        }
-        // off-diagonal norm of this warp's rows (the pair of step 0)
-        double off = 0.0;
-        if (activeA) {
-            jac_pair(m, 0, gw, p, q);
-            for (int k = lane; k < n; k += 32) {
-                if (k != p) off += sA[k].x * sA[k].x + sA[k].y * sA[k].y;
-                if (q < n && k != q) off += sA[n + k].x * sA[n + k].x + sA[n + k].y * sA[n + k].y;
-            }
-        }
-        off = block_sum(off, red);
-        if (threadIdx.x == 0) atomicAdd(&scratch[1 + sweep], off);
-        grid.sync();
-        converged = scratch[1 + sweep] <= tol2 * total;
-    }
-    if (activeA) {
-        jac_pair(m, 0, gw, p, q);
-        for (int k = lane; k < n; k += 32) {
-            A[(size_t)p * n + k] = sA[k];
-            if (q < n) A[(size_t)q * n + k] = sA[n + k];
-        }
-    }
-    if (activeV) {
-        for (int k = lane; k < n; k += 32) {
-            if (r0 < n) V[(size_t)r0 * n + k] = sV[k];
-            if (r1 < n) V[(size_t)r1 * n + k] = sV[n + k];
-        }
-    }
-    if (gtid == 0) *sweeps_out = converged ? sweep : max_sweeps;
-}
-
-// The k_jacobi3 rotation sequence inside one thread-block cluster, for the
-// sizes whose rows fit the cluster's shared memory: the X rows of a pair go
-// straight into the shared memory of the warp that owns them at the next step
-// (distributed shared memory), the rotation parameters are broadcast to
-// every block of the cluster, and one cluster barrier per step replaces the
-// grid barrier and the global round trip.  Staging rows and parameters are
-// double-buffered by step parity, so a block that runs ahead into step s + 1
-// never overwrites what a slower block still reads in step s.
-// Each pair has two warps: one rotates the pair and rebuilds its A rows, the
-// other updates its two V rows in the same phase.
-// Shared layout (double2): params [2][2 * npairs] | per pair: A rows [2n],
-// V rows [2n], staging [2][2n].
-__global__ void __launch_bounds__(512)
-k_jacobi_cluster(double2* __restrict__ A, double2* __restrict__ V, int n, int max_sweeps,
-                 double tol2, double* scratch, int* sweeps_out) {
-    cg::cluster_group cluster = cg::this_cluster();
-    extern __shared__ double2 csm[];
-    __shared__ double red[32];
-    // two warps per pair: role 0 rotates and rebuilds the pair's A rows, role 1
-    // updates the pair's two V rows in the same phase
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, wpb = blockDim.x >> 6;
-    const int role = wib / wpb, pw = wib - role * wpb;
-    const int crank = (int)cluster.block_rank();
-    const int gw = crank * wpb + pw;
-    const int m = n + (n & 1), npairs = m / 2, nsteps = m - 1;
-    double* prm = reinterpret_cast<double*>(csm);  // [2][4 * npairs]
-    double2* wbase = csm + 4 * (size_t)npairs + (size_t)pw * 8 * n;
-    double2* sA = wbase;
-    double2* sV = wbase + 2 * n;
-    double2* stg = wbase + 4 * n;  // [2][2n]
-    const bool activeA = gw < npairs && role == 0;
-    const bool activeV = gw < npairs && role == 1;
-    const int r0 = 2 * gw, r1 = 2 * gw + 1;
-    // total |A|^2
-    double tot = 0.0;
-    const size_t nn = (size_t)n * n;
-    for (size_t t = crank * (size_t)blockDim.x + threadIdx.x; t < nn;
-         t += (size_t)cluster.num_blocks() * blockDim.x)
-        tot += A[t].x * A[t].x + A[t].y * A[t].y;
-    tot = block_sum(tot, red);
-    if (threadIdx.x == 0) atomicAdd(&scratch[0], tot);
-    int p = 0, q = 0;
-    if (activeA) {
-        jac_pair(m, 0, gw, p, q);
-        for (int k = lane; k < n; k += 32) {
-            sA[k] = A[(size_t)p * n + k];
-            sA[n + k] = q < n ? A[(size_t)q * n + k] : make_double2(0.0, 0.0);
-        }
-    }
-    if (activeV) {
-        for (int k = lane; k < n; k += 32) {
-            sV[k] = make_double2(k == r0 ? 1.0 : 0.0, 0.0);
-            sV[n + k] = make_double2(k == r1 ? 1.0 : 0.0, 0.0);
-        }
-    }
-    __threadfence();
-    cluster.sync();
-    const double total = *(volatile double*)&scratch[0];
-    int sweep = 0;
-    bool converged = false;
-    for (; sweep < max_sweeps && !converged; ++sweep) {
-        for (int s = 0; s < nsteps; ++s) {
-            const int par = s & 1;
-            const int s2 = (s + 1) % nsteps;
-            // ---- phase 1: rotate this warp's pair, send X rows to their next owners
-            if (activeA) {
-                jac_pair(m, s, gw, p, q);
-                double c = 1.0, sn = 0.0, phr = 1.0, phi = 0.0;
-                if (q < n) {
-                    const double2 apq = sA[q];
-                    const double app = sA[p].x, aqq = sA[n + q].x;
-                    const double bm = hypot(apq.x, apq.y);
-                    if (bm > 1e-300 && bm > 1e-18 * sqrt(fabs(app * aqq))) {
-                        phr = apq.x / bm;
-                        phi = apq.y / bm;
-                        const double tau = (aqq - app) / (2.0 * bm);
-                        const double t = (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
-                        c = 1.0 / sqrt(1.0 + t * t);
-                        sn = t * c;
-                    }
-                }
-                // destinations: the owners of rows p and q at step s + 1
-                double2* dst[2] = {nullptr, nullptr};
-                const int rows[2] = {p, q};
-                for (int h = 0; h < 2; ++h) {
-                    const int r = rows[h];
-                    if (r >= n) continue;
-                    int pi, partner;
-                    jac_partner(m, s2, r, pi, partner);
-                    const int owner_rank = pi / wpb, owner_w = pi % wpb;
-                    const int slot = r < partner ? 0 : 1;
-                    double2* local = csm + 4 * (size_t)npairs + (size_t)owner_w * 8 * n + 4 * n +
-                                     (size_t)par * 2 * n + (size_t)slot * n;
-                    dst[h] = cluster.map_shared_rank(local, owner_rank);
-                }
-                for (int k = lane; k < n; k += 32) {
-                    const double2 apk = sA[k];
-                    if (q < n) {
-                        const double2 aqk = sA[n + k];
-                        const double2 pa = make_double2(phr * aqk.x - phi * aqk.y, phr * aqk.y + phi * aqk.x);
-                        dst[0][k] = make_double2(c * apk.x - sn * pa.x, c * apk.y - sn * pa.y);
-                        dst[1][k] = make_double2(sn * apk.x + c * pa.x, sn * apk.y + c * pa.y);
-                    } else {
-                        dst[0][k] = apk;
-                    }
-                }
-                // broadcast the rotation to every block of the cluster
-                for (int b = lane; b < (int)cluster.num_blocks(); b += 32) {
-                    double* rp = cluster.map_shared_rank(prm + (size_t)par * 4 * npairs + 4 * gw, b);
-                    rp[0] = c; rp[1] = sn; rp[2] = phr; rp[3] = phi;
-                }
-            }
-            cluster.sync();
-            // ---- phase 2: rows of the next pair, A[r] = X[r] G(s); V <- V G(s)
-            if (activeA || activeV) {
-                const double* rs = prm + (size_t)par * 4 * npairs;
-                const double2* sT = stg + (size_t)par * 2 * n;
-                int p2, q2;
-                jac_pair(m, s2, gw, p2, q2);
-                auto mix = [&](const double2* src, int k) -> double2 {
-                    int pi, partner;
-                    jac_partner(m, s, k, pi, partner);
-                    const double2 xk = src[k];
-                    if (partner >= n) return xk;
-                    const double c = rs[4 * pi + 0], sn = rs[4 * pi + 1];
-                    const double phr = rs[4 * pi + 2], phi = rs[4 * pi + 3];
-                    const double2 xp = src[partner];
-                    if (k < partner) {
-                        const double2 qc = make_double2(phr * xp.x + phi * xp.y, phr * xp.y - phi * xp.x);
-                        return make_double2(c * xk.x - sn * qc.x, c * xk.y - sn * qc.y);
-                    }
-                    const double2 qc = make_double2(phr * xk.x + phi * xk.y, phr * xk.y - phi * xk.x);
-                    return make_double2(sn * xp.x + c * qc.x, sn * xp.y + c * qc.y);
-                };
-                if (activeA) {
-                    for (int k = lane; k < n; k += 32) {
-                        sA[k] = mix(sT, k);
-                        if (q2 < n) sA[n + k] = mix(sT + n, k);
-                    }
-                } else {
-                    // V rows in place through registers (n <= 32 * kJacClusterMaxPerLane)
-                    double2 v0[kJacClusterMaxPerLane], v1[kJacClusterMaxPerLane];
-#pragma unroll
-                    for (int j = 0; j < kJacClusterMaxPerLane; ++j) {
-                        const int k = lane + 32 * j;
-                        if (k < n) {
-                            v0[j] = mix(sV, k);
-                            v1[j] = mix(sV + n, k);
-                        }
-                    }
-                    __syncwarp();
-#pragma unroll
-                    for (int j = 0; j < kJacClusterMaxPerLane; ++j) {
-                        const int k = lane + 32 * j;
-                        if (k < n) {
-                            if (r0 < n) sV[k] = v0[j];
-                            if (r1 < n) sV[n + k] = v1[j];
-                        }
-                    }
-                }
-                __syncwarp();
-            }
-        }
-        double off = 0.0;
-        if (activeA) {
-            jac_pair(m, 0, gw, p, q);
-            for (int k = lane; k < n; k += 32) {
-                if (k != p) off += sA[k].x * sA[k].x + sA[k].y * sA[k].y;
-                if (q < n && k != q) off += sA[n + k].x * sA[n + k].x + sA[n + k].y * sA[n + k].y;
-            }
-        }
-        off = block_sum(off, red);
-        if (threadIdx.x == 0) atomicAdd(&scratch[1 + sweep], off);
-        __threadfence();
-        cluster.sync();
-        converged = *(volatile double*)&scratch[1 + sweep] <= tol2 * total;
-    }
-    if (activeA) {
-        jac_pair(m, 0, gw, p, q);
-        for (int k = lane; k < n; k += 32) {
-            A[(size_t)p * n + k] = sA[k];
-            if (q < n) A[(size_t)q * n + k] = sA[n + k];
-        }
-    }
-    if (activeV) {
-        for (int k = lane; k < n; k += 32) {
-            if (r0 < n) V[(size_t)r0 * n + k] = sV[k];
-            if (r1 < n) V[(size_t)r1 * n + k] = sV[n + k];
-        }
-    }
-    if (crank == 0 && threadIdx.x == 0) *sweeps_out = converged ? sweep : max_sweeps;
-    // no block may leave while others can still write into its shared memory
-    cluster.sync();
 }
 
 // Sort eigenvalues ascending (stable by index) and permute eigenvector columns.
@@ -928,21 +463,6 @@ void symmetrize(const double2* in, double2* out, int n, cudaStream_t st) {
     count_launch();
     k_symmetrize<<<grid_for((size_t)n * n), 256, 0, st>>>(in, out, n);
 }
-void cholesky(double2* A, int n, int* info, cudaStream_t st) {
-    count_launch();
-    k_cholesky<<<1, 1024, 0, st>>>(A, n, info);
-}
-void tri_inv(const double2* L, double2* X, int n, cudaStream_t st) {
-    count_launch();
-    const size_t sm = (size_t)8 * n * sizeof(double2);
-    if (sm <= 200 * 1024) {
-        if (sm > 48 * 1024)
-            cudaFuncSetAttribute(k_tri_inv_w, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        k_tri_inv_w<<<(n + 7) / 8, 256, sm, st>>>(L, X, n);
-    } else {
-        k_tri_inv<<<(n + 63) / 64, 64, 0, st>>>(L, X, n);
-    }
-}
 void small_gemm(int opa, int opb, const double2* A, const double2* B, double2* C, int n,
                 cudaStream_t st) {
     count_launch();
@@ -964,52 +484,9 @@ cudaError_t jacobi(double2* A, double2* V, int n, int max_sweeps, double tol2, d
     double* rot = scratch + 1 + max_sweeps;
     double2* X = (double2*)(rot + 8 * (size_t)(npairs + 1));
     if (((uintptr_t)X) & 15) X = (double2*)(((uintptr_t)X + 15) & ~(uintptr_t)15);
-    // one thread-block cluster when its shared memory holds every pair's rows
-    if (n <= 32 * kJacClusterMaxPerLane) {
-        const int wpb = std::max(1, std::min(8, (npairs + 15) / 16));
-        const int nc = (npairs + wpb - 1) / wpb;
-        const size_t smc = (size_t)npairs * 8 * sizeof(double) + (size_t)wpb * 8 * n * sizeof(double2);
-        if (nc <= 16 && smc <= 200 * 1024) {
-            cudaFuncSetAttribute(k_jacobi_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smc);
-            if (nc > 8) cudaFuncSetAttribute(k_jacobi_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-            cudaLaunchConfig_t lc = {};
-            lc.gridDim = dim3(nc);
-            lc.blockDim = dim3(64 * wpb);  // two warps per pair
-            lc.dynamicSmemBytes = smc;
-            lc.stream = st;
-            cudaLaunchAttribute at[1];
-            at[0].id = cudaLaunchAttributeClusterDimension;
-            at[0].val.clusterDim.x = nc;
-            at[0].val.clusterDim.y = 1;
-            at[0].val.clusterDim.z = 1;
-            lc.attrs = at;
-            lc.numAttrs = 1;
-            int clusters = 0;
-            if (cudaOccupancyMaxActiveClusters(&clusters, k_jacobi_cluster, &lc) == cudaSuccess &&
-                clusters >= 1) {
-                cudaError_t e = cudaLaunchKernelEx(&lc, k_jacobi_cluster, A, V, n, max_sweeps, tol2,
-                                                   scratch, sweeps_out);
-                if (e == cudaSuccess) return e;
-            }
-            cudaGetLastError();  // clear a refused configuration; fall through
-        }
-    }
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    // on-chip variant: one warp per pair, all warps co-resident
-    for (int wpb = 8; wpb >= 1; wpb >>= 1) {  // pairs per block, two warps each
-        const size_t smem3 = (size_t)npairs * 4 * sizeof(double) + (size_t)wpb * 8 * n * sizeof(double2);
-        if (smem3 > 200 * 1024) continue;
-        cudaFuncSetAttribute(k_jacobi3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem3);
-        int per_sm3 = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm3, k_jacobi3, 64 * wpb, smem3);
-        const int blocks3 = (npairs + wpb - 1) / wpb;
-        if (per_sm3 < 1 || blocks3 > sms * per_sm3) continue;
-        void* args3[] = {&A, &V, &X, &n, &max_sweeps, &tol2, &scratch, &rot, &sweeps_out};
-        return cudaLaunchCooperativeKernel((const void*)k_jacobi3, dim3(blocks3), dim3(64 * wpb),
-                                           args3, smem3, st);
-    }
     const int warps_per_block = 8;
     int blocks = (npairs + warps_per_block - 1) / warps_per_block;
     const size_t smem = (size_t)warps_per_block * n * sizeof(double2);

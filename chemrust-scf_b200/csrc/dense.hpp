@@ -9,10 +9,18 @@ namespace chfsi {
 constexpr int kPulayMax = 8;
 
 void symmetrize(const double2* in, double2* out, int n, cudaStream_t st);
-void cholesky(double2* A, int n, int* info, cudaStream_t st);
-void tri_inv(const double2* L, double2* X, int n, cudaStream_t st);
+// X = L^-1 of S = L L^H (heev.cu); A: S, overwritten.  info: 0 or failing column + 1
+cudaError_t chol_inv(double2* A, double2* X, int n, int* info, cudaStream_t st);
+// A = U diag(w) U^H, w ascending, U row-major with the eigenvectors as columns
+// (heev.cu), for the sizes heev_fits() says; A is kept.  sweeps_out: Jacobi
+// sweeps of the leaf problems (huge when A is not finite)
+bool heev_fits(int n);
+size_t heev_scratch_doubles(int n);
+cudaError_t heev(const double2* A, int n, double* w, double2* U, double* scratch, int* sweeps_out,
+                 cudaStream_t st);
 void small_gemm(int opa, int opb, const double2* A, const double2* B, double2* C, int n,
                 cudaStream_t st);
+// the sizes past heev_fits()
 size_t jacobi_scratch_doubles(int n, int max_sweeps);
 cudaError_t jacobi(double2* A, double2* V, int n, int max_sweeps, double tol2, double* scratch,
                    int* sweeps_out, cudaStream_t st);
