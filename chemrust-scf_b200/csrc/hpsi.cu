@@ -167,34 +167,9 @@ __device__ __forceinline__ void p2_line_forward(C* line, bool act, int i, int es
 }
 
 // ---------------------------------------------------------------- pass 1
-// z lines of a block of columns transformed by one lane group per line with
-// the compile-time two-radix plan (R0 > 0) or by the generic engine
-template <int R0, int R1, bool FWD, typename C>
-__device__ __forceinline__ void zlines_fft(C* lines, int nl, const HGeom& g, const C* tw) {
-    if constexpr (R0 > 0) {
-        constexpr int T = R0 > R1 ? R0 : R1, PW = 32 / T;
-        const int lane = threadIdx.x & 31, gi = lane / T, li = lane - gi * T;
-        const bool ing = gi < PW;
-        const int groups = (blockDim.x >> 5) * PW, gid = (threadIdx.x >> 5) * PW + gi;
-        for (int l0 = 0; l0 < nl; l0 += groups) {
-            const int l = l0 + gid;
-            const bool act = ing && l < nl;
-            C* line = lines + (act ? l * g.lsz : 0);
-            if (FWD) p2_line_forward<R0, R1, false>(line, act, li, 1, tw);
-            else p2_line_inverse<R0, R1, false>(line, act, li, 1, tw);
-        }
-        __syncthreads();
-    } else {
-        fft_lines_grouped<FWD>(lines, nl, LinesStrided{g.lsz}, 1, g.az, tw);
-    }
-}
-
-// 3 resident blocks per SM with the compile-time plans (their registers
-// allow it), 1 guaranteed with the generic engine
-template <int R0> struct ZCfg { static constexpr int min_blocks = R0 > 0 ? 3 : 1; };
-
-template <typename C, int kColsPerBlock, int R0, int R1>
-__global__ void __launch_bounds__(256, ZCfg<R0>::min_blocks)
+// z lines of a block of columns, generic plans (one lane group per line)
+template <typename C, int kColsPerBlock>
+__global__ void __launch_bounds__(256)
 k_zsticks_inverse(const C* __restrict__ psi, int ldp, C* __restrict__ work, HGeom g) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C* tw = reinterpret_cast<C*>(smem_raw);
@@ -211,11 +186,67 @@ k_zsticks_inverse(const C* __restrict__ psi, int ldp, C* __restrict__ work, HGeo
     for (int q = g0 + threadIdx.x; q < g1; q += blockDim.x)
         lines[(g.pw_col[q] - c0) * g.lsz + swz(g.pw_zpos[q], g.nz)] = pb[q];
     __syncthreads();
-    zlines_fft<R0, R1, false>(lines, nl, g, tw);
+    fft_lines_grouped<false>(lines, nl, LinesStrided{g.lsz}, 1, g.az, tw);
     C* wb = work + (size_t)b * g.nz * g.ncol;
     for (int u = threadIdx.x; u < g.nz * kColsPerBlock; u += blockDim.x) {
         const int z = u / kColsPerBlock, cl = u - z * kColsPerBlock;
         if (cl < nl) wb[(size_t)z * g.ncol + c0 + cl] = lines[cl * g.lsz + swz(z, g.nz)];
+    }
+}
+
+// Two-radix plans: 32 columns per block, a lane per column and a warp per
+// butterfly of the stage (R0 warps with blocks, R1 with spans), lines stored
+// [position][column].  The work array is [z][column] as well, so the stage that
+// meets it moves between registers and global memory in 512-byte rows without a
+// pass through shared memory; a butterfly's twiddles are the same for the whole
+// warp, and every shared access is one row.  The column is XORed with the low
+// bits of the position's block, which spreads the plane waves of one column
+// (consecutive frequencies, a block apart) over the banks for the scatter and the
+// gather.  Against lane groups along each line (which spent 81 % of the
+// shared-memory wavefronts, 6.2 per access, half of them on twiddles and
+// conflicts): see the launchers.
+template <int R0, int R1> struct ZTwo {
+    static constexpr int N = R0 * R1, warps = R0 > R1 ? R0 : R1, threads = 32 * warps;
+    static constexpr int min_blocks = 65536 / (80 * threads) > 0 ? 65536 / (80 * threads) : 1;
+};
+template <int R1> __device__ __forceinline__ int zslot(int p, int c) { return p * 32 + (c ^ ((p / R1) & 7)); }
+__device__ __forceinline__ const double2* ztable(const HGeom& g, double2) { return g.twd_z; }
+__device__ __forceinline__ const float2* ztable(const HGeom& g, float2) { return g.twf_z; }
+
+template <typename C, int R0, int R1>
+__global__ void __launch_bounds__(ZTwo<R0, R1>::threads, ZTwo<R0, R1>::min_blocks)
+k_zsticks_inverse2(const C* __restrict__ psi, int ldp, C* __restrict__ work, HGeom g) {
+    constexpr int N = R0 * R1;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    C* lines = reinterpret_cast<C*>(smem_raw);
+    const int b = blockIdx.y, c0 = blockIdx.x * 32, nl = min(32, g.ncol - c0);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int i = threadIdx.x; i < N * 32; i += blockDim.x) lines[i] = czero<C>();
+    __syncthreads();
+    const int g0 = g.col_start[c0], g1 = g.col_start[c0 + nl];
+    const C* pb = psi + (size_t)b * ldp;
+    for (int q = g0 + threadIdx.x; q < g1; q += blockDim.x)
+        lines[zslot<R1>(g.pw_zpos[q], g.pw_col[q] - c0)] = pb[q];
+    __syncthreads();
+    if (warp < R0) {
+        C* l = lines + warp * R1 * 32 + (lane ^ (warp & 7));
+        C x[R1];
+#pragma unroll
+        for (int j = 0; j < R1; ++j) x[j] = l[j * 32];
+        dft_r<R1, 1>(x);
+#pragma unroll
+        for (int j = 0; j < R1; ++j) l[j * 32] = x[j];
+    }
+    __syncthreads();
+    if (warp < R1) {
+        C x[R0];
+#pragma unroll
+        for (int j = 0; j < R0; ++j) x[j] = lines[(warp + j * R1) * 32 + (lane ^ (j & 7))];
+        p2_span_inverse<R0, R1, false>(x, warp, ztable(g, C{}));
+        C* wb = work + ((size_t)b * N + warp) * g.ncol + c0 + lane;
+        if (lane < nl)
+#pragma unroll
+            for (int j = 0; j < R0; ++j) wb[(size_t)(j * R1) * g.ncol] = x[j];
     }
 }
 
@@ -664,27 +695,15 @@ k_planes_vloc_p3x2(float2* __restrict__ work, const double* __restrict__ veff, i
 }
 
 // ---------------------------------------------------------------- pass 3
-template <typename C, int MODE, int kColsPerBlock, int R0, int R1>
-__global__ void __launch_bounds__(256, ZCfg<R0>::min_blocks)
-k_zsticks_forward(const C* __restrict__ work, const C* __restrict__ psi, int ldp, C* out, int ldo,
-                  HGeom g, Epilogue e) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    C* tw = reinterpret_cast<C*>(smem_raw);
-    C* lines = reinterpret_cast<C*>(smem_raw + align16<C>(g.nz));
+// gather + kinetic + non-local + epilogue over the plane waves of columns c0 ..
+// c1 - 1; slot(position, column) is the place of a value in `lines`
+template <typename C, int MODE, typename Slot>
+__device__ __forceinline__ void z_epilogue(const C* lines, Slot slot, int c0, int c1,
+                                           const C* __restrict__ psi, int ldp, C* out, int ldo,
+                                           const HGeom& g, const Epilogue& e) {
     __shared__ double red[32];
     using R = typename RealOf<C>::type;
     const int b = blockIdx.y;
-    const int c0 = blockIdx.x * kColsPerBlock;
-    const int c1 = min(c0 + kColsPerBlock, g.ncol);
-    const int nl = c1 - c0;
-    copy_twiddles(tw, g.twd_z, g.twf_z, g.nz);
-    const C* wb = work + (size_t)b * g.nz * g.ncol;
-    for (int u = threadIdx.x; u < g.nz * kColsPerBlock; u += blockDim.x) {
-        const int z = u / kColsPerBlock, cl = u - z * kColsPerBlock;
-        lines[cl * g.lsz + swz(z, g.nz)] = cl < nl ? wb[(size_t)z * g.ncol + c0 + cl] : czero<C>();
-    }
-    __syncthreads();
-    zlines_fft<R0, R1, true>(lines, nl, g, tw);
     const int g0 = g.col_start[c0], g1 = g.col_start[c1];
     const C* pb = psi + (size_t)b * ldp;
     C* ob = out + (size_t)b * ldo;
@@ -709,7 +728,7 @@ k_zsticks_forward(const C* __restrict__ work, const C* __restrict__ psi, int ldp
     C* pob = plain ? reinterpret_cast<C*>(e.plain_out) : nullptr;
     double nacc = 0.0;
     for (int q = g0 + threadIdx.x; q < g1; q += blockDim.x) {
-        const C v = lines[(g.pw_col[q] - c0) * g.lsz + swz(g.pw_zpos[q], g.nz)];
+        const C v = lines[slot(g.pw_zpos[q], g.pw_col[q] - c0)];
         const C p = pb[q];
         const R k = (R)e.kin[q];
         C h = mk(p.x * k, p.y * k);
@@ -740,6 +759,63 @@ k_zsticks_forward(const C* __restrict__ work, const C* __restrict__ psi, int ldp
         double s = block_sum(nacc, red);
         if (threadIdx.x == 0) atomicAdd(e.norm_acc, s);
     }
+}
+
+template <typename C, int MODE, int kColsPerBlock>
+__global__ void __launch_bounds__(256)
+k_zsticks_forward(const C* __restrict__ work, const C* __restrict__ psi, int ldp, C* out, int ldo,
+                  HGeom g, Epilogue e) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    C* tw = reinterpret_cast<C*>(smem_raw);
+    C* lines = reinterpret_cast<C*>(smem_raw + align16<C>(g.nz));
+    const int b = blockIdx.y;
+    const int c0 = blockIdx.x * kColsPerBlock;
+    const int c1 = min(c0 + kColsPerBlock, g.ncol);
+    const int nl = c1 - c0;
+    copy_twiddles(tw, g.twd_z, g.twf_z, g.nz);
+    const C* wb = work + (size_t)b * g.nz * g.ncol;
+    for (int u = threadIdx.x; u < g.nz * kColsPerBlock; u += blockDim.x) {
+        const int z = u / kColsPerBlock, cl = u - z * kColsPerBlock;
+        lines[cl * g.lsz + swz(z, g.nz)] = cl < nl ? wb[(size_t)z * g.ncol + c0 + cl] : czero<C>();
+    }
+    __syncthreads();
+    fft_lines_grouped<true>(lines, nl, LinesStrided{g.lsz}, 1, g.az, tw);
+    z_epilogue<C, MODE>(lines, [&](int p, int c) { return c * g.lsz + swz(p, g.nz); }, c0, c1, psi, ldp,
+                        out, ldo, g, e);
+}
+
+// two-radix plans, laid out as k_zsticks_inverse2
+template <typename C, int MODE, int R0, int R1>
+__global__ void __launch_bounds__(ZTwo<R0, R1>::threads, ZTwo<R0, R1>::min_blocks)
+k_zsticks_forward2(const C* __restrict__ work, const C* __restrict__ psi, int ldp, C* out, int ldo,
+                   HGeom g, Epilogue e) {
+    constexpr int N = R0 * R1;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    C* lines = reinterpret_cast<C*>(smem_raw);
+    const int b = blockIdx.y, c0 = blockIdx.x * 32, nl = min(32, g.ncol - c0);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp < R1) {
+        const C* wb = work + ((size_t)b * N + warp) * g.ncol + c0 + lane;
+        C x[R0];
+#pragma unroll
+        for (int j = 0; j < R0; ++j) x[j] = lane < nl ? wb[(size_t)(j * R1) * g.ncol] : czero<C>();
+        p2_span_forward<R0, R1, false>(x, warp, ztable(g, C{}));
+#pragma unroll
+        for (int j = 0; j < R0; ++j) lines[(warp + j * R1) * 32 + (lane ^ (j & 7))] = x[j];
+    }
+    __syncthreads();
+    if (warp < R0) {
+        C* l = lines + warp * R1 * 32 + (lane ^ (warp & 7));
+        C x[R1];
+#pragma unroll
+        for (int j = 0; j < R1; ++j) x[j] = l[j * 32];
+        dft_r<R1, -1>(x);
+#pragma unroll
+        for (int j = 0; j < R1; ++j) l[j * 32] = x[j];
+    }
+    __syncthreads();
+    z_epilogue<C, MODE>(lines, [](int p, int c) { return zslot<R1>(p, c); }, c0, c0 + nl, psi, ldp, out,
+                        ldo, g, e);
 }
 
 // ------------------------------------------------------ density (pass 2')
@@ -951,36 +1027,65 @@ int grid_for(size_t n, int threads) {
 }  // namespace
 
 // ------------------------------------------------------------------ launchers
-template <typename C, int COLS, int R0, int R1>
+// Two-radix plans with compile-time kernels.  FP32 keeps to the first six.
+// clang-format off
+#define CHFSI_ZPLANS32(X) X(9, 8) X(12, 9) X(8, 5) X(12, 12) X(8, 8) X(8, 6)
+#define CHFSI_ZPLANS64(X) CHFSI_ZPLANS32(X) X(6, 5) X(8, 4) X(6, 6) X(9, 5) X(10, 5) X(9, 6) X(10, 6) \
+    X(15, 5) X(10, 8) X(9, 9) X(10, 9) X(12, 8) X(10, 10) X(12, 10)
+// clang-format on
+
+// The plan's key, and whether the kernels for it are built for C
+template <typename C> bool two_radix(const AxisPlan& P, int& key) {
+    key = P.nst == 2 ? P.r[0] * 100 + P.r[1] : 0;
+    switch (key) {
+#define CHFSI_KEY(A, B) case A * 100 + B:
+        CHFSI_ZPLANS32(CHFSI_KEY) return true;
+    default: break;
+    }
+    if constexpr (sizeof(C) == 16) {
+        switch (key) {
+            CHFSI_ZPLANS64(CHFSI_KEY) return true;
+        default: break;
+        }
+    }
+#undef CHFSI_KEY
+    return false;
+}
+
+template <typename C, int R0, int R1>
+void zsticks_inverse2_launch(const C* psi, int ldp, C* work, int nb, const HGeom& g, cudaStream_t st) {
+    dim3 grid((g.ncol + 31) / 32, nb);
+    const size_t sm = (size_t)R0 * R1 * 32 * sizeof(C);
+    allow_smem(k_zsticks_inverse2<C, R0, R1>, sm);
+    k_zsticks_inverse2<C, R0, R1><<<grid, ZTwo<R0, R1>::threads, sm, st>>>(psi, ldp, work, g);
+}
+
+template <typename C, int COLS>
 void zsticks_inverse_launch(const C* psi, int ldp, C* work, int nb, const HGeom& g, cudaStream_t st) {
     dim3 grid((g.ncol + COLS - 1) / COLS, nb);
     size_t sm = align16<C>(g.nz) + (size_t)COLS * g.lsz * sizeof(C);
-    allow_smem(k_zsticks_inverse<C, COLS, R0, R1>, sm);
-    k_zsticks_inverse<C, COLS, R0, R1><<<grid, 256, sm, st>>>(psi, ldp, work, g);
-}
-
-// two-radix z plans with compile-time kernels (the xy-plane list)
-#define CHFSI_ZPLANS(X) X(9, 8) X(12, 9) X(8, 5) X(12, 12) X(8, 8) X(8, 6)
-
-template <typename C, int COLS>
-void zsticks_inverse_cols(const C* psi, int ldp, C* work, int nb, const HGeom& g, cudaStream_t st) {
-    const int key = g.az.nst == 2 ? g.az.r[0] * 100 + g.az.r[1] : 0;
-    switch (key) {
-#define CHFSI_ZI(A, B) case A * 100 + B: zsticks_inverse_launch<C, COLS, A, B>(psi, ldp, work, nb, g, st); return;
-        CHFSI_ZPLANS(CHFSI_ZI)
-#undef CHFSI_ZI
-    default: zsticks_inverse_launch<C, COLS, 0, 0>(psi, ldp, work, nb, g, st);
-    }
+    allow_smem(k_zsticks_inverse<C, COLS>, sm);
+    k_zsticks_inverse<C, COLS><<<grid, 256, sm, st>>>(psi, ldp, work, g);
 }
 
 template <typename C>
 void launch_zsticks_inverse(const C* psi, int ldp, C* work, int nb, const HGeom& g,
                             cudaStream_t st) {
     count_launch();
+    int key;
+    if (two_radix<C>(g.az, key)) {
+#define CHFSI_ZI(A, B) case A * 100 + B: zsticks_inverse2_launch<C, A, B>(psi, ldp, work, nb, g, st); return;
+        if constexpr (sizeof(C) == 16) {
+            switch (key) { CHFSI_ZPLANS64(CHFSI_ZI) }
+        } else {
+            switch (key) { CHFSI_ZPLANS32(CHFSI_ZI) }
+        }
+#undef CHFSI_ZI
+    }
     switch (g.tune_cols) {
-    case 16: zsticks_inverse_cols<C, 16>(psi, ldp, work, nb, g, st); break;
-    case 64: zsticks_inverse_cols<C, 64>(psi, ldp, work, nb, g, st); break;
-    default: zsticks_inverse_cols<C, 32>(psi, ldp, work, nb, g, st); break;
+    case 16: zsticks_inverse_launch<C, 16>(psi, ldp, work, nb, g, st); break;
+    case 64: zsticks_inverse_launch<C, 64>(psi, ldp, work, nb, g, st); break;
+    default: zsticks_inverse_launch<C, 32>(psi, ldp, work, nb, g, st); break;
     }
 }
 
@@ -1070,35 +1175,42 @@ void launch_planes_vloc(C* work, const double* veff, int nb, const HGeom& g, cud
     }
 }
 
-template <typename C, int MODE, int COLS, int R0, int R1>
+template <typename C, int MODE, int R0, int R1>
+void zsticks_forward2_launch(const C* work, const C* psi, int ldp, C* out, int ldo, int nb,
+                             const HGeom& g, const Epilogue& e, cudaStream_t st) {
+    dim3 grid((g.ncol + 31) / 32, nb);
+    const size_t sm = (size_t)R0 * R1 * 32 * sizeof(C);
+    allow_smem(k_zsticks_forward2<C, MODE, R0, R1>, sm);
+    k_zsticks_forward2<C, MODE, R0, R1><<<grid, ZTwo<R0, R1>::threads, sm, st>>>(work, psi, ldp, out, ldo,
+                                                                              g, e);
+}
+
+template <typename C, int MODE, int COLS>
 void zsticks_forward_launch(const C* work, const C* psi, int ldp, C* out, int ldo, int nb,
                             const HGeom& g, const Epilogue& e, cudaStream_t st) {
     dim3 grid((g.ncol + COLS - 1) / COLS, nb);
     size_t sm = align16<C>(g.nz) + (size_t)COLS * g.lsz * sizeof(C);
-    allow_smem(k_zsticks_forward<C, MODE, COLS, R0, R1>, sm);
-    k_zsticks_forward<C, MODE, COLS, R0, R1><<<grid, 256, sm, st>>>(work, psi, ldp, out, ldo, g, e);
+    allow_smem(k_zsticks_forward<C, MODE, COLS>, sm);
+    k_zsticks_forward<C, MODE, COLS><<<grid, 256, sm, st>>>(work, psi, ldp, out, ldo, g, e);
 }
 
-template <typename C, int COLS, int R0, int R1>
-void zsticks_forward_modes(const C* work, const C* psi, int ldp, C* out, int ldo, int nb,
-                           const HGeom& g, const Epilogue& e, cudaStream_t st) {
-    switch (e.mode) {
-    case kEpiApply: zsticks_forward_launch<C, kEpiApply, COLS, R0, R1>(work, psi, ldp, out, ldo, nb, g, e, st); break;
-    case kEpiChebFirst: zsticks_forward_launch<C, kEpiChebFirst, COLS, R0, R1>(work, psi, ldp, out, ldo, nb, g, e, st); break;
-    case kEpiResid: zsticks_forward_launch<C, kEpiResid, COLS, R0, R1>(work, psi, ldp, out, ldo, nb, g, e, st); break;
-    default: zsticks_forward_launch<C, kEpiCheb, COLS, R0, R1>(work, psi, ldp, out, ldo, nb, g, e, st); break;
-    }
-}
-
-template <typename C, int COLS>
-void zsticks_forward_cols(const C* work, const C* psi, int ldp, C* out, int ldo, int nb,
+template <typename C, int MODE>
+void zsticks_forward_mode(const C* work, const C* psi, int ldp, C* out, int ldo, int nb,
                           const HGeom& g, const Epilogue& e, cudaStream_t st) {
-    const int key = g.az.nst == 2 ? g.az.r[0] * 100 + g.az.r[1] : 0;
-    switch (key) {
-#define CHFSI_ZF(A, B) case A * 100 + B: zsticks_forward_modes<C, COLS, A, B>(work, psi, ldp, out, ldo, nb, g, e, st); return;
-        CHFSI_ZPLANS(CHFSI_ZF)
+    int key;
+    if (two_radix<C>(g.az, key)) {
+#define CHFSI_ZF(A, B) case A * 100 + B: zsticks_forward2_launch<C, MODE, A, B>(work, psi, ldp, out, ldo, nb, g, e, st); return;
+        if constexpr (sizeof(C) == 16) {
+            switch (key) { CHFSI_ZPLANS64(CHFSI_ZF) }
+        } else {
+            switch (key) { CHFSI_ZPLANS32(CHFSI_ZF) }
+        }
 #undef CHFSI_ZF
-    default: zsticks_forward_modes<C, COLS, 0, 0>(work, psi, ldp, out, ldo, nb, g, e, st);
+    }
+    switch (g.tune_cols) {
+    case 16: zsticks_forward_launch<C, MODE, 16>(work, psi, ldp, out, ldo, nb, g, e, st); break;
+    case 64: zsticks_forward_launch<C, MODE, 64>(work, psi, ldp, out, ldo, nb, g, e, st); break;
+    default: zsticks_forward_launch<C, MODE, 32>(work, psi, ldp, out, ldo, nb, g, e, st); break;
     }
 }
 
@@ -1106,10 +1218,11 @@ template <typename C>
 void launch_zsticks_forward(const C* work, const C* psi, int ldp, C* out, int ldo, int nb,
                             const HGeom& g, const Epilogue& e, cudaStream_t st) {
     count_launch();
-    switch (g.tune_cols) {
-    case 16: zsticks_forward_cols<C, 16>(work, psi, ldp, out, ldo, nb, g, e, st); break;
-    case 64: zsticks_forward_cols<C, 64>(work, psi, ldp, out, ldo, nb, g, e, st); break;
-    default: zsticks_forward_cols<C, 32>(work, psi, ldp, out, ldo, nb, g, e, st); break;
+    switch (e.mode) {
+    case kEpiApply: zsticks_forward_mode<C, kEpiApply>(work, psi, ldp, out, ldo, nb, g, e, st); break;
+    case kEpiChebFirst: zsticks_forward_mode<C, kEpiChebFirst>(work, psi, ldp, out, ldo, nb, g, e, st); break;
+    case kEpiResid: zsticks_forward_mode<C, kEpiResid>(work, psi, ldp, out, ldo, nb, g, e, st); break;
+    default: zsticks_forward_mode<C, kEpiCheb>(work, psi, ldp, out, ldo, nb, g, e, st); break;
     }
 }
 
