@@ -58,113 +58,27 @@ template <typename C> __host__ __device__ __forceinline__ size_t align16(size_t 
 
 // ---- two-radix line transforms with compile-time plans (N = R0 R1; DIF
 // stage 0: radix R0 with span R1; stage 1: radix R1 on blocks of R1
-// consecutive elements, all twiddles 1), used by the z-stick and plane passes
-// radix-R1 stage on block blk (elements blk R1 .. blk R1 + R1 - 1)
-template <int R0, int R1, int SIGN, typename C>
-__device__ __forceinline__ void p2_blocks(C* line, int es, int blk) {
-    constexpr int N = R0 * R1;
-    C x[R1];
+// consecutive elements, all twiddles 1), used by the z-stick and plane passes.
+// tw[m] = w^(n1 m), w = exp(2 pi i / N), for the span n1
+// DIT stage 0: twiddle, radix-R0 DFT (sign +1)
+template <int R0, typename C>
+__device__ __forceinline__ void span_inverse(C* x, const C* tw) {
 #pragma unroll
-    for (int j = 0; j < R1; ++j) x[j] = line[swz(blk * R1 + j, N) * es];
-    dft_r<R1, SIGN>(x);
-#pragma unroll
-    for (int m = 0; m < R1; ++m) line[swz(blk * R1 + m, N) * es] = x[m];
-}
-template <int R0, int R1, typename C>
-__device__ __forceinline__ void p2_load_span(const C* line, int es, int n1, C* x) {
-#pragma unroll
-    for (int j = 0; j < R0; ++j) x[j] = line[swz(n1 + j * R1, R0 * R1) * es];
-}
-template <int R0, int R1, typename C>
-__device__ __forceinline__ void p2_store_span(C* line, int es, int n1, const C* x) {
-#pragma unroll
-    for (int j = 0; j < R0; ++j) line[swz(n1 + j * R1, R0 * R1) * es] = x[j];
-}
-// Span twiddles in the order the lanes of a group read them:
-// twm[(m - 1) R1 + n1] = w^(n1 m), w = exp(2 pi i / (R0 R1)).  For a fixed m
-// the lanes n1 = 0 .. R1 - 1 read consecutive entries (no bank conflicts;
-// the table w^j indexed by n1 m puts lanes on the same bank group whenever m
-// shares a factor with 8).
-__device__ __forceinline__ double2 tw_entry(const double2* twd, const float2*, int j, double2) {
-    return twd[j];
-}
-__device__ __forceinline__ float2 tw_entry(const double2*, const float2* twf, int j, float2) {
-    return twf[j];
-}
-template <int R0, int R1, typename C>
-__device__ __forceinline__ void p2_twiddles(C* twm, const double2* twd, const float2* twf) {
-    for (int i = threadIdx.x; i < (R0 - 1) * R1; i += blockDim.x) {
-        const int m = i / R1 + 1, n1 = i - (m - 1) * R1;
-        twm[i] = tw_entry(twd, twf, n1 * m, C{});
-    }
-}
-// Lane -> (group, index in group) of the two-radix line transforms with T
-// lanes per line and PW lines per warp.  Indices 0-7 of every group fill
-// whole 8-lane phases (one line per phase), the higher indices follow
-// packed: the 16-byte shared-memory accesses of a phase then fall on one
-// line, whose XOR-swizzled elements span all eight bank groups.
-template <int T, int PW>
-__device__ __forceinline__ void p2_lane(int lane, int& gi, int& li) {
-    if constexpr (T <= 8) {
-        gi = lane / T;
-        li = lane - gi * T;
-    } else {
-        if (lane < PW * 8) {
-            gi = lane >> 3;
-            li = lane & 7;
-        } else {
-            const int r = lane - PW * 8;
-            gi = r / (T - 8);
-            li = 8 + (r - gi * (T - 8));
-        }
-    }
-}
-// Span twiddle w^(n1 m) from the table w^j (TWM false) or from the
-// lane-ordered table of p2_twiddles (TWM true)
-template <int R1, bool TWM, typename C>
-__device__ __forceinline__ C span_tw(const C* tw, int n1, int m) {
-    return TWM ? tw[(m - 1) * R1 + n1] : tw[n1 * m];
-}
-// DIT stage 0 on span n1: twiddle w^(n1 m), radix-R0 DFT (sign +1)
-template <int R0, int R1, bool TWM, typename C>
-__device__ __forceinline__ void p2_span_inverse(C* x, int n1, const C* tw) {
-#pragma unroll
-    for (int m = 1; m < R0; ++m) x[m] = cmul(span_tw<R1, TWM>(tw, n1, m), x[m]);
+    for (int m = 1; m < R0; ++m) x[m] = cmul(tw[m], x[m]);
     dft_r<R0, 1>(x);
 }
-// DIF stage 0 on span n1: radix-R0 DFT (sign -1), twiddle w^(-n1 m)
-template <int R0, int R1, bool TWM, typename C>
-__device__ __forceinline__ void p2_span_forward(C* x, int n1, const C* tw) {
+// DIF stage 0: radix-R0 DFT (sign -1), twiddle
+template <int R0, typename C>
+__device__ __forceinline__ void span_forward(C* x, const C* tw) {
     dft_r<R0, -1>(x);
 #pragma unroll
-    for (int m = 1; m < R0; ++m) x[m] = cmulc(span_tw<R1, TWM>(tw, n1, m), x[m]);
+    for (int m = 1; m < R0; ++m) x[m] = cmulc(tw[m], x[m]);
 }
-// whole-line transforms by one lane group (lane i); every lane of the warp
-// calls them (act = false: idle)
-template <int R0, int R1, bool TWM, typename C>
-__device__ __forceinline__ void p2_line_inverse(C* line, bool act, int i, int es, const C* tw) {
-    if (act && i < R0) p2_blocks<R0, R1, 1>(line, es, i);
-    __syncwarp();
-    if (act && i < R1) {
-        C x[R0];
-        p2_load_span<R0, R1>(line, es, i, x);
-        p2_span_inverse<R0, R1, TWM>(x, i, tw);
-        p2_store_span<R0, R1>(line, es, i, x);
-    }
-    __syncwarp();
-}
-template <int R0, int R1, bool TWM, typename C>
-__device__ __forceinline__ void p2_line_forward(C* line, bool act, int i, int es, const C* tw) {
-    if (act && i < R1) {
-        C x[R0];
-        p2_load_span<R0, R1>(line, es, i, x);
-        p2_span_forward<R0, R1, TWM>(x, i, tw);
-        p2_store_span<R0, R1>(line, es, i, x);
-    }
-    __syncwarp();
-    if (act && i < R0) p2_blocks<R0, R1, -1>(line, es, i);
-    __syncwarp();
-}
+// tables w^j of the x and z axes
+__device__ __forceinline__ const double2* xtable(const HGeom& g, double2) { return g.twd_x; }
+__device__ __forceinline__ const float2* xtable(const HGeom& g, float2) { return g.twf_x; }
+__device__ __forceinline__ const double2* ztable(const HGeom& g, double2) { return g.twd_z; }
+__device__ __forceinline__ const float2* ztable(const HGeom& g, float2) { return g.twf_z; }
 
 // ---------------------------------------------------------------- pass 1
 // z lines of a block of columns, generic plans (one lane group per line)
@@ -204,14 +118,13 @@ k_zsticks_inverse(const C* __restrict__ psi, int ldp, C* __restrict__ work, HGeo
 // (consecutive frequencies, a block apart) over the banks for the scatter and the
 // gather.  Against lane groups along each line (which spent 81 % of the
 // shared-memory wavefronts, 6.2 per access, half of them on twiddles and
-// conflicts): see the launchers.
+// conflicts), 160 bands on 72^3, us a launch: FP64 inverse 138 -> 125, H apply
+// 190 -> 120, Chebyshev step 227 -> 175; FP32 100 -> 53 and 195 -> 87.
 template <int R0, int R1> struct ZTwo {
     static constexpr int N = R0 * R1, warps = R0 > R1 ? R0 : R1, threads = 32 * warps;
     static constexpr int min_blocks = 65536 / (80 * threads) > 0 ? 65536 / (80 * threads) : 1;
 };
 template <int R1> __device__ __forceinline__ int zslot(int p, int c) { return p * 32 + (c ^ ((p / R1) & 7)); }
-__device__ __forceinline__ const double2* ztable(const HGeom& g, double2) { return g.twd_z; }
-__device__ __forceinline__ const float2* ztable(const HGeom& g, float2) { return g.twf_z; }
 
 template <typename C, int R0, int R1>
 __global__ void __launch_bounds__(ZTwo<R0, R1>::threads, ZTwo<R0, R1>::min_blocks)
@@ -242,7 +155,10 @@ k_zsticks_inverse2(const C* __restrict__ psi, int ldp, C* __restrict__ work, HGe
         C x[R0];
 #pragma unroll
         for (int j = 0; j < R0; ++j) x[j] = lines[(warp + j * R1) * 32 + (lane ^ (j & 7))];
-        p2_span_inverse<R0, R1, false>(x, warp, ztable(g, C{}));
+        C tw[R0];
+#pragma unroll
+        for (int m = 1; m < R0; ++m) tw[m] = __ldg(ztable(g, C{}) + warp * m);
+        span_inverse<R0>(x, tw);
         C* wb = work + ((size_t)b * N + warp) * g.ncol + c0 + lane;
         if (lane < nl)
 #pragma unroll
@@ -308,224 +224,320 @@ k_planes_vloc(C* __restrict__ work, const double* __restrict__ veff, HGeom g) {
 }
 
 // ------------------------------------------ pass 2, two-radix compile-time plans
-// The same plane pipeline for axes whose plan has two radices, N = R0 R1
-// (DIF stage 0: radix R0 with span R1; stage 1: radix R1 on blocks of R1
-// consecutive elements, where every twiddle is 1).  Radices, spans and
-// twiddle indices are compile-time constants, and along x the last inverse
-// stage, the V(r) multiply and the first forward stage share registers:
-// lane n1 of a row's lane group holds the R0 elements n1 + m R1, which is
-// what those two stages read and write.
-
-// Square planes (nx = ny = R0 R1, both axes on the same plan); shared memory
-// layout and launch shape as k_planes_vloc.
-template <typename C, int V, int R0, int R1>
-__global__ void __launch_bounds__(PlanesCfg<C, V>::threads, PlanesCfg<C, V>::min_blocks)
-k_planes_vloc_p2(C* __restrict__ work, const double* __restrict__ veff, HGeom g) {
-    constexpr int N = R0 * R1, LS = N | 1, T = R0 > R1 ? R0 : R1, PW = 32 / T;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    C* twx = reinterpret_cast<C*>(smem_raw);
-    C* twy = reinterpret_cast<C*>(smem_raw + align16<C>(N));
-    C* plane = reinterpret_cast<C*>(smem_raw + 2 * align16<C>(N));
-    int* xl = reinterpret_cast<int*>(plane + (size_t)N * LS);
-    const int z = blockIdx.x, b = blockIdx.y;
-    const int nxact = g.nxact;
-    p2_twiddles<R0, R1, C>(twx, g.twd_x, g.twf_x);
-    p2_twiddles<R0, R1, C>(twy, g.twd_y, g.twf_y);
-    for (int i = threadIdx.x; i < nxact; i += blockDim.x) xl[i] = g.xact[i];
-    for (int i = threadIdx.x; i < N * LS; i += blockDim.x) plane[i] = czero<C>();
-    __syncthreads();
-    C* wp = work + ((size_t)b * g.nz + z) * g.ncol;
-    for (int c = threadIdx.x; c < g.ncol; c += blockDim.x) plane[g.col_pos[c]] = wp[c];
-    __syncthreads();
-    const int lane = threadIdx.x & 31;
-    int gi, li;
-    p2_lane<T, PW>(lane, gi, li);
-    const bool ing = gi < PW;
-    const int groups = (blockDim.x >> 5) * PW, gid = (threadIdx.x >> 5) * PW + gi;
-    // y lines through the active x positions
-    for (int l0 = 0; l0 < nxact; l0 += groups) {
-        const int l = l0 + gid;
-        const bool act = ing && l < nxact;
-        p2_line_inverse<R0, R1, true>(plane + (act ? xl[l] : 0), act, li, LS, twy);
-    }
-    __syncthreads();
-    // x rows: inverse, x V(r), forward
-    using R = typename RealOf<C>::type;
-    const double* vz = veff + (size_t)z * N * N;
-    for (int y0 = 0; y0 < N; y0 += groups) {
-        const int y = y0 + gid;
-        const bool act = ing && y < N;
-        C* row = plane + (act ? swz(y, N) * LS : 0);
-        if (act && li < R0) p2_blocks<R0, R1, 1>(row, 1, li);
-        __syncwarp();
-        if (act && li < R1) {
-            C x[R0];
-            p2_load_span<R0, R1>(row, 1, li, x);
-            p2_span_inverse<R0, R1, true>(x, li, twx);
-            const double* vr = vz + (size_t)y * N + li;
-#pragma unroll
-            for (int m = 0; m < R0; ++m) x[m] = cscale(x[m], (R)vr[m * R1]);
-            p2_span_forward<R0, R1, true>(x, li, twx);
-            p2_store_span<R0, R1>(row, 1, li, x);
+// Square planes on a two-radix plan.  The plane's columns are read and written in
+// place of a scatter and a gather: the first inverse y stage of every active x
+// line loads its inputs from the column array (zero where (x, y) holds no column),
+// the last forward y stage stores its outputs straight to the columns, the first
+// inverse x stage takes zero for x positions without columns, and the last
+// forward x stage stores only the positions the forward y stage reads; nothing is
+// zeroed.  Along x the last inverse stage, the V(r) multiply and the first forward
+// stage share registers.
+// Bound by shared-memory wavefronts and the FP64 pipe.  A warp takes 8 lines x 4
+// butterflies of a stage: the 8 lanes of an access phase hold the same element of
+// 8 neighbouring lines, a bank group each (rows are an odd number of 16-byte
+// elements long; active x lines come in the order of x, which the digit reversal, with
+// positions XOR-swizzled for even R1, spreads over the groups, and whose columns lie
+// side by side in memory), a lane's span index is the same
+// throughout, so that its twiddles stay in registers, and every lane works in most rounds whatever the radices (with a lane group per
+// line a 12 x 9 plan left a quarter of the lanes idle and took 3.7 times the
+// wavefronts of its data).  Stages are separated by block barriers and the blocks of
+// one SM overlap; on planes up to 50 x 50 a warp keeps its lines instead (40 x 40,
+// 200 bands: 134 us a local H against 153; 72 x 72: 815 against 811).  Local H in
+// all, us, before / with this kernel: 40^3 x 200 bands 183 / 134, 64^3 x 160 577 /
+// 508, 72^3 x 160 820 / 811, 80^3 x 100 1,840 / 746 (generic kernel before),
+// 108^3 x 576 17,880 / 11,550.
+// NB bands per 16-byte element: 1 in FP64; in FP32 bands 2p and 2p + 1, so that
+// each twiddle and V(r) load serves both (an odd last band runs alone: its
+// partner's loads repeat it and are not stored).
+template <int R0, int R1> struct PlaneTwo {
+    static constexpr int N = R0 * R1, LS = N | 1, G = (N + 7) / 8;
+    static constexpr int Q0 = (R0 + 3) / 4, Q1 = (R1 + 3) / 4;
+    static constexpr int bytes = N * LS * 16 + ((N + 3) & ~3) * 4 + (R0 - 1) * R1 * 16;
+    static constexpr int fit = 227 * 1024 / (bytes + 1024);  // blocks by shared memory
+    // warps: near 9 (14 where one block fills the SM), a multiple of Q1 so that a
+    // warp keeps its spans, wasting the fewest warp rounds of the x stages
+    static constexpr int pick() {
+        const int lo = fit > 1 ? 8 : 12, hi = fit > 1 ? 10 : 16;
+        int best = lo, waste = 1 << 30;
+        for (int w = lo; w <= hi; ++w) {
+            if (w % Q1) continue;
+            const int r = w * (2 * ((G * Q0 + w - 1) / w) + (G + w / Q1 - 1) / (w / Q1));
+            if (r <= waste) {
+                waste = r;
+                best = w;
+            }
         }
-        __syncwarp();
-        if (act && li < R0) p2_blocks<R0, R1, -1>(row, 1, li);
-        __syncwarp();
+        return best;
     }
-    __syncthreads();
-    for (int l0 = 0; l0 < nxact; l0 += groups) {
-        const int l = l0 + gid;
-        const bool act = ing && l < nxact;
-        p2_line_forward<R0, R1, true>(plane + (act ? xl[l] : 0), act, li, LS, twy);
-    }
-    __syncthreads();
-    for (int c = threadIdx.x; c < g.ncol; c += blockDim.x) wp[c] = plane[g.col_pos[c]];
+    // small planes (up to 50 x 50): a warp takes a group of lines through all its
+    // stages, without block barriers between them
+    static constexpr bool own = fit >= 5;
+    static constexpr int warps = own ? G : pick(), threads = 32 * warps;
+    static constexpr int by_regs = 65536 / (threads * 96);
+    static constexpr int min_blocks = fit < by_regs ? fit : by_regs > 0 ? by_regs : 1;
+    // place of x position p in a row
+    __device__ __forceinline__ static int at(int p) { return R1 % 2 ? p : swz(p, N); }
+};
+
+__device__ __forceinline__ void unpack(double2 e, double2 (&x)[1]) { x[0] = e; }
+__device__ __forceinline__ void unpack(float4 e, float2 (&x)[2]) {
+    x[0] = make_float2(e.x, e.y);
+    x[1] = make_float2(e.z, e.w);
 }
+__device__ __forceinline__ double2 pack(const double2 (&x)[1]) { return x[0]; }
+__device__ __forceinline__ float4 pack(const float2 (&x)[2]) { return make_float4(x[0].x, x[0].y, x[1].x, x[1].y); }
+template <int NB> struct PlaneElem { using type = double2; };
+template <> struct PlaneElem<2> { using type = float4; };
 
-// ------------------------------- pass 2, compile-time plans, no zero fill
-// The compile-time pipeline with the plane's columns read and written in
-// place of the shared-memory scatter and gather: the first inverse y stage
-// of every active x line loads its inputs from the column array (zero where
-// (x, y) holds no column), the last forward y stage stores its outputs
-// straight to the columns, the first inverse x stage reads zero for x
-// positions without columns instead of loading them, and the last forward x
-// stage stores only the x positions the forward y stage reads.  No position
-// of the plane is ever read before this CTA writes it, so the plane is not
-// zeroed, and the shared-memory traffic per plane drops by about 30 %.
-template <typename C, int V, int R0, int R1>
-__global__ void __launch_bounds__(PlanesCfg<C, V>::threads, PlanesCfg<C, V>::min_blocks)
-k_planes_vloc_p3(C* __restrict__ work, const double* __restrict__ veff, HGeom g) {
-    constexpr int N = R0 * R1, LS = N | 1, T = R0 > R1 ? R0 : R1, PW = 32 / T;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    C* twx = reinterpret_cast<C*>(smem_raw);
-    C* twy = reinterpret_cast<C*>(smem_raw + align16<C>(N));
-    C* plane = reinterpret_cast<C*>(smem_raw + 2 * align16<C>(N));
-    int* xl = reinterpret_cast<int*>(plane + (size_t)N * LS);
-    const int z = blockIdx.x, b = blockIdx.y;
-    const int nxact = g.nxact;
-    p2_twiddles<R0, R1, C>(twx, g.twd_x, g.twf_x);
-    p2_twiddles<R0, R1, C>(twy, g.twd_y, g.twf_y);
-    for (int i = threadIdx.x; i < nxact; i += blockDim.x) xl[i] = g.xact[i];
-    __syncthreads();
-    C* wp = work + ((size_t)b * g.nz + z) * g.ncol;
-    const int lane = threadIdx.x & 31;
-    int gi, li;
-    p2_lane<T, PW>(lane, gi, li);
-    const bool ing = gi < PW;
-    const int groups = (blockDim.x >> 5) * PW, gid = (threadIdx.x >> 5) * PW + gi;
+// values of a butterfly, band by band
+template <typename C, int NB, int R> struct Bfly {
+    C x[NB][R];
+    template <typename S> __device__ __forceinline__ void set(int j, S e) {
+        C v[NB];
+        unpack(e, v);
+#pragma unroll
+        for (int b = 0; b < NB; ++b) x[b][j] = v[b];
+    }
+    __device__ __forceinline__ typename PlaneElem<NB>::type get(int j) const {
+        C v[NB];
+#pragma unroll
+        for (int b = 0; b < NB; ++b) v[b] = x[b][j];
+        return pack(v);
+    }
+    template <int SIGN> __device__ __forceinline__ void dft() {
+#pragma unroll
+        for (int b = 0; b < NB; ++b) dft_r<R, SIGN>(x[b]);
+    }
+};
+
+template <typename C, int NB, int R0, int R1>
+__global__ void __launch_bounds__(PlaneTwo<R0, R1>::threads, PlaneTwo<R0, R1>::min_blocks)
+k_planes_vloc2(C* __restrict__ work, const double* __restrict__ veff, int nb, HGeom g) {
+    using P = PlaneTwo<R0, R1>;
+    using S = typename PlaneElem<NB>::type;
     using R = typename RealOf<C>::type;
-    // y lines through the active x positions: inverse, inputs from the columns
-    for (int l0 = 0; l0 < nxact; l0 += groups) {
-        const int l = l0 + gid;
-        const bool act = ing && l < nxact;
-        C* line = plane + (act ? xl[l] : 0);
-        if (act && li < R0) {
-            const int* ci = g.colidx + (size_t)l * N + li * R1;
-            C x[R1];
+    constexpr int N = P::N, LS = P::LS, W = P::warps;
+    constexpr bool own = P::own;          // a warp takes its lines through all stages
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    S* plane = reinterpret_cast<S*>(smem_raw);
+    int* xl = reinterpret_cast<int*>(plane + (size_t)N * LS);
+    const int z = blockIdx.x, b0 = NB * blockIdx.y, nxact = g.nxact;
+    for (int i = threadIdx.x; i < nxact; i += blockDim.x) xl[i] = P::at(g.xline[i]);
+    C* wp[NB];
+    bool live[NB];
 #pragma unroll
-            for (int j = 0; j < R1; ++j) {
-                const int c = __ldg(ci + j);
-                x[j] = c >= 0 ? wp[c] : czero<C>();
-            }
-            dft_r<R1, 1>(x);
+    for (int b = 0; b < NB; ++b) {
+        live[b] = b0 + b < nb;
+        wp[b] = work + ((size_t)(live[b] ? b0 + b : b0) * g.nz + z) * g.ncol;
+    }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane & 7, t = lane >> 3;
+    const int gy = (nxact + 7) >> 3;
+    // twiddles w^(n1 m) of this lane's spans: one span where a warp keeps to its
+    // quad, else from the lane-ordered table in shared memory
+    C* twm = reinterpret_cast<C*>(xl + ((N + 3) & ~3));
+    C tw[R0];
+    if constexpr (own) {
+        for (int i = threadIdx.x; i < (R0 - 1) * R1; i += blockDim.x) {
+            const int m = i / R1 + 1;
+            twm[i] = xtable(g, C{})[(i - (m - 1) * R1) * m];
+        }
+    } else {
+        const int n1 = (warp % P::Q1) * 4 + t;
 #pragma unroll
-            for (int m = 0; m < R1; ++m) line[swz(li * R1 + m, N) * LS] = x[m];
-        }
-        __syncwarp();
-        if (act && li < R1) {
-            C x[R0];
-            p2_load_span<R0, R1>(line, LS, li, x);
-            p2_span_inverse<R0, R1, true>(x, li, twy);
-            p2_store_span<R0, R1>(line, LS, li, x);
-        }
-        __syncwarp();
+        for (int m = 1; m < R0; ++m) tw[m] = n1 < R1 ? __ldg(xtable(g, C{}) + n1 * m) : czero<C>();
     }
     __syncthreads();
-    // x rows: inverse (x positions without columns read as zero), x V(r),
-    // forward (only x positions with columns stored)
+    auto stage_sync = [&]() {
+        if constexpr (own) __syncwarp();
+        else __syncthreads();
+    };
+    // the butterflies of one stage over `groups` groups of 8 lines: f(line, index)
+    auto blocks = [&](int groups, int grp, auto&& f) {
+        if constexpr (own) {
+#pragma unroll
+            for (int q = 0; q < P::Q0; ++q)
+                if (q * 4 + t < R0) f(grp * 8 + r, q * 4 + t);
+        } else {
+            for (int it = warp; it < groups * P::Q0; it += W)
+                if ((it % P::Q0) * 4 + t < R0) f((it / P::Q0) * 8 + r, (it % P::Q0) * 4 + t);
+        }
+    };
+    auto spans = [&](int groups, int grp, auto&& f) {
+        if constexpr (own) {
+#pragma unroll
+            for (int q = 0; q < P::Q1; ++q) {
+                const int n1 = q * 4 + t;
+                if (n1 < R1) {
+#pragma unroll
+                    for (int m = 1; m < R0; ++m) tw[m] = twm[(m - 1) * R1 + n1];
+                    f(grp * 8 + r, n1);
+                }
+            }
+        } else {
+            const int n1 = (warp % P::Q1) * 4 + t;
+            if (n1 < R1)
+                for (int it = warp / P::Q1; it < groups; it += W / P::Q1) f(it * 8 + r, n1);
+        }
+    };
+    auto y_blocks_in = [&](int l, int blk) {  // inverse, from the columns
+        if (l >= nxact) return;
+        Bfly<C, NB, R1> v;
+        const int* ci = g.colidx_t + (size_t)blk * R1 * nxact + l;
+#pragma unroll
+        for (int j = 0; j < R1; ++j) {
+            const int c = __ldg(ci + j * nxact);
+#pragma unroll
+            for (int b = 0; b < NB; ++b) v.x[b][j] = c >= 0 ? wp[b][c] : czero<C>();
+        }
+        v.template dft<1>();
+        S* p = plane + (size_t)blk * R1 * LS + xl[l];
+#pragma unroll
+        for (int j = 0; j < R1; ++j) p[j * LS] = v.get(j);
+    };
+    auto y_span = [&](int l, int n1, bool fwd) {
+        if (l >= nxact) return;
+        Bfly<C, NB, R0> v;
+        S* p = plane + (size_t)n1 * LS + xl[l];
+#pragma unroll
+        for (int j = 0; j < R0; ++j) v.set(j, p[j * R1 * LS]);
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+            if (fwd) span_forward<R0>(v.x[b], tw);
+            else span_inverse<R0>(v.x[b], tw);
+        }
+#pragma unroll
+        for (int j = 0; j < R0; ++j) p[j * R1 * LS] = v.get(j);
+    };
+    auto y_blocks_out = [&](int l, int blk) {  // forward, to the columns
+        if (l >= nxact) return;
+        Bfly<C, NB, R1> v;
+        const S* p = plane + (size_t)blk * R1 * LS + xl[l];
+#pragma unroll
+        for (int j = 0; j < R1; ++j) v.set(j, p[j * LS]);
+        v.template dft<-1>();
+        const int* ci = g.colidx_t + (size_t)blk * R1 * nxact + l;
+#pragma unroll
+        for (int j = 0; j < R1; ++j) {
+            const int c = __ldg(ci + j * nxact);
+            if (c >= 0)
+#pragma unroll
+                for (int b = 0; b < NB; ++b)
+                    if (live[b]) wp[b][c] = v.x[b][j];
+        }
+    };
+    auto x_blocks_in = [&](int y, int blk) {
+        if (y >= N) return;
+        Bfly<C, NB, R1> v;
+        S* row = plane + y * LS;
+#pragma unroll
+        for (int j = 0; j < R1; ++j) {
+            const int px = blk * R1 + j;
+            const bool on = (g.xbits[px >> 5] >> (px & 31)) & 1u;
+            v.set(j, on ? row[P::at(px)] : S{});
+        }
+        v.template dft<1>();
+#pragma unroll
+        for (int j = 0; j < R1; ++j) row[P::at(blk * R1 + j)] = v.get(j);
+    };
     const double* vz = veff + (size_t)z * N * N;
-    for (int y0 = 0; y0 < N; y0 += groups) {
-        const int y = y0 + gid;
-        const bool act = ing && y < N;
-        C* row = plane + (act ? swz(y, N) * LS : 0);
-        if (act && li < R0) {
-            C x[R1];
+    auto x_spans = [&](int y, int n1) {  // last inverse stage, V(r), first forward stage
+        if (y >= N) return;
+        Bfly<C, NB, R0> v;
+        S* row = plane + y * LS;
+        const double* vr = vz + (size_t)y * N + n1;
 #pragma unroll
-            for (int j = 0; j < R1; ++j) {
-                const int px = li * R1 + j;
-                const bool on = (g.xbits[px >> 5] >> (px & 31)) & 1u;
-                x[j] = on ? row[swz(px, N)] : czero<C>();
-            }
-            dft_r<R1, 1>(x);
+        for (int j = 0; j < R0; ++j) v.set(j, row[P::at(n1 + j * R1)]);
 #pragma unroll
-            for (int m = 0; m < R1; ++m) row[swz(li * R1 + m, N)] = x[m];
+        for (int b = 0; b < NB; ++b) span_inverse<R0>(v.x[b], tw);
+#pragma unroll
+        for (int j = 0; j < R0; ++j) {
+            const R s = (R)__ldg(vr + j * R1);
+#pragma unroll
+            for (int b = 0; b < NB; ++b) v.x[b][j] = cscale(v.x[b][j], s);
         }
-        __syncwarp();
-        if (act && li < R1) {
-            C x[R0];
-            p2_load_span<R0, R1>(row, 1, li, x);
-            p2_span_inverse<R0, R1, true>(x, li, twx);
-            const double* vr = vz + (size_t)y * N + li;
 #pragma unroll
-            for (int m = 0; m < R0; ++m) x[m] = cscale(x[m], (R)vr[m * R1]);
-            p2_span_forward<R0, R1, true>(x, li, twx);
-            p2_store_span<R0, R1>(row, 1, li, x);
+        for (int b = 0; b < NB; ++b) span_forward<R0>(v.x[b], tw);
+#pragma unroll
+        for (int j = 0; j < R0; ++j) row[P::at(n1 + j * R1)] = v.get(j);
+    };
+    auto x_blocks_out = [&](int y, int blk) {
+        if (y >= N) return;
+        Bfly<C, NB, R1> v;
+        S* row = plane + y * LS;
+#pragma unroll
+        for (int j = 0; j < R1; ++j) v.set(j, row[P::at(blk * R1 + j)]);
+        v.template dft<-1>();
+#pragma unroll
+        for (int j = 0; j < R1; ++j) {
+            const int px = blk * R1 + j;
+            if ((g.xbits[px >> 5] >> (px & 31)) & 1u) row[P::at(px)] = v.get(j);
         }
-        __syncwarp();
-        if (act && li < R0) {
-            C x[R1];
-#pragma unroll
-            for (int j = 0; j < R1; ++j) x[j] = row[swz(li * R1 + j, N)];
-            dft_r<R1, -1>(x);
-#pragma unroll
-            for (int m = 0; m < R1; ++m) {
-                const int px = li * R1 + m;
-                if ((g.xbits[px >> 5] >> (px & 31)) & 1u) row[swz(px, N)] = x[m];
-            }
-        }
-        __syncwarp();
+    };
+    for (int grp = warp; grp < (own ? gy : warp + 1); grp += W) {
+        blocks(gy, grp, y_blocks_in);
+        stage_sync();
+        spans(gy, grp, [&](int l, int n1) { y_span(l, n1, false); });
     }
     __syncthreads();
-    // y lines forward, outputs to the columns
-    for (int l0 = 0; l0 < nxact; l0 += groups) {
-        const int l = l0 + gid;
-        const bool act = ing && l < nxact;
-        C* line = plane + (act ? xl[l] : 0);
-        if (act && li < R1) {
-            C x[R0];
-            p2_load_span<R0, R1>(line, LS, li, x);
-            p2_span_forward<R0, R1, true>(x, li, twy);
-            p2_store_span<R0, R1>(line, LS, li, x);
-        }
-        __syncwarp();
-        if (act && li < R0) {
-            C x[R1];
-#pragma unroll
-            for (int j = 0; j < R1; ++j) x[j] = line[swz(li * R1 + j, N) * LS];
-            dft_r<R1, -1>(x);
-            const int* ci = g.colidx + (size_t)l * N + li * R1;
-#pragma unroll
-            for (int m = 0; m < R1; ++m) {
-                const int c = __ldg(ci + m);
-                if (c >= 0) wp[c] = x[m];
-            }
-        }
-        __syncwarp();
+    for (int grp = warp; grp < (own ? P::G : warp + 1); grp += W) {
+        blocks(P::G, grp, x_blocks_in);
+        stage_sync();
+        spans(P::G, grp, x_spans);
+        stage_sync();
+        blocks(P::G, grp, x_blocks_out);
+    }
+    __syncthreads();
+    for (int grp = warp; grp < (own ? gy : warp + 1); grp += W) {
+        spans(gy, grp, [&](int l, int n1) { y_span(l, n1, true); });
+        stage_sync();
+        blocks(gy, grp, y_blocks_out);
     }
 }
 
 // ------------------------- pass 2, FP32, two bands per CTA (compile-time plans)
-// The pipeline of k_planes_vloc_p3 for the FP32 filter with the same plane
-// position of bands 2p and 2p + 1 in one 16-byte shared-memory element: every
-// shared access is a 16-byte access in 8-lane phases, the case the lane
-// mapping and lane-ordered twiddles make conflict-free (8-byte elements in
-// 16-lane phases put two lines on the same bank groups), and each twiddle and
-// V(r) load serves both bands.  An odd last band runs alone (its partner
-// loads repeat it and are not stored).
+// The same pipeline with a lane group per line and whole lines per warp, for the
+// FP32 filter on planes of which two blocks fit an SM: without the FP64 pipe as a
+// second limit its fewer V(r) wavefronts win (72 x 72, 160 bands: 326 us a launch
+// against 351 for k_planes_vloc2).
 __device__ __forceinline__ float4 pair4(float2 a, float2 b) { return make_float4(a.x, a.y, b.x, b.y); }
 __device__ __forceinline__ float2 lo2(float4 v) { return make_float2(v.x, v.y); }
 __device__ __forceinline__ float2 hi2(float4 v) { return make_float2(v.z, v.w); }
 
+// lane-ordered span twiddles: twm[(m - 1) R1 + n1] = w^(n1 m)
+template <int R0, int R1>
+__device__ __forceinline__ void lane_twiddles(float2* twm, const float2* tab) {
+    for (int i = threadIdx.x; i < (R0 - 1) * R1; i += blockDim.x) {
+        const int m = i / R1 + 1, n1 = i - (m - 1) * R1;
+        twm[i] = tab[n1 * m];
+    }
+}
+template <int R0, int R1>
+__device__ __forceinline__ void lane_tw(float2* tw, const float2* twm, int n1) {
+#pragma unroll
+    for (int m = 1; m < R0; ++m) tw[m] = twm[(m - 1) * R1 + n1];
+}
+
+// Lane -> (group, index in group) of the two-radix line transforms with T
+// lanes per line and PW lines per warp.  Indices 0-7 of every group fill
+// whole 8-lane phases (one line per phase), the higher indices follow
+// packed: the 16-byte shared-memory accesses of a phase then fall on one
+// line, whose XOR-swizzled elements span all eight bank groups.
+template <int T, int PW>
+__device__ __forceinline__ void p2_lane(int lane, int& gi, int& li) {
+    if constexpr (T <= 8) {
+        gi = lane / T;
+        li = lane - gi * T;
+    } else {
+        if (lane < PW * 8) {
+            gi = lane >> 3;
+            li = lane & 7;
+        } else {
+            const int r = lane - PW * 8;
+            gi = r / (T - 8);
+            li = 8 + (r - gi * (T - 8));
+        }
+    }
+}
 template <int V, int R0, int R1>
 __global__ void __launch_bounds__(PlanesCfg<double2, V>::threads, PlanesCfg<double2, V>::min_blocks)
 k_planes_vloc_p3x2(float2* __restrict__ work, const double* __restrict__ veff, int nb, HGeom g) {
@@ -538,9 +550,9 @@ k_planes_vloc_p3x2(float2* __restrict__ work, const double* __restrict__ veff, i
     const int z = blockIdx.x, b0 = 2 * blockIdx.y;
     const bool two = b0 + 1 < nb;
     const int nxact = g.nxact;
-    p2_twiddles<R0, R1, float2>(twx, g.twd_x, g.twf_x);
-    p2_twiddles<R0, R1, float2>(twy, g.twd_y, g.twf_y);
-    for (int i = threadIdx.x; i < nxact; i += blockDim.x) xl[i] = g.xact[i];
+    lane_twiddles<R0, R1>(twx, g.twf_x);
+    lane_twiddles<R0, R1>(twy, g.twf_y);
+    for (int i = threadIdx.x; i < nxact; i += blockDim.x) xl[i] = swz(g.xline[i], N);
     __syncthreads();
     float2* wa = work + ((size_t)b0 * g.nz + z) * g.ncol;
     float2* wb = two ? work + ((size_t)(b0 + 1) * g.nz + z) * g.ncol : wa;
@@ -556,11 +568,11 @@ k_planes_vloc_p3x2(float2* __restrict__ work, const double* __restrict__ veff, i
         const bool act = ing && l < nxact;
         float4* line = plane + (act ? xl[l] : 0);
         if (act && li < R0) {
-            const int* ci = g.colidx + (size_t)l * N + li * R1;
+            const int* ci = g.colidx_t + (size_t)li * R1 * nxact + l;
             float2 xa[R1], xb[R1];
 #pragma unroll
             for (int j = 0; j < R1; ++j) {
-                const int c = __ldg(ci + j);
+                const int c = __ldg(ci + j * nxact);
                 xa[j] = c >= 0 ? wa[c] : zero;
                 xb[j] = c >= 0 ? wb[c] : zero;
             }
@@ -578,8 +590,10 @@ k_planes_vloc_p3x2(float2* __restrict__ work, const double* __restrict__ veff, i
                 xa[j] = lo2(v);
                 xb[j] = hi2(v);
             }
-            p2_span_inverse<R0, R1, true>(xa, li, twy);
-            p2_span_inverse<R0, R1, true>(xb, li, twy);
+            float2 tw[R0];
+            lane_tw<R0, R1>(tw, twy, li);
+            span_inverse<R0>(xa, tw);
+            span_inverse<R0>(xb, tw);
 #pragma unroll
             for (int j = 0; j < R0; ++j) line[swz(li + j * R1, N) * LS] = pair4(xa[j], xb[j]);
         }
@@ -617,8 +631,10 @@ k_planes_vloc_p3x2(float2* __restrict__ work, const double* __restrict__ veff, i
                 xa[j] = lo2(v);
                 xb[j] = hi2(v);
             }
-            p2_span_inverse<R0, R1, true>(xa, li, twx);
-            p2_span_inverse<R0, R1, true>(xb, li, twx);
+            float2 tw[R0];
+            lane_tw<R0, R1>(tw, twx, li);
+            span_inverse<R0>(xa, tw);
+            span_inverse<R0>(xb, tw);
             const double* vr = vz + (size_t)y * N + li;
 #pragma unroll
             for (int m = 0; m < R0; ++m) {
@@ -626,8 +642,8 @@ k_planes_vloc_p3x2(float2* __restrict__ work, const double* __restrict__ veff, i
                 xa[m] = cscale(xa[m], s);
                 xb[m] = cscale(xb[m], s);
             }
-            p2_span_forward<R0, R1, true>(xa, li, twx);
-            p2_span_forward<R0, R1, true>(xb, li, twx);
+            span_forward<R0>(xa, tw);
+            span_forward<R0>(xb, tw);
 #pragma unroll
             for (int j = 0; j < R0; ++j) row[swz(li + j * R1, N)] = pair4(xa[j], xb[j]);
         }
@@ -664,8 +680,10 @@ k_planes_vloc_p3x2(float2* __restrict__ work, const double* __restrict__ veff, i
                 xa[j] = lo2(v);
                 xb[j] = hi2(v);
             }
-            p2_span_forward<R0, R1, true>(xa, li, twy);
-            p2_span_forward<R0, R1, true>(xb, li, twy);
+            float2 tw[R0];
+            lane_tw<R0, R1>(tw, twy, li);
+            span_forward<R0>(xa, tw);
+            span_forward<R0>(xb, tw);
 #pragma unroll
             for (int j = 0; j < R0; ++j) line[swz(li + j * R1, N) * LS] = pair4(xa[j], xb[j]);
         }
@@ -680,10 +698,10 @@ k_planes_vloc_p3x2(float2* __restrict__ work, const double* __restrict__ veff, i
             }
             dft_r<R1, -1>(xa);
             dft_r<R1, -1>(xb);
-            const int* ci = g.colidx + (size_t)l * N + li * R1;
+            const int* ci = g.colidx_t + (size_t)li * R1 * nxact + l;
 #pragma unroll
             for (int m = 0; m < R1; ++m) {
-                const int c = __ldg(ci + m);
+                const int c = __ldg(ci + m * nxact);
                 if (c >= 0) {
                     wa[c] = xa[m];
                     if (two) wb[c] = xb[m];
@@ -799,7 +817,10 @@ k_zsticks_forward2(const C* __restrict__ work, const C* __restrict__ psi, int ld
         C x[R0];
 #pragma unroll
         for (int j = 0; j < R0; ++j) x[j] = lane < nl ? wb[(size_t)(j * R1) * g.ncol] : czero<C>();
-        p2_span_forward<R0, R1, false>(x, warp, ztable(g, C{}));
+        C tw[R0];
+#pragma unroll
+        for (int m = 1; m < R0; ++m) tw[m] = __ldg(ztable(g, C{}) + warp * m);
+        span_forward<R0>(x, tw);
 #pragma unroll
         for (int j = 0; j < R0; ++j) lines[(warp + j * R1) * 32 + (lane ^ (j & 7))] = x[j];
     }
@@ -1032,6 +1053,10 @@ int grid_for(size_t n, int threads) {
 #define CHFSI_ZPLANS32(X) X(9, 8) X(12, 9) X(8, 5) X(12, 12) X(8, 8) X(8, 6)
 #define CHFSI_ZPLANS64(X) CHFSI_ZPLANS32(X) X(6, 5) X(8, 4) X(6, 6) X(9, 5) X(10, 5) X(9, 6) X(10, 6) \
     X(15, 5) X(10, 8) X(9, 9) X(10, 9) X(12, 8) X(10, 10) X(12, 10)
+// planes up to 108 x 108 fit an SM's shared memory in 16-byte elements
+#define CHFSI_PLANES32(X) X(9, 8) X(12, 9) X(8, 5) X(8, 8) X(8, 6)
+#define CHFSI_PLANES64(X) CHFSI_PLANES32(X) X(6, 5) X(8, 4) X(6, 6) X(9, 5) X(10, 5) X(9, 6) X(10, 6) \
+    X(15, 5) X(10, 8) X(9, 9) X(10, 9) X(12, 8) X(10, 10)
 // clang-format on
 
 // The plan's key, and whether the kernels for it are built for C
@@ -1103,71 +1128,52 @@ void planes_vloc_variant(C* work, const double* veff, int nb, const HGeom& g, cu
     k_planes_vloc<C, V><<<grid, PlanesCfg<C, V>::threads, sm, st>>>(work, veff, g);
 }
 
-template <typename C, int V, int R0, int R1>
-void planes_vloc_p2(C* work, const double* veff, int nb, const HGeom& g, cudaStream_t st) {
-    dim3 grid(g.nz, nb);
-    size_t sm = planes_smem_bytes(g, sizeof(C));
-    if constexpr (sizeof(C) == 8) {
-        // FP32: two bands per CTA in 16-byte elements, where two such CTAs
-        // still fit one SM's shared memory (planes up to 80 x 80)
-        const size_t sm2 = 2 * align16<float2>(R0 * R1) +
-                           (size_t)R0 * R1 * ((R0 * R1) | 1) * sizeof(float4) +
-                           (size_t)g.nxact * sizeof(int);
-        if (g.colidx && R0 * R1 <= 256 && sm2 <= 112 * 1024) {
-            dim3 grid2(g.nz, (nb + 1) / 2);
-            allow_smem(k_planes_vloc_p3x2<V, R0, R1>, sm2);
-            k_planes_vloc_p3x2<V, R0, R1><<<grid2, PlanesCfg<double2, V>::threads, sm2, st>>>(
-                reinterpret_cast<float2*>(work), veff, nb, g);
-            return;
-        }
-    }
-    if (g.colidx && R0 * R1 <= 256) {
-        allow_smem(k_planes_vloc_p3<C, V, R0, R1>, sm);
-        k_planes_vloc_p3<C, V, R0, R1><<<grid, PlanesCfg<C, V>::threads, sm, st>>>(work, veff, g);
-        return;
-    }
-    allow_smem(k_planes_vloc_p2<C, V, R0, R1>, sm);
-    k_planes_vloc_p2<C, V, R0, R1><<<grid, PlanesCfg<C, V>::threads, sm, st>>>(work, veff, g);
+template <int V, int R0, int R1>
+void planes_vloc_x2(float2* work, const double* veff, int nb, const HGeom& g, cudaStream_t st) {
+    const size_t sm = 2 * align16<float2>(R0 * R1) + (size_t)R0 * R1 * ((R0 * R1) | 1) * sizeof(float4) +
+                      (size_t)g.nxact * sizeof(int);
+    allow_smem(k_planes_vloc_p3x2<V, R0, R1>, sm);
+    k_planes_vloc_p3x2<V, R0, R1><<<dim3(g.nz, (nb + 1) / 2), PlanesCfg<double2, V>::threads, sm, st>>>(
+        work, veff, nb, g);
 }
 
 template <typename C, int R0, int R1>
-void planes_vloc_p2_variant(C* work, const double* veff, int nb, const HGeom& g, cudaStream_t st) {
-    switch (g.tune_planes) {
-    case 1: planes_vloc_p2<C, 1, R0, R1>(work, veff, nb, g, st); break;
-    case 2: planes_vloc_p2<C, 2, R0, R1>(work, veff, nb, g, st); break;
-    default: planes_vloc_p2<C, 0, R0, R1>(work, veff, nb, g, st); break;
+void planes_vloc2_launch(C* work, const double* veff, int nb, const HGeom& g, cudaStream_t st) {
+    constexpr int NB = sizeof(C) == 8 ? 2 : 1;
+    using P = PlaneTwo<R0, R1>;
+    if constexpr (NB == 2 && P::fit >= 2) {
+        switch (g.tune_planes) {
+        case 1: planes_vloc_x2<1, R0, R1>(work, veff, nb, g, st); return;
+        case 2: planes_vloc_x2<2, R0, R1>(work, veff, nb, g, st); return;
+        default: planes_vloc_x2<0, R0, R1>(work, veff, nb, g, st); return;
+        }
     }
+    dim3 grid(g.nz, (nb + NB - 1) / NB);
+    allow_smem(k_planes_vloc2<C, NB, R0, R1>, P::bytes);
+    k_planes_vloc2<C, NB, R0, R1><<<grid, P::threads, P::bytes, st>>>(work, veff, nb, g);
 }
 
-// Radix pairs with a compile-time plane kernel (square planes only); other
-// plans run the generic kernel.
-static bool planes_vloc_fixed(void* work, const double* veff, int nb, const HGeom& g, cudaStream_t st,
-                       bool fp32) {
-    if (g.nx != g.ny || g.ax.nst != 2 || g.ay.nst != 2 || g.ax.r[0] != g.ay.r[0] ||
-        g.ax.r[1] != g.ay.r[1])
+// Square planes on a plan that is compiled in
+template <typename C>
+bool planes_vloc_fixed(C* work, const double* veff, int nb, const HGeom& g, cudaStream_t st) {
+    int key, ky;
+    if (!g.fixed_planes || !g.colidx_t || g.nx != g.ny || !two_radix<C>(g.ax, key) ||
+        !two_radix<C>(g.ay, ky) || key != ky)
         return false;
-    const int key = g.ax.r[0] * 100 + g.ax.r[1];
-#define CHFSI_P2(A, B)                                                                          \
-    case A * 100 + B:                                                                         \
-        if (fp32) planes_vloc_p2_variant<float2, A, B>((float2*)work, veff, nb, g, st);        \
-        else planes_vloc_p2_variant<double2, A, B>((double2*)work, veff, nb, g, st);           \
-        return true;
-    switch (key) {
-        CHFSI_P2(9, 8)    // 72
-        CHFSI_P2(12, 9)   // 108
-        CHFSI_P2(8, 5)    // 40
-        CHFSI_P2(12, 12)  // 144
-        CHFSI_P2(8, 8)    // 64
-        CHFSI_P2(8, 6)    // 48
-    default: return false;
+#define CHFSI_PV(A, B) case A * 100 + B: planes_vloc2_launch<C, A, B>(work, veff, nb, g, st); return true;
+    if constexpr (sizeof(C) == 16) {
+        switch (key) { CHFSI_PLANES64(CHFSI_PV) }
+    } else {
+        switch (key) { CHFSI_PLANES32(CHFSI_PV) }
     }
-#undef CHFSI_P2
+#undef CHFSI_PV
+    return false;
 }
 
 template <typename C>
 void launch_planes_vloc(C* work, const double* veff, int nb, const HGeom& g, cudaStream_t st) {
     count_launch();
-    if (g.fixed_planes && planes_vloc_fixed(work, veff, nb, g, st, sizeof(C) == 8)) return;
+    if (planes_vloc_fixed<C>(work, veff, nb, g, st)) return;
     switch (g.tune_planes) {
     case 1: planes_vloc_variant<C, 1>(work, veff, nb, g, st); break;
     case 2: planes_vloc_variant<C, 2>(work, veff, nb, g, st); break;

@@ -35,10 +35,12 @@ struct HGeom {
     // xy-plane kernels with compile-time radices where the plan has one
     // (square planes, two radices); 0 = always the generic kernel
     int fixed_planes = 1;
-    // direct column I/O of the compile-time plane kernel: colidx[l * ny + py]
-    // = column at (active x line l, digit-reversed y position py) or -1;
-    // xbits: bit px set when digit-reversed x position px carries columns
-    const int* colidx = nullptr;
+    // direct column I/O of the compile-time plane kernel: xline[l] = digit-
+    // reversed x position of active line l; colidx_t[py * nxact + l] = column at
+    // (digit-reversed y position py, line l) or -1; xbits: bit px set when
+    // digit-reversed x position px carries columns
+    const int* xline = nullptr;
+    const int* colidx_t = nullptr;
     unsigned int xbits[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 };
 
