@@ -548,6 +548,7 @@ struct chfsi_ctx {
     double* d_qvec = nullptr;     // Cartesian G + k per plane wave, 3 x n_pw
     int* d_atom_of_ion = nullptr;
     std::vector<int32_t> miller_ctx;  // Miller indices in the context's plane-wave order
+    double* d_rho_part = nullptr; // its partial sums over groups of bands
     double* d_rho_w = nullptr;    // smooth density on the wavefunction grid
     double2* d_wgrid = nullptr;   // wavefunction-grid complex scratch
     // ultrasoft augmentation Q_ij(r) = q_ij g(|r - R_I|)
@@ -1574,11 +1575,12 @@ chfsi_status density_dev(chfsi_ctx* ctx, double* rho) {
     cudaStream_t st = ctx->st;
     const bool direct = !ctx->fine && !ctx->aug;
     double* rw = direct ? rho : ctx->d_rho_w;
-    CK(cudaMemsetAsync(rw, 0, sizeof(double) * ctx->ng, st));
     if (nocc > 0) {
         launch_zsticks_inverse<double2>(ctx->d_psi, ctx->n_pw, ctx->d_work, nocc, ctx->geo, st);
-        launch_planes_density<double2>(ctx->d_work, ctx->d_occ, nocc, 1.0 / ctx->omega, rw,
-                                       ctx->geo, st);
+        launch_planes_density(ctx->d_work, ctx->d_occ, nocc, 1.0 / ctx->omega, rw, ctx->d_rho_part,
+                              ctx->geo, st);
+    } else {
+        CK(cudaMemsetAsync(rw, 0, sizeof(double) * ctx->ng, st));
     }
     if (direct) {
         CK(cudaGetLastError());
@@ -1740,6 +1742,12 @@ chfsi_status alloc_all(chfsi_ctx* ctx) {
     CK(dalloc(&ctx->d_pw_zpos, ctx->n_pw));
     CK(dalloc(&ctx->d_veff, ctx->ng));
     CK(dalloc(&ctx->d_rho_w, ctx->ng));
+    {
+        size_t groups = 1;
+        for (int n = 1; n <= ctx->nb; ++n)
+            groups = std::max(groups, (size_t)density_groups(ctx->nz, n));
+        CK(dalloc(&ctx->d_rho_part, groups * ctx->ng));
+    }
     CK(dalloc(&ctx->d_wgrid, ctx->ng));
     CK(dalloc(&ctx->d_minmax, 2));
     CK(dalloc(&ctx->d_psi, nbpw));
@@ -1827,7 +1835,7 @@ void free_all(chfsi_ctx* ctx) {
                   ctx->d_cgv, ctx->d_cgc, ctx->d_cgov, ctx->d_cgpart, ctx->d_cgdot, ctx->d_cgG,
                   ctx->d_psi_save, ctx->d_rc_hx, ctx->d_rc_y, ctx->d_rc_r0, ctx->d_rc_r1,
                   ctx->d_rc_y32, ctx->d_rc_coef, ctx->d_rc_lam, ctx->d_gga, ctx->d_gga_v1,
-                  ctx->d_ion, ctx->d_qvec, ctx->d_atom_of_ion, ctx->d_colidx, ctx->d_xline, ctx->d_bmatT,
+                  ctx->d_ion, ctx->d_qvec, ctx->d_atom_of_ion, ctx->d_colidx, ctx->d_xline, ctx->d_rho_part, ctx->d_bmatT,
                   ctx->d_i8, ctx->d_i8_beta};
     for (void* p : mp)
         if (p) cudaFree(p);

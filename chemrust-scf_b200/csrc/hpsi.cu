@@ -20,6 +20,7 @@
 #include "kernels.hpp"
 #include "launch_count.hpp"
 
+#include <algorithm>
 #include <cstdio>
 
 namespace chfsi {
@@ -272,7 +273,7 @@ template <int R0, int R1> struct PlaneTwo {
     // small planes (up to 50 x 50): a warp takes a group of lines through all its
     // stages, without block barriers between them
     static constexpr bool own = fit >= 5;
-    static constexpr int warps = own ? G : pick(), threads = 32 * warps;
+    static constexpr int shared_warps = pick(), warps = own ? G : shared_warps, threads = 32 * warps;
     static constexpr int by_regs = 65536 / (threads * 96);
     static constexpr int min_blocks = fit < by_regs ? fit : by_regs > 0 ? by_regs : 1;
     // place of x position p in a row
@@ -843,7 +844,7 @@ k_zsticks_forward2(const C* __restrict__ work, const C* __restrict__ psi, int ld
 template <typename C, int MAXPT>
 __global__ void __launch_bounds__(512)
 k_planes_density(const C* __restrict__ work, const double* __restrict__ occ, int nb, int bpg,
-                 double scale, double* rho, HGeom g) {
+                 double scale, double* part, HGeom g) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C* twx = reinterpret_cast<C*>(smem_raw);
     C* twy = reinterpret_cast<C*>(smem_raw + align16<C>(g.nx));
@@ -879,11 +880,124 @@ k_planes_density(const C* __restrict__ work, const double* __restrict__ occ, int
         }
         __syncthreads();
     }
-    double* rz = rho + (size_t)z * npl;
+    double* rz = part + ((size_t)blockIdx.y * g.nz + z) * npl;
 #pragma unroll
     for (int k = 0; k < MAXPT; ++k) {
         const int i = threadIdx.x + k * blockDim.x;
-        if (i < npl) atomicAdd(&rz[i], acc[k]);
+        if (i < npl) rz[i] = acc[k];
+    }
+}
+
+// Two-radix square planes: the inverse half of k_planes_vloc2 for each band of the
+// group, f |psi|^2 summed in the registers of the last x stage.  128 bands on 72^3:
+// 440 us, 959 with the generic kernel; 16 bands on 40^3: 20 and 58.  Bound as
+// k_planes_vloc2 is.  The parts are added by k_sum_parts (5 us).
+template <int R0, int R1>
+__global__ void __launch_bounds__(32 * PlaneTwo<R0, R1>::shared_warps, 1)
+k_planes_density2(const double2* __restrict__ work, const double* __restrict__ occ, int nb, int bpg,
+                  double scale, double* part, HGeom g) {
+    using P = PlaneTwo<R0, R1>;
+    constexpr int N = P::N, LS = P::LS, W = P::shared_warps, WS = W / P::Q1, kItems = (P::G + WS - 1) / WS;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double2* plane = reinterpret_cast<double2*>(smem_raw);
+    int* xl = reinterpret_cast<int*>(plane + (size_t)N * LS);
+    const int z = blockIdx.x, nxact = g.nxact;
+    const int b0 = blockIdx.y * bpg, b1 = min(b0 + bpg, nb);
+    for (int i = threadIdx.x; i < nxact; i += blockDim.x) xl[i] = P::at(g.xline[i]);
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane & 7, t = lane >> 3;
+    const int gy = (nxact + 7) >> 3, n1 = (warp % P::Q1) * 4 + t, gs = warp / P::Q1;
+    const double2* wt = g.twd_x;
+    double acc[kItems][R0];
+#pragma unroll
+    for (int k = 0; k < kItems; ++k)
+#pragma unroll
+        for (int j = 0; j < R0; ++j) acc[k][j] = 0.0;
+    for (int b = b0; b < b1; ++b) {
+        const double f = occ[b] * scale;
+        if (f == 0.0) continue;
+        const double2* wp = work + ((size_t)b * g.nz + z) * g.ncol;
+        for (int it = warp; it < gy * P::Q0; it += W) {
+            const int l = (it / P::Q0) * 8 + r, blk = (it % P::Q0) * 4 + t;
+            if (l >= nxact || blk >= R0) continue;
+            double2 x[R1];
+            const int* ci = g.colidx_t + (size_t)blk * R1 * nxact + l;
+#pragma unroll
+            for (int j = 0; j < R1; ++j) {
+                const int c = __ldg(ci + j * nxact);
+                x[j] = c >= 0 ? wp[c] : czero<double2>();
+            }
+            dft_r<R1, 1>(x);
+            double2* p = plane + (size_t)blk * R1 * LS + xl[l];
+#pragma unroll
+            for (int j = 0; j < R1; ++j) p[j * LS] = x[j];
+        }
+        __syncthreads();
+        for (int it = gs; it < gy; it += WS) {
+            const int l = it * 8 + r;
+            if (l >= nxact || n1 >= R1) continue;
+            double2 x[R0], tw[R0];
+            double2* p = plane + (size_t)n1 * LS + xl[l];
+#pragma unroll
+            for (int j = 0; j < R0; ++j) x[j] = p[j * R1 * LS];
+#pragma unroll
+            for (int m = 1; m < R0; ++m) tw[m] = __ldg(wt + n1 * m);
+            span_inverse<R0>(x, tw);
+#pragma unroll
+            for (int j = 0; j < R0; ++j) p[j * R1 * LS] = x[j];
+        }
+        __syncthreads();
+        for (int it = warp; it < P::G * P::Q0; it += W) {
+            const int y = (it / P::Q0) * 8 + r, blk = (it % P::Q0) * 4 + t;
+            if (y >= N || blk >= R0) continue;
+            double2 x[R1];
+            double2* row = plane + y * LS;
+#pragma unroll
+            for (int j = 0; j < R1; ++j) {
+                const int px = blk * R1 + j;
+                const bool on = (g.xbits[px >> 5] >> (px & 31)) & 1u;
+                x[j] = on ? row[P::at(px)] : czero<double2>();
+            }
+            dft_r<R1, 1>(x);
+#pragma unroll
+            for (int j = 0; j < R1; ++j) row[P::at(blk * R1 + j)] = x[j];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kItems; ++k) {
+            const int y = (gs + k * WS) * 8 + r;
+            if (y >= N || n1 >= R1) continue;
+            double2 x[R0], tw[R0];
+            const double2* row = plane + y * LS;
+#pragma unroll
+            for (int j = 0; j < R0; ++j) x[j] = row[P::at(n1 + j * R1)];
+#pragma unroll
+            for (int m = 1; m < R0; ++m) tw[m] = __ldg(wt + n1 * m);
+            span_inverse<R0>(x, tw);
+#pragma unroll
+            for (int j = 0; j < R0; ++j) acc[k][j] += f * (x[j].x * x[j].x + x[j].y * x[j].y);
+        }
+        __syncthreads();
+    }
+    double* rz = part + ((size_t)blockIdx.y * g.nz + z) * N * N;
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) {
+        const int y = (gs + k * WS) * 8 + r;
+        if (y >= N || n1 >= R1) continue;
+#pragma unroll
+        for (int j = 0; j < R0; ++j) rz[(size_t)y * N + n1 + j * R1] = acc[k][j];
+    }
+}
+
+// rho = sum of the band groups' parts, in group order (the same bits every time:
+// with atomics an SCF run that is restarted took another path at the level of
+// rounding, which the mixing amplifies)
+__global__ void k_sum_parts(const double* __restrict__ part, int groups, size_t n, double* __restrict__ rho) {
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
+         i += (size_t)gridDim.x * blockDim.x) {
+        double s = part[i];
+        for (int q = 1; q < groups; ++q) s += part[q * n + i];
+        rho[i] = s;
     }
 }
 
@@ -1232,19 +1346,41 @@ void launch_zsticks_forward(const C* work, const C* psi, int ldp, C* out, int ld
     }
 }
 
-template <typename C>
-void launch_planes_density(const C* work, const double* occ, int nb, double scale, double* rho,
-                           const HGeom& g, cudaStream_t st) {
-    count_launch();
-    int groups = (2 * 148 + g.nz - 1) / g.nz;
-    if (groups > nb) groups = nb;
-    if (groups < 1) groups = 1;
+int density_groups(int nz, int nb) {
+    const int groups = std::max(1, std::min(nb, (2 * 148 + nz - 1) / nz));
     const int bpg = (nb + groups - 1) / groups;
-    groups = (nb + bpg - 1) / bpg;
-    dim3 grid(g.nz, groups);
-    size_t sm = planes_smem_bytes(g, sizeof(C));
-    allow_smem(k_planes_density<C, 24>, sm);
-    k_planes_density<C, 24><<<grid, 512, sm, st>>>(work, occ, nb, bpg, scale, rho, g);
+    return (nb + bpg - 1) / bpg;
+}
+
+template <int R0, int R1>
+void planes_density2_launch(const double2* work, const double* occ, int nb, int bpg, int groups,
+                            double scale, double* part, const HGeom& g, cudaStream_t st) {
+    using P = PlaneTwo<R0, R1>;
+    allow_smem(k_planes_density2<R0, R1>, P::bytes);
+    k_planes_density2<R0, R1><<<dim3(g.nz, groups), 32 * P::shared_warps, P::bytes, st>>>(work, occ, nb, bpg, scale,
+                                                                                 part, g);
+}
+
+void launch_planes_density(const double2* work, const double* occ, int nb, double scale, double* rho,
+                           double* part, const HGeom& g, cudaStream_t st) {
+    count_launch(2);
+    const int groups = density_groups(g.nz, nb), bpg = (nb + groups - 1) / groups;
+    int key = 0, ky;
+    const bool fixed = g.colidx_t && g.nx == g.ny && two_radix<double2>(g.ax, key) &&
+                       two_radix<double2>(g.ay, ky) && key == ky;
+    switch (fixed ? key : 0) {
+#define CHFSI_PD(A, B) \
+    case A * 100 + B: planes_density2_launch<A, B>(work, occ, nb, bpg, groups, scale, part, g, st); break;
+        CHFSI_PLANES64(CHFSI_PD)
+#undef CHFSI_PD
+    default: {
+        const size_t sm = planes_smem_bytes(g, sizeof(double2));
+        allow_smem(k_planes_density<double2, 24>, sm);
+        k_planes_density<double2, 24><<<dim3(g.nz, groups), 512, sm, st>>>(work, occ, nb, bpg, scale, part, g);
+    }
+    }
+    const size_t n = (size_t)g.nx * g.ny * g.nz;
+    k_sum_parts<<<grid_for(n, 256), 256, 0, st>>>(part, groups, n, rho);
 }
 
 template <typename C>
@@ -1292,8 +1428,6 @@ void launch_energy_terms(const double* rho_out, const double* veff, const double
     template void launch_planes_vloc<C>(C*, const double*, int, const HGeom&, cudaStream_t);     \
     template void launch_zsticks_forward<C>(const C*, const C*, int, C*, int, int, const HGeom&, \
                                             const Epilogue&, cudaStream_t);                      \
-    template void launch_planes_density<C>(const C*, const double*, int, double, double*,        \
-                                           const HGeom&, cudaStream_t);                          \
     template void launch_axis_fft<C>(C*, int, int, int, int, bool, const AxisPlan&, cudaStream_t);
 CHFSI_INST(double2)
 CHFSI_INST(float2)

@@ -80,10 +80,11 @@ void launch_planes_vloc(C* work, const double* veff, int nb, const HGeom& g, cud
 template <typename C>
 void launch_zsticks_forward(const C* work, const C* psi, int ldp, C* out, int ldo, int nb,
                             const HGeom& g, const Epilogue& e, cudaStream_t st);
-// density: rho[r] += sum_b occ[b] |psi_b(r)|^2 * scale from inverse-z work.
-template <typename C>
-void launch_planes_density(const C* work, const double* occ, int nb, double scale, double* rho,
-                           const HGeom& g, cudaStream_t st);
+// density: rho[r] = sum_b occ[b] |psi_b(r)|^2 * scale from inverse-z work; part:
+// density_groups(nz, nb) partial grids
+int density_groups(int nz, int nb);
+void launch_planes_density(const double2* work, const double* occ, int nb, double scale, double* rho,
+                           double* part, const HGeom& g, cudaStream_t st);
 size_t planes_smem_bytes(const HGeom& g, size_t csize);
 
 // Full-grid 1D transforms along one axis (0 = x, 1 = y, 2 = z) of a

@@ -1,7 +1,7 @@
-"""Local H|psi> on every FFT plan with compile-time kernels and
+"""Local H|psi> and the density on every FFT plan with compile-time kernels and
 on grids that take the generic ones, against torch FFTs in 64 bits: columns of
 all lengths, plane-wave sets with holes and in any order, z axes on another plan
-than x and y, one band and odd counts.
+than x and y, one band and odd counts, occupations with zeros.
 
 Bound: a 3D FFT of N^3 points errs by a few 2^-53 log2(N^3) of the 2-norm; there
 and back 16 x 2^-53 x 21 = 4e-14 of each band's norm."""
@@ -79,3 +79,22 @@ def test_local_h_with_infinite_and_nan_bands(chfsi):
     torch.cuda.synchronize()
     ctx.apply_h_local(psi.data_ptr(), b.data_ptr(), 3)
     assert bool((a[[0, 2]] == b[[0, 2]]).all()) and bool(torch.isnan(b[1].real).all())
+
+
+@pytest.mark.parametrize("n", [30, 32, 36, 40, 45, 48, 50, 54, 60, 64, 72, 75, 80, 81, 90, 96, 100, 108, 27])
+def test_density(chfsi, n):
+    s = chfsi.SyntheticSystem(config_index=0, ecut=4.0, ngrid=[n] * 3, ngrid_density=[n] * 3, n_bands=23)
+    ctx = chfsi.Context(s)
+    occ = np.random.default_rng(n).random(23) * 2
+    occ[[1, 4, 5]] = 0.0
+    ctx.set_occupations(occ)
+    psi = s.psi0()
+    ctx.set_psi(psi)
+    rho = ctx.construct_density()
+    grid, _ = _grid(torch.from_numpy(psi).cuda(), s.miller(), (n, n, n))
+    ref = (torch.from_numpy(occ).cuda()[:, None, None, None] * grid.abs() ** 2).sum(0) / s.omega
+    ref = ref.reshape(-1).cpu().numpy()
+    assert np.linalg.norm(rho - ref) < TOL * np.linalg.norm(ref)
+    assert np.array_equal(rho, ctx.construct_density())
+    ctx.set_occupations(np.zeros(23))
+    assert not ctx.construct_density().any()
