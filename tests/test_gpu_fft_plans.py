@@ -98,3 +98,20 @@ def test_density(chfsi, n):
     assert np.array_equal(rho, ctx.construct_density())
     ctx.set_occupations(np.zeros(23))
     assert not ctx.construct_density().any()
+
+
+@pytest.mark.parametrize("at", [0, 31, 8192, 100003])
+def test_spectral_bound_sees_every_potential_value(chfsi, at):
+    """The filter's upper bound holds the potential's range, wherever its
+    extremes lie."""
+    n3 = (48, 48, 48)
+    m, kin = _basis(n3, 1, False)
+    ctx = chfsi.Context(dims={"ngrid": n3, "n_pw": len(m), "n_bands": 4})
+    ctx.set_basis(m, kin, 2.0)
+    v = np.zeros(48 ** 3)
+    v[at], v[-1] = 3.0, -2.0
+    ctx.set_veff(v)
+    rng = np.random.default_rng(2)
+    ctx.set_psi(rng.standard_normal((4, len(m))) + 1j * rng.standard_normal((4, len(m))))
+    ctx.chebyshev_filter(1)
+    assert abs(ctx.bounds()[0] - (2.0 + 5.0)) < 1e-13
