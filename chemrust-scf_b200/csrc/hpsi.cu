@@ -119,51 +119,87 @@ k_zsticks_inverse(const C* __restrict__ psi, int ldp, C* __restrict__ work, HGeo
 // (consecutive frequencies, a block apart) over the banks for the scatter and the
 // gather.  Against lane groups along each line (which spent 81 % of the
 // shared-memory wavefronts, 6.2 per access, half of them on twiddles and
-// conflicts), 160 bands on 72^3, us a launch: FP64 inverse 138 -> 125, H apply
-// 190 -> 120, Chebyshev step 227 -> 175; FP32 100 -> 53 and 195 -> 87.
+// conflicts), 160 bands on 72^3, us a launch, with the bands in turn below and the
+// epilogue's batches: FP64 inverse 138 -> 97, H apply 190 -> 109, Chebyshev step
+// 227 -> 128; FP32 100 -> 48 and 195 -> 85.
 template <int R0, int R1> struct ZTwo {
     static constexpr int N = R0 * R1, warps = R0 > R1 ? R0 : R1, threads = 32 * warps;
     static constexpr int min_blocks = 65536 / (80 * threads) > 0 ? 65536 / (80 * threads) : 1;
 };
 template <int R1> __device__ __forceinline__ int zslot(int p, int c) { return p * 32 + (c ^ ((p / R1) & 7)); }
 
+template <typename C> __device__ __forceinline__ void cp_async_elem(C* dst, const C* src) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    if constexpr (sizeof(C) == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
+}
+
+// A block takes the same columns of bpb bands.  With more than one band the plane
+// waves of the next are copied to a second buffer while this one is transformed:
+// with a band per block the pass waited for its loads (registers allow two or
+// three blocks an SM, DRAM was 35 % busy): 160 bands on 72^3 122 -> 97 us, 576 on
+// 108^3 1,654 -> 1,584.  The last stage leaves zeros behind for the band after the
+// next.
 template <typename C, int R0, int R1>
 __global__ void __launch_bounds__(ZTwo<R0, R1>::threads, ZTwo<R0, R1>::min_blocks)
-k_zsticks_inverse2(const C* __restrict__ psi, int ldp, C* __restrict__ work, HGeom g) {
-    constexpr int N = R0 * R1;
+k_zsticks_inverse2(const C* __restrict__ psi, int ldp, C* __restrict__ work, int nb, int bpb, HGeom g) {
+    constexpr int N = R0 * R1, kSlots = 4, T = ZTwo<R0, R1>::threads;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C* lines = reinterpret_cast<C*>(smem_raw);
-    const int b = blockIdx.y, c0 = blockIdx.x * 32, nl = min(32, g.ncol - c0);
+    const int b0 = blockIdx.y * bpb, b1 = min(b0 + bpb, nb);
+    const int c0 = blockIdx.x * 32, nl = min(32, g.ncol - c0);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int i = threadIdx.x; i < N * 32; i += blockDim.x) lines[i] = czero<C>();
-    __syncthreads();
-    const int g0 = g.col_start[c0], g1 = g.col_start[c0 + nl];
-    const C* pb = psi + (size_t)b * ldp;
-    for (int q = g0 + threadIdx.x; q < g1; q += blockDim.x)
-        lines[zslot<R1>(g.pw_zpos[q], g.pw_col[q] - c0)] = pb[q];
-    __syncthreads();
-    if (warp < R0) {
-        C* l = lines + warp * R1 * 32 + (lane ^ (warp & 7));
-        C x[R1];
+    for (int i = threadIdx.x; i < N * 32 * (bpb > 1 ? 2 : 1); i += T) lines[i] = czero<C>();
+    const int g0 = g.col_start[c0] + threadIdx.x, g1 = g.col_start[c0 + nl];
+    int slot[kSlots];
 #pragma unroll
-        for (int j = 0; j < R1; ++j) x[j] = l[j * 32];
-        dft_r<R1, 1>(x);
-#pragma unroll
-        for (int j = 0; j < R1; ++j) l[j * 32] = x[j];
+    for (int k = 0; k < kSlots; ++k) {
+        const int q = g0 + k * T;
+        slot[k] = q < g1 ? zslot<R1>(g.pw_zpos[q], g.pw_col[q] - c0) : 0;
     }
+    auto fetch = [&](C* dst, int b) {
+        const C* pb = psi + (size_t)b * ldp;
+#pragma unroll
+        for (int k = 0; k < kSlots; ++k)
+            if (g0 + k * T < g1) cp_async_elem(dst + slot[k], pb + g0 + k * T);
+        for (int q = g0 + kSlots * T; q < g1; q += T)
+            cp_async_elem(dst + zslot<R1>(g.pw_zpos[q], g.pw_col[q] - c0), pb + q);
+    };
     __syncthreads();
-    if (warp < R1) {
-        C x[R0];
+    fetch(lines, b0);
+    for (int b = b0; b < b1; ++b) {
+        C* cur = lines + ((b - b0) & 1) * N * 32;
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+        __syncthreads();
+        if (b + 1 < b1) fetch(lines + ((b + 1 - b0) & 1) * N * 32, b + 1);
+        if (warp < R0) {
+            C* l = cur + warp * R1 * 32 + (lane ^ (warp & 7));
+            C x[R1];
 #pragma unroll
-        for (int j = 0; j < R0; ++j) x[j] = lines[(warp + j * R1) * 32 + (lane ^ (j & 7))];
-        C tw[R0];
+            for (int j = 0; j < R1; ++j) x[j] = l[j * 32];
+            dft_r<R1, 1>(x);
 #pragma unroll
-        for (int m = 1; m < R0; ++m) tw[m] = __ldg(ztable(g, C{}) + warp * m);
-        span_inverse<R0>(x, tw);
-        C* wb = work + ((size_t)b * N + warp) * g.ncol + c0 + lane;
-        if (lane < nl)
+            for (int j = 0; j < R1; ++j) l[j * 32] = x[j];
+        }
+        __syncthreads();
+        if (warp < R1) {
+            C x[R0];
 #pragma unroll
-            for (int j = 0; j < R0; ++j) wb[(size_t)(j * R1) * g.ncol] = x[j];
+            for (int j = 0; j < R0; ++j) x[j] = cur[(warp + j * R1) * 32 + (lane ^ (j & 7))];
+            if (b + 2 < b1)
+#pragma unroll
+                for (int j = 0; j < R0; ++j) cur[(warp + j * R1) * 32 + (lane ^ (j & 7))] = czero<C>();
+            C tw[R0];
+#pragma unroll
+            for (int m = 1; m < R0; ++m) tw[m] = __ldg(ztable(g, C{}) + warp * m);
+            span_inverse<R0>(x, tw);
+            C* wb = work + ((size_t)b * N + warp) * g.ncol + c0 + lane;
+            if (lane < nl)
+#pragma unroll
+                for (int j = 0; j < R0; ++j) wb[(size_t)(j * R1) * g.ncol] = x[j];
+        }
     }
 }
 
@@ -746,32 +782,86 @@ __device__ __forceinline__ void z_epilogue(const C* lines, Slot slot, int c0, in
     const bool plain = b == e.plain_band;
     C* pob = plain ? reinterpret_cast<C*>(e.plain_out) : nullptr;
     double nacc = 0.0;
-    for (int q = g0 + threadIdx.x; q < g1; q += blockDim.x) {
-        const C v = lines[slot(g.pw_zpos[q], g.pw_col[q] - c0)];
-        const C p = pb[q];
-        const R k = (R)e.kin[q];
-        C h = mk(p.x * k, p.y * k);
-        h = mk(h.x + v.x * inv_n, h.y + v.y * inv_n);
-        if (nlb) h = cadd(h, nlb[q]);
-        if (plain) {
-            pob[q] = h;
-        } else if (MODE == kEpiApply) {
-            ob[q] = h;
-        } else if (MODE == kEpiResid) {
-            const C prev = ob[q];
-            const C y = yb[q];
-            ob[q] = mk(ra * h.x + rb * p.x + rcc * prev.x + rly * y.x,
-                       ra * h.y + rb * p.y + rcc * prev.y + rly * y.y);
-        } else {
-            C s = mk(h.x * ie + nc * p.x, h.y * ie + nc * p.y);
-            C o;
-            if (MODE == kEpiChebFirst) o = s;
-            else {
+    if constexpr (sizeof(C) == 8) {
+        // FP32 keeps one plane wave at a time: with the batches below the compiler
+        // contracts the sums the other way round, another rounding of the filtered
+        // bands (3e-8), for 1 % of a mixed pass
+        for (int q = g0 + threadIdx.x; q < g1; q += blockDim.x) {
+            const C v = lines[slot(g.pw_zpos[q], g.pw_col[q] - c0)];
+            const C p = pb[q];
+            const R k = (R)e.kin[q];
+            C h = mk(p.x * k, p.y * k);
+            h = mk(h.x + v.x * inv_n, h.y + v.y * inv_n);
+            if (nlb) h = cadd(h, nlb[q]);
+            if (plain) {
+                pob[q] = h;
+            } else if (MODE == kEpiApply) {
+                ob[q] = h;
+            } else if (MODE == kEpiResid) {
                 const C prev = ob[q];
-                o = mk((R)2 * s.x - prev.x, (R)2 * s.y - prev.y);
+                const C y = yb[q];
+                ob[q] = mk(ra * h.x + rb * p.x + rcc * prev.x + rly * y.x,
+                           ra * h.y + rb * p.y + rcc * prev.y + rly * y.y);
+            } else {
+                C s = mk(h.x * ie + nc * p.x, h.y * ie + nc * p.y);
+                C o;
+                if (MODE == kEpiChebFirst) o = s;
+                else {
+                    const C prev = ob[q];
+                    o = mk((R)2 * s.x - prev.x, (R)2 * s.y - prev.y);
+                }
+                ob[q] = o;
+                nacc += (double)o.x * (double)o.x + (double)o.y * (double)o.y;
             }
-            ob[q] = o;
-            nacc += (double)o.x * (double)o.x + (double)o.y * (double)o.y;
+        }
+        if (MODE != kEpiApply && e.norm_acc) {
+            double s = block_sum(nacc, red);
+            if (threadIdx.x == 0) atomicAdd(e.norm_acc, s);
+        }
+        return;
+    }
+    // the loads of kU plane waves before their arithmetic: one at a time, with
+    // `out` both read and written, each waits for the one before (160 bands on 72^3,
+    // Chebyshev step 172 -> 128 us)
+    constexpr int kU = MODE == kEpiResid ? 2 : 4;
+    for (int q0 = g0 + threadIdx.x; q0 < g1; q0 += kU * blockDim.x) {
+        C p[kU], nv[kU], prev[kU], y[kU];
+        R k[kU];
+        int at[kU];
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            const int q = q0 + u * blockDim.x;
+            if (q >= g1) continue;
+            p[u] = pb[q];
+            k[u] = (R)e.kin[q];
+            if (nlb) nv[u] = nlb[q];
+            if ((MODE == kEpiCheb || MODE == kEpiResid) && !plain) prev[u] = ob[q];
+            if (MODE == kEpiResid && !plain) y[u] = yb[q];
+            at[u] = slot(g.pw_zpos[q], g.pw_col[q] - c0);
+        }
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            const int q = q0 + u * blockDim.x;
+            if (q >= g1) continue;
+            const C v = lines[at[u]];
+            C h = mk(p[u].x * k[u], p[u].y * k[u]);
+            h = mk(h.x + v.x * inv_n, h.y + v.y * inv_n);
+            if (nlb) h = cadd(h, nv[u]);
+            if (plain) {
+                pob[q] = h;
+            } else if (MODE == kEpiApply) {
+                ob[q] = h;
+            } else if (MODE == kEpiResid) {
+                ob[q] = mk(ra * h.x + rb * p[u].x + rcc * prev[u].x + rly * y[u].x,
+                           ra * h.y + rb * p[u].y + rcc * prev[u].y + rly * y[u].y);
+            } else {
+                const C c = mk(h.x * ie + nc * p[u].x, h.y * ie + nc * p[u].y);
+                C o;
+                if (MODE == kEpiChebFirst) o = c;
+                else o = mk((R)2 * c.x - prev[u].x, (R)2 * c.y - prev[u].y);
+                ob[q] = o;
+                nacc += (double)o.x * (double)o.x + (double)o.y * (double)o.y;
+            }
         }
     }
     if (MODE != kEpiApply && e.norm_acc) {
@@ -1193,10 +1283,17 @@ template <typename C> bool two_radix(const AxisPlan& P, int& key) {
 
 template <typename C, int R0, int R1>
 void zsticks_inverse2_launch(const C* psi, int ldp, C* work, int nb, const HGeom& g, cudaStream_t st) {
-    dim3 grid((g.ncol + 31) / 32, nb);
-    const size_t sm = (size_t)R0 * R1 * 32 * sizeof(C);
+    // bands per block: as many as leave three waves of blocks, so that the last one
+    // stays short; one where two buffers a block would cost resident blocks
+    using Z = ZTwo<R0, R1>;
+    constexpr size_t buf = (size_t)R0 * R1 * 32 * sizeof(C);
+    constexpr bool two = Z::min_blocks * (2 * buf + 1024) <= 227 * 1024;
+    const int cg = (g.ncol + 31) / 32;
+    const int most = two ? (int)((long long)cg * nb / (3 * 148 * Z::min_blocks)) : 1;
+    const int bpb = most < 1 ? 1 : most > 16 ? 16 : most;
+    const size_t sm = bpb > 1 ? 2 * buf : buf;
     allow_smem(k_zsticks_inverse2<C, R0, R1>, sm);
-    k_zsticks_inverse2<C, R0, R1><<<grid, ZTwo<R0, R1>::threads, sm, st>>>(psi, ldp, work, g);
+    k_zsticks_inverse2<C, R0, R1><<<dim3(cg, (nb + bpb - 1) / bpb), Z::threads, sm, st>>>(psi, ldp, work, nb, bpb, g);
 }
 
 template <typename C, int COLS>

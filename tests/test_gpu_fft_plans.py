@@ -64,6 +64,41 @@ def test_local_h(chfsi, n3, holes):
         assert bool(torch.isnan(out[bands:].real).all())
 
 
+@pytest.mark.parametrize("n", [40, 64, 72, 100, 30])
+def test_local_h_many_bands(chfsi, n):
+    """Blocks of the inverse z pass that take several bands in turn, of columns
+    that fill the axis (more plane waves than a thread keeps places of)."""
+    h = np.arange(-9, 10)
+    x, y, z = np.meshgrid(h, h, np.arange(-((n - 1) // 2), (n - 1) // 2 + 1), indexing="ij")
+    on = x ** 2 + y ** 2 <= 90
+    m = np.stack([x[on], y[on], z[on]], axis=1).astype(np.int32)
+    m = np.ascontiguousarray(m[np.lexsort((m[:, 2], m[:, 0] % n, m[:, 1] % n))])  # device order
+    rng = np.random.default_rng(n)
+    kin, v, nb = rng.random(len(m)), rng.standard_normal(n ** 3), 322
+    ctx = chfsi.Context(dims={"ngrid": (n, n, n), "n_pw": len(m), "n_bands": nb})
+    ctx.set_basis(m, kin, 2.0)
+    ctx.set_veff(v)
+    gen = torch.Generator("cuda").manual_seed(n)
+    psi = torch.randn(nb, len(m), dtype=torch.complex128, device="cuda", generator=gen)
+    out = torch.full_like(psi, float("nan"))
+    torch.cuda.synchronize()
+    ctx.apply_h_local(psi.data_ptr(), out.data_ptr(), nb)
+    vr, kt = torch.from_numpy(v).cuda().view(n, n, n), torch.from_numpy(kin).cuda()
+    for b in range(0, nb, 46):
+        part = psi[b:b + 46]
+        grid, at = _grid(part, m, (n, n, n))
+        ref = torch.fft.fftn(grid * vr, dim=(1, 2, 3), norm="forward").reshape(len(part), -1)[:, at] + part * kt
+        err = torch.linalg.vector_norm(out[b:b + 46] - ref, dim=1)
+        scale = torch.linalg.vector_norm(ref, dim=1) + v.std() * torch.linalg.vector_norm(part, dim=1)
+        assert float((err / scale).max()) < TOL
+    one = torch.empty_like(psi[:1])
+    torch.cuda.synchronize()
+    for b in (0, 1, 2, nb - 1):
+        ctx.apply_h_local(psi[b:b + 1].data_ptr(), one.data_ptr(), 1)
+        torch.cuda.synchronize()
+        assert bool((one[0] == out[b]).all())
+
+
 def test_local_h_with_infinite_and_nan_bands(chfsi):
     """A band with an inf or NaN leaves the others alone."""
     n3 = (40, 40, 40)
