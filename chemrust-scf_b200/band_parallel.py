@@ -16,8 +16,8 @@ needs every band: it follows the reference's planned Row/Column design
   6. all-to-all back to the band split.
 
 The math of steps 2, 4 and 5 goes through an `ops` object: `DeviceOps` uses
-the library's own FP64 tensor-path GEMMs (chfsi_zgemm_cn / chfsi_zgemm_tn)
-and its Cholesky + Jacobi eigensolver (chfsi_hegv_dev) on CUDA tensors, the
+the library's own FP64 GEMMs (chfsi_zgemm_cn / chfsi_zgemm_tn) and its
+subspace eigensolver (chfsi_hegv_dev) on CUDA tensors, the
 collectives are NCCL.
 
 For the ultrasoft overlap S = 1 + beta q beta^H the subspace overlap is

@@ -3696,9 +3696,9 @@ extern "C" chfsi_status chfsi_batch_run(chfsi_batch* b, double* eig_out, int* st
 
 // Launch configurations of the local H|psi> for this context's sizes: the
 // xy-plane kernel at 128, 256 or 512 threads per block and the z-stick
-// kernels at 16, 32 or 64 columns per block, each with the compile-time plane
-// kernel (choices 0-8, where the grid has one) and with the generic one
-// (9-17), timed on the current psi (all bands); the fastest is kept.
+// kernels at 16, 32 or 64 columns per block, each with the compile-time
+// kernels (choices 0-8, where the grid has them; these fix their block shapes,
+// but for the FP32 planes) and with the generic ones (9-17), timed on the current psi (all bands); the fastest is kept.
 // times_ms (optional, kLaunchConfigs entries) gets every timing.
 constexpr int kLaunchConfigs = 18;
 static void apply_launch_config(chfsi_ctx* ctx, int i) {

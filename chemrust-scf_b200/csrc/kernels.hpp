@@ -29,7 +29,8 @@ struct HGeom {
     const float2* twf_x; const float2* twf_y; const float2* twf_z;
     // launch configuration chosen by chfsi_autotune: xy-plane kernel
     // 0 = 256 threads, 1 = 128 threads, 2 = 512 threads per block; z-stick
-    // kernels at tune_cols (16, 32, 64) columns per block
+    // kernels at tune_cols (16, 32, 64) columns per block; of the compile-time
+    // kernels only k_planes_vloc_p3x2 has the choice of block size
     int tune_planes = 0;
     int tune_cols = 32;
     // xy-plane kernels with compile-time radices where the plan has one

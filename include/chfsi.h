@@ -224,7 +224,9 @@ chfsi_status chfsi_set_qmat(chfsi_ctx* ctx, const chfsi_c128* qmat);
  * padding in G and V_eff is brought down by truncation
  * (downsample_array_to_wave_grid, src/scf.rs:413-454). */
 chfsi_status chfsi_set_density_grid(chfsi_ctx* ctx, const int* ngrid);
-/* Jacobi sweeps of the last Rayleigh-Ritz eigensolve (diagnostics). */
+/* Jacobi sweeps of the last Rayleigh-Ritz eigensolve (diagnostics): of its leaf
+ * problems, at most 24 rows, or of the whole matrix past the sizes of the
+ * divide-and-conquer solver. */
 chfsi_status chfsi_get_rr_sweeps(chfsi_ctx* ctx, int* sweeps);
 chfsi_status chfsi_get_density_grid(chfsi_ctx* ctx, int* ngrid);
 /* Ultrasoft augmentation: Q_ij(r) = q_ij g(|r - R_I|), g a unit Gaussian of
@@ -453,7 +455,9 @@ chfsi_status chfsi_batch_graph_nodes(chfsi_batch* b, size_t* nodes);
  * configurations (xy-plane kernel with compile-time radices where the grid's
  * plan has one, or the generic kernel; 256 / 128 / 512 threads per block;
  * z-stick kernels 16 / 32 / 64 columns per block) on its current psi and
- * keeps the fastest; choice = generic * 9 + planes * 3 + columns, times_ms
+ * keeps the fastest (the block shapes act on the generic kernels; the
+ * compile-time ones fix their own, except that of FP32 planes, which planes
+ * selects); choice = generic * 9 + planes * 3 + columns, times_ms
  * (18 floats) may be NULL.  chfsi_set_launch_config applies a choice (e.g.
  * one tuned per size class). */
 chfsi_status chfsi_autotune(chfsi_ctx* ctx, int* choice, float* times_ms);
@@ -504,7 +508,7 @@ chfsi_status chfsi_zgemm_tn(const chfsi_c128* w_dev, int ldw, const chfsi_c128* 
                             double beta, void* stream);
 /* Subspace eigenproblem H x = e S x (n x n, device, row-major), the ZHEGVD
  * itype-1 contract of src/device/solver.rs:47-95 solved by Cholesky
- * reduction and the library's Jacobi eigensolver: eigenvalues ascending to
+ * reduction and the library's Hermitian eigensolver: eigenvalues ascending to
  * w_host, eigenvectors as the columns of v_dev (V[j][i]).  Blocks until done. */
 chfsi_status chfsi_hegv_dev(const chfsi_c128* h_dev, const chfsi_c128* s_dev, int n,
                             double* w_host, chfsi_c128* v_dev, void* stream);
