@@ -326,7 +326,9 @@ k_tridiag(const double2* __restrict__ A, int n, int rows, double2* Vh, double2* 
     double2 alpha = A[1];  // x_{j+1}
     alpha.y = -alpha.y;
     double dj = A[0].x;
-    __syncthreads();
+    // a block's shared memory may be stored to only once the block runs
+    if constexpr (CL) cg::this_cluster().sync();
+    else __syncthreads();
     for (int j = 0; j < n - 1; ++j) {
         double2* Pj = (CL ? pl : P) + (size_t)(j & 1) * 2 * n;
         for (int l0 = 0; l0 < rows; l0 += rpp) {
