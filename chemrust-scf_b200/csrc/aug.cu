@@ -21,6 +21,7 @@
 
 #include "kernels.hpp"
 #include "launch_count.hpp"
+#include "smem_limit.hpp"
 
 namespace chfsi {
 namespace {
@@ -182,7 +183,7 @@ void launch_aug_add(double2* F, const GridRecip& gr, const double2* ph, const do
                     double width, double scale, cudaStream_t st) {
     count_launch();
     const size_t sm = (size_t)nions * sizeof(double2);
-    if (sm > 48 * 1024) cudaFuncSetAttribute(k_aug_add, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    raise_smem_limit(k_aug_add, sm);
     dim3 grid(gr.ny, gr.nz);
     k_aug_add<<<grid, 256, sm, st>>>(F, gr, ph, c, nions, width, scale);
 }

@@ -12,6 +12,7 @@
 // ordering, one cooperative launch) serves the sizes past those of heev().
 #include "dense.hpp"
 #include "launch_count.hpp"
+#include "smem_limit.hpp"
 
 #include <cooperative_groups.h>
 
@@ -516,8 +517,7 @@ cudaError_t jacobi(double2* A, double2* V, int n, int max_sweeps, double tol2, d
     const int warps_per_block = 8;
     int blocks = (npairs + warps_per_block - 1) / warps_per_block;
     const size_t smem = (size_t)warps_per_block * n * sizeof(double2);
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(k_jacobi2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (cudaError_t e = raise_smem_limit(k_jacobi2, smem)) return e;
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_jacobi2, 256, smem);
     if (per_sm < 1) per_sm = 1;

@@ -16,6 +16,7 @@
 #include <algorithm>
 #include "gemm.hpp"
 #include "launch_count.hpp"
+#include "smem_limit.hpp"
 
 namespace chfsi {
 
@@ -272,11 +273,8 @@ constexpr size_t kSmemCn = (size_t)kStages * (BM + BN) * kSK * sizeof(double2);
 constexpr size_t kSmemTn = (size_t)kStages * 2 * BK * kSM * sizeof(double2);
 
 void gemm_smem_setup() {
-    static bool done = false;
-    if (done) return;
-    cudaFuncSetAttribute(k_zgemm_cn_dmma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCn);
-    cudaFuncSetAttribute(k_zgemm_tn_dmma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemTn);
-    done = true;
+    raise_smem_limit(k_zgemm_cn_dmma, kSmemCn);
+    raise_smem_limit(k_zgemm_tn_dmma, kSmemTn);
 }
 
 // Hermitian product from its upper tiles: out[m][n] = sum of partials where

@@ -34,10 +34,10 @@
 #include "gemm_i8.hpp"
 #include "gemm.hpp"
 #include "launch_count.hpp"
+#include "smem_limit.hpp"
 #include "tcgen05.cuh"
 
 #include <algorithm>
-#include <mutex>
 
 namespace chfsi {
 
@@ -607,18 +607,6 @@ CnPlan cn_plan(int M, int N, int K, bool herm, int fixed_spc, size_t bytes) {
     return p;
 }
 
-cudaError_t i8_smem_setup() {
-    static std::once_flag once[64];
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-    std::call_once(once[dev], [] {
-        cudaFuncSetAttribute(k_umma_i8, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
-    });
-    return cudaSuccess;
-}
-
 I8Side side_of(const I8Operand& op, int slab0) {
     return {op.data, op.exps, op.tiles, op.tiles * op.tile, op.nslab, slab0, slab0 / op.spc};
 }
@@ -702,7 +690,7 @@ bool gemm_cn_i8(const double2* A, int lda, const I8Operand* pre, const double2* 
                 int N, int K, bool herm, void* scratch, size_t bytes, double2* out, int* err,
                 cudaStream_t st) {
     const CnPlan p = cn_plan(M, N, K, herm, pre ? pre->spc : 0, bytes);
-    if (p.groups == 0 || i8_smem_setup() != cudaSuccess) return false;
+    if (p.groups == 0 || raise_smem_limit(k_umma_i8, kSmemBytes) != cudaSuccess) return false;
     for (int g = 0; g < p.groups; ++g) {
         const int slab0 = g * p.slabs_per_group, k0 = slab0 * kSlab;
         if (slab0 >= p.nslab) break;
@@ -732,7 +720,7 @@ bool gemm_cn_i8(const double2* A, int lda, const I8Operand* pre, const double2* 
 bool gemm_tn_i8(const double2* W, int ldw, const double2* X, int ldx, const I8Operand* pre,
                 double2* O, int ldo, int M, int N, int K, double alpha, double beta, void* scratch,
                 size_t bytes, int* err, cudaStream_t st) {
-    if (K > kI8MaxK || i8_smem_setup() != cudaSuccess) return false;
+    if (K > kI8MaxK || raise_smem_limit(k_umma_i8, kSmemBytes) != cudaSuccess) return false;
     const int spc = ceil_div(K, kSlab), mt = ceil_div(M, kTN);
     const size_t wb = i8_operand_bytes(M, kTN, K, spc);
     // rows of X^T per group: what the rest of the scratch holds

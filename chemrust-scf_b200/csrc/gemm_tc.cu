@@ -30,6 +30,7 @@
 // TMEM and returns, so the context stays usable and the host reads the error.
 #include "gemm_tc.hpp"
 #include "launch_count.hpp"
+#include "smem_limit.hpp"
 #include "tcgen05.cuh"
 
 #include <cuda.h>
@@ -441,24 +442,6 @@ bool cached_map(CUtensorMap* m, const void* ptr, int rows, int kp, int box_rows,
     return true;
 }
 
-// Dynamic shared memory limit of a kernel, raised on a device only when a
-// launch needs more than it was last set to.
-std::mutex g_attr_mu;
-std::unordered_map<const void*, int> g_attr_smem[64];
-
-cudaError_t ensure_smem(const void* kernel, int bytes) {
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= 64) return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    std::lock_guard<std::mutex> lk(g_attr_mu);
-    int& have = g_attr_smem[dev][kernel];
-    if (have >= bytes) return cudaSuccess;
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess) have = bytes;
-    return e;
-}
-
 int pick_bn(int n, int cap) {
     const int tiles = (n + cap - 1) / cap;
     int bn = (n + tiles - 1) / tiles;
@@ -577,7 +560,7 @@ cudaError_t tc_gemm(const TcPlanes& a, const TcPlanes& b, int M, int N, int K, i
         }
     count_launch();
     auto launch = [&](auto kernel, void* dst, long long ld) {
-        ensure_smem((const void*)kernel, (int)sm);
+        raise_smem_limit((const void*)kernel, (int)sm);
         kernel<<<grid, kThreads, sm, st>>>(maps, 2 * M, N, bn, ktiles, kps, dst, ld, err, wait_ns,
                                            no_loads);
     };

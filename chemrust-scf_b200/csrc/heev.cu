@@ -22,6 +22,7 @@
 // LAPACK Working Note 89 (1994)) inside a bracket.
 #include "dense.hpp"
 #include "launch_count.hpp"
+#include "smem_limit.hpp"
 
 #include <algorithm>
 #include <cooperative_groups.h>
@@ -663,8 +664,7 @@ template <int NQ>
 cudaError_t launch_back(const double2* Vh, const double2* Tg, const double* Zt, int n, double2* U,
                         cudaStream_t st) {
     const size_t smem = (size_t)2 * kGrp * 32 * NQ * sizeof(double2);
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(k_back<NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (cudaError_t e = raise_smem_limit(k_back<NQ>, smem)) return e;
     k_back<NQ><<<(n + kBackWarps - 1) / kBackWarps, 32 * kBackWarps, smem, st>>>(Vh, Tg, Zt, n, U);
     return cudaGetLastError();
 }
@@ -1222,7 +1222,7 @@ int device_sms() {
 
 cudaError_t chol_inv(double2* A, double2* X, int n, int* info, cudaStream_t st) {
     const size_t smem = 4 * kCTile * sizeof(double2) + (size_t)n * sizeof(double);
-    cudaFuncSetAttribute(k_chol_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (cudaError_t e = raise_smem_limit(k_chol_inv, smem)) return e;
     const int nbk = (n + kCB - 1) / kCB;
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_chol_inv, 256, smem);
@@ -1277,7 +1277,7 @@ cudaError_t heev(const double2* A, int n, double* w, double2* U, double* scratch
     bool done = false;
     if (n <= kTriCluster) {
         const TriPlan p = tri_plan(n, std::min(16, (n + 3) / 4), TriCfg<true>::vectors);
-        cudaFuncSetAttribute(k_tridiag<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
+        raise_smem_limit(k_tridiag<true>, p.smem);
         cudaFuncSetAttribute(k_tridiag<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         cudaLaunchConfig_t lc = {};
         lc.gridDim = dim3(p.blocks);
@@ -1299,7 +1299,7 @@ cudaError_t heev(const double2* A, int n, double* w, double2* U, double* scratch
     }
     if (!done) {
         TriPlan p = tri_plan(n, std::min(device_sms(), std::max(1, (n + 3) / 4)), TriCfg<false>::vectors);
-        cudaFuncSetAttribute(k_tridiag<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
+        if ((e = raise_smem_limit(k_tridiag<false>, p.smem)) != cudaSuccess) return e;
         void* args[] = {&A, &n, &p.rows, &Vh, &tau, &q.d, &q.e, &P};
         e = cudaLaunchCooperativeKernel((const void*)k_tridiag<false>, dim3(p.blocks),
                                         dim3(TriCfg<false>::threads), args, p.smem, st);
@@ -1313,8 +1313,7 @@ cudaError_t heev(const double2* A, int n, double* w, double2* U, double* scratch
     for (int l = levels - 1; l >= 0; --l, par ^= 1) {
         const int most = (n >> l) + 1;
         const size_t smem = (size_t)most * (4 * sizeof(double) + 4 * sizeof(int));
-        if (smem > 48 * 1024)
-            cudaFuncSetAttribute(k_dc_deflate, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if ((e = raise_smem_limit(k_dc_deflate, smem)) != cudaSuccess) return e;
         k_dc_deflate<<<1 << l, 256, smem, st>>>(q, l, par);
         k_dc_secular<<<(n + 3) / 4, 128, 0, st>>>(q, l);
         k_dc_zhat<<<(n + 3) / 4, 128, 0, st>>>(q, l);

@@ -19,6 +19,7 @@
 // FFT/gather sequence.
 #include "kernels.hpp"
 #include "launch_count.hpp"
+#include "smem_limit.hpp"
 
 #include <algorithm>
 #include <cstdio>
@@ -1238,12 +1239,6 @@ k_energy_terms(const double* rho_out, const double* veff, const double* vloc, si
     if (threadIdx.x == 0) atomicAdd(dc_acc, s * dv);
 }
 
-// Opt a kernel into more than 48 KB of dynamic shared memory (once per
-// kernel and size class).
-template <typename K> void allow_smem(K kernel, size_t bytes) {
-    if (bytes > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
-
 int grid_for(size_t n, int threads) {
     size_t b = (n + threads - 1) / threads;
     return (int)(b < 148 * 8 ? b : 148 * 8);
@@ -1292,7 +1287,7 @@ void zsticks_inverse2_launch(const C* psi, int ldp, C* work, int nb, const HGeom
     const int most = two ? (int)((long long)cg * nb / (3 * 148 * Z::min_blocks)) : 1;
     const int bpb = most < 1 ? 1 : most > 16 ? 16 : most;
     const size_t sm = bpb > 1 ? 2 * buf : buf;
-    allow_smem(k_zsticks_inverse2<C, R0, R1>, sm);
+    raise_smem_limit(k_zsticks_inverse2<C, R0, R1>, sm);
     k_zsticks_inverse2<C, R0, R1><<<dim3(cg, (nb + bpb - 1) / bpb), Z::threads, sm, st>>>(psi, ldp, work, nb, bpb, g);
 }
 
@@ -1300,7 +1295,7 @@ template <typename C, int COLS>
 void zsticks_inverse_launch(const C* psi, int ldp, C* work, int nb, const HGeom& g, cudaStream_t st) {
     dim3 grid((g.ncol + COLS - 1) / COLS, nb);
     size_t sm = align16<C>(g.nz) + (size_t)COLS * g.lsz * sizeof(C);
-    allow_smem(k_zsticks_inverse<C, COLS>, sm);
+    raise_smem_limit(k_zsticks_inverse<C, COLS>, sm);
     k_zsticks_inverse<C, COLS><<<grid, 256, sm, st>>>(psi, ldp, work, g);
 }
 
@@ -1335,7 +1330,7 @@ template <typename C, int V>
 void planes_vloc_variant(C* work, const double* veff, int nb, const HGeom& g, cudaStream_t st) {
     dim3 grid(g.nz, nb);
     size_t sm = planes_smem_bytes(g, sizeof(C));
-    allow_smem(k_planes_vloc<C, V>, sm);
+    raise_smem_limit(k_planes_vloc<C, V>, sm);
     k_planes_vloc<C, V><<<grid, PlanesCfg<C, V>::threads, sm, st>>>(work, veff, g);
 }
 
@@ -1343,7 +1338,7 @@ template <int V, int R0, int R1>
 void planes_vloc_x2(float2* work, const double* veff, int nb, const HGeom& g, cudaStream_t st) {
     const size_t sm = 2 * align16<float2>(R0 * R1) + (size_t)R0 * R1 * ((R0 * R1) | 1) * sizeof(float4) +
                       (size_t)g.nxact * sizeof(int);
-    allow_smem(k_planes_vloc_p3x2<V, R0, R1>, sm);
+    raise_smem_limit(k_planes_vloc_p3x2<V, R0, R1>, sm);
     k_planes_vloc_p3x2<V, R0, R1><<<dim3(g.nz, (nb + 1) / 2), PlanesCfg<double2, V>::threads, sm, st>>>(
         work, veff, nb, g);
 }
@@ -1360,7 +1355,7 @@ void planes_vloc2_launch(C* work, const double* veff, int nb, const HGeom& g, cu
         }
     }
     dim3 grid(g.nz, (nb + NB - 1) / NB);
-    allow_smem(k_planes_vloc2<C, NB, R0, R1>, P::bytes);
+    raise_smem_limit(k_planes_vloc2<C, NB, R0, R1>, P::bytes);
     k_planes_vloc2<C, NB, R0, R1><<<grid, P::threads, P::bytes, st>>>(work, veff, nb, g);
 }
 
@@ -1397,7 +1392,7 @@ void zsticks_forward2_launch(const C* work, const C* psi, int ldp, C* out, int l
                              const HGeom& g, const Epilogue& e, cudaStream_t st) {
     dim3 grid((g.ncol + 31) / 32, nb);
     const size_t sm = (size_t)R0 * R1 * 32 * sizeof(C);
-    allow_smem(k_zsticks_forward2<C, MODE, R0, R1>, sm);
+    raise_smem_limit(k_zsticks_forward2<C, MODE, R0, R1>, sm);
     k_zsticks_forward2<C, MODE, R0, R1><<<grid, ZTwo<R0, R1>::threads, sm, st>>>(work, psi, ldp, out, ldo,
                                                                               g, e);
 }
@@ -1407,7 +1402,7 @@ void zsticks_forward_launch(const C* work, const C* psi, int ldp, C* out, int ld
                             const HGeom& g, const Epilogue& e, cudaStream_t st) {
     dim3 grid((g.ncol + COLS - 1) / COLS, nb);
     size_t sm = align16<C>(g.nz) + (size_t)COLS * g.lsz * sizeof(C);
-    allow_smem(k_zsticks_forward<C, MODE, COLS>, sm);
+    raise_smem_limit(k_zsticks_forward<C, MODE, COLS>, sm);
     k_zsticks_forward<C, MODE, COLS><<<grid, 256, sm, st>>>(work, psi, ldp, out, ldo, g, e);
 }
 
@@ -1453,7 +1448,7 @@ template <int R0, int R1>
 void planes_density2_launch(const double2* work, const double* occ, int nb, int bpg, int groups,
                             double scale, double* part, const HGeom& g, cudaStream_t st) {
     using P = PlaneTwo<R0, R1>;
-    allow_smem(k_planes_density2<R0, R1>, P::bytes);
+    raise_smem_limit(k_planes_density2<R0, R1>, P::bytes);
     k_planes_density2<R0, R1><<<dim3(g.nz, groups), 32 * P::shared_warps, P::bytes, st>>>(work, occ, nb, bpg, scale,
                                                                                  part, g);
 }
@@ -1472,7 +1467,7 @@ void launch_planes_density(const double2* work, const double* occ, int nb, doubl
 #undef CHFSI_PD
     default: {
         const size_t sm = planes_smem_bytes(g, sizeof(double2));
-        allow_smem(k_planes_density<double2, 24>, sm);
+        raise_smem_limit(k_planes_density<double2, 24>, sm);
         k_planes_density<double2, 24><<<dim3(g.nz, groups), 512, sm, st>>>(work, occ, nb, bpg, scale, part, g);
     }
     }
@@ -1489,8 +1484,8 @@ void launch_axis_fft(C* data, int nx, int ny, int nz, int axis, bool forward, co
     if (axis == 0) blocks = (ny * nz + lb - 1) / lb;
     else blocks = ((nx + lb - 1) / lb) * (axis == 1 ? nz : ny);
     size_t sm = align16<C>(P.n) + (size_t)lb * (P.n | 1) * sizeof(C);
-    allow_smem(k_axis_fft<C, true>, sm);
-    allow_smem(k_axis_fft<C, false>, sm);
+    raise_smem_limit(k_axis_fft<C, true>, sm);
+    raise_smem_limit(k_axis_fft<C, false>, sm);
     if (forward) k_axis_fft<C, true><<<blocks, 256, sm, st>>>(data, nx, ny, nz, axis, P, lb);
     else k_axis_fft<C, false><<<blocks, 256, sm, st>>>(data, nx, ny, nz, axis, P, lb);
 }
