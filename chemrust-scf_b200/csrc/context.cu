@@ -517,7 +517,7 @@ struct chfsi_ctx {
     // per projector set; scratch for the other operands; error word in mapped
     // host memory, read after each synchronisation
     I8Operand i8_beta, i8_betaT;
-    void* d_i8_beta = nullptr; void* d_i8 = nullptr; size_t i8_bytes = 0;
+    char* d_i8_beta = nullptr; char* d_i8 = nullptr; size_t i8_bytes = 0;
     int* h_i8_err = nullptr;
     bool beta_planes_ready = false;
     // tcgen05 launch shapes of the projection and the expansion (-1: time
@@ -643,13 +643,17 @@ void alloc_i8(chfsi_ctx* ctx) {
     if (np > 0 && i8_tn_pays(np, nb, np, false)) need = std::max(need, i8_tn_scratch_bytes(np, nb, np, false));
     if (need == 0) return;
     need = std::min(need, kI8Scratch);
-    if (cudaHostAlloc((void**)&ctx->h_i8_err, sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
-        cudaMalloc(&ctx->d_i8, need) != cudaSuccess) {
+    if (cudaHostAlloc((void**)&ctx->h_i8_err, sizeof(int), cudaHostAllocMapped) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->h_i8_err = nullptr;
+        return;
+    }
+    *ctx->h_i8_err = 0;  // read after every synchronisation, scratch or not
+    if (dalloc(&ctx->d_i8, need) != cudaSuccess) {
         cudaGetLastError();
         ctx->d_i8 = nullptr;
         return;
     }
-    *ctx->h_i8_err = 0;
     ctx->i8_bytes = need;
 }
 
@@ -666,7 +670,7 @@ void cut_beta(chfsi_ctx* ctx) {
     const size_t ba = rows ? i8_operand_bytes(np, kI8RowTile, npw, spc) : 0;
     const size_t bt = cols ? i8_operand_bytes(npw, kI8RowTile, np, spcT) : 0;
     if (ba + bt == 0) return;
-    if (cudaMalloc(&ctx->d_i8_beta, ba + bt) != cudaSuccess) {
+    if (dalloc(&ctx->d_i8_beta, ba + bt) != cudaSuccess) {
         cudaGetLastError();
         ctx->d_i8_beta = nullptr;
         return;
@@ -676,7 +680,7 @@ void cut_beta(chfsi_ctx* ctx) {
         i8_slice(ctx->d_beta, npw, false, -1, ctx->i8_beta, ctx->st);
     }
     if (cols) {
-        i8_operand_place(ctx->i8_betaT, (char*)ctx->d_i8_beta + ba, npw, kI8RowTile, np, spcT);
+        i8_operand_place(ctx->i8_betaT, ctx->d_i8_beta + ba, npw, kI8RowTile, np, spcT);
         i8_slice(ctx->d_beta, npw, true, 1, ctx->i8_betaT, ctx->st);
     }
 }

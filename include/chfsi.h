@@ -521,7 +521,8 @@ chfsi_status chfsi_hpsi_device_ptr(chfsi_ctx* ctx, chfsi_c128** out);
  *   a producer that issues no loads; the consumer's wait runs out after 20 ms
  *   and the call returns CHFSI_ERR_TIMEOUT (no GPU fault, nothing in flight).
  * CHFSI_INJECT_ALLOC_FAIL: the arg-th device allocation of a context from now
- *   (0 = the next) fails as out of memory.
+ *   (0 = the next) fails as out of memory.  The INT8 scratch and the projector
+ *   digits are counted too; a context works without them.
  * CHFSI_INJECT_NONE clears both. */
 enum { CHFSI_INJECT_NONE = 0, CHFSI_INJECT_TC_NO_LOADS = 1, CHFSI_INJECT_ALLOC_FAIL = 2 };
 chfsi_status chfsi_test_inject(int what, long long arg);

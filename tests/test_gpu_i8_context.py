@@ -1,0 +1,95 @@
+"""The INT8 products of a context (digits of the projectors, scratch and error
+word beside its FP64 buffers) when something about them fails or changes: memory
+that is not to be had, waits that run out, projectors set anew.  The FP64 tensor
+path computes the same products, so each case is compared with a context that
+nothing happened to.
+
+Bound: H psi of unit-norm bands, two ways of summing the same FP64 products: K
+terms each at most |beta||psi| in sum, 64 2^-52 of the largest |H psi| holds it
+with room (the products themselves are compared in test_gpu_i8_gemm.py)."""
+import ctypes
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+TOL = 64 * 2.0 ** -52
+
+
+@pytest.fixture(scope="module")
+def sys_kb(chfsi):
+    # 64-atom supercell at a low cutoff: projections and expansions on INT8
+    return chfsi.SyntheticSystem(config_index=0, n_rep=2, ngrid=[45] * 3, ngrid_density=[45] * 3,
+                                 ecut=8.0, n_bands=160, n_shell=1, lmax=1,
+                                 rc_proj=[1.2, 1.4, 0, 0], d_min=0.5, d_max=2.0)
+
+
+@pytest.fixture(autouse=True)
+def _clear(chfsi):
+    yield
+    chfsi.inject_fault(chfsi.INJECT_NONE)
+
+
+def _psi(s, nb=None):
+    g = torch.Generator(device="cuda").manual_seed(3)
+    psi = torch.view_as_complex(torch.randn(nb or s.n_bands, s.n_pw, 2, generator=g, device="cuda",
+                                            dtype=torch.float64))
+    return psi / torch.linalg.vector_norm(psi, dim=1, keepdim=True)
+
+
+def _apply_h(ctx, psi):
+    out = torch.full_like(psi, float("nan"))
+    torch.cuda.synchronize()
+    ctx.apply_h(psi.data_ptr(), out.data_ptr(), len(psi))
+    return out
+
+
+def _context(chfsi, s, **kw):
+    ctx = chfsi.Context(s, **kw)
+    ctx.set_veff(ctx.get_vloc())
+    return ctx
+
+
+def _same(a, b):
+    return float((a - b).abs().max()) <= TOL * float(b.abs().max())
+
+
+def test_context_without_the_scratch(chfsi, sys_kb):
+    """The scratch is the one allocation of a creation that may fail: what was
+    asked for still runs, and its status does not come from memory that the
+    process gave back before (the error word is mapped host memory)."""
+    rt = ctypes.CDLL("libcudart.so.12")
+    dirty = []
+    for _ in range(64):
+        p = ctypes.c_void_p()
+        assert rt.cudaHostAlloc(ctypes.byref(p), ctypes.c_size_t(4), 2) == 0
+        ctypes.cast(p, ctypes.POINTER(ctypes.c_int))[0] = 7
+        dirty.append(p)
+    for p in dirty:
+        rt.cudaFreeHost(p)
+    psi = _psi(sys_kb)
+    ref = _apply_h(_context(chfsi, sys_kb), psi)
+    dims = {"ngrid": list(sys_kb.ngrid), "n_pw": sys_kb.n_pw, "n_bands": sys_kb.n_bands,
+            "n_proj": sys_kb.n_proj, "n_ions": sys_kb.n_ions}
+    made = []
+    for nth in range(200):
+        chfsi.inject_fault(chfsi.INJECT_ALLOC_FAIL, nth)
+        try:
+            chfsi.Context(dims=dims)
+            made.append(nth)
+        except chfsi.OutOfMemory:
+            pass
+        chfsi.inject_fault(chfsi.INJECT_NONE)
+        if made[-3:] == [nth - 2, nth - 1, nth]:
+            break  # past the last allocation
+    optional = [k for k in made if k < nth - 2]
+    assert len(optional) == 1
+    chfsi.inject_fault(chfsi.INJECT_ALLOC_FAIL, optional[0])
+    ctx = chfsi.Context(sys_kb)
+    chfsi.inject_fault(chfsi.INJECT_NONE)
+    ctx.set_veff(ctx.get_vloc())
+    out = _apply_h(ctx, psi)
+    assert _same(out, ref)
+    assert not bool((out == ref).all())  # the other path did compute it
