@@ -26,7 +26,7 @@ LIB_PATH = os.path.join(HERE, "libchfsi_b200.so")
 
 OK, NOT_CONVERGED, NOT_IMPLEMENTED, CHEB_DIVERGED, RR_FAILED, CUDA_ERROR, BAD_INPUT, \
     NO_DEVICE, OUT_OF_MEMORY, NUMERIC, TIMEOUT = 0, -1, -2, -3, -4, -5, -6, -7, -8, -9, -10
-INJECT_NONE, INJECT_TC_NO_LOADS, INJECT_ALLOC_FAIL = 0, 1, 2
+INJECT_NONE, INJECT_TC_NO_LOADS, INJECT_ALLOC_FAIL, INJECT_I8_NO_LOADS = 0, 1, 2, 3
 PREC_FP64, PREC_MIXED = 0, 1
 BOUND_HEURISTIC, BOUND_LANCZOS, BOUND_LANCZOS_FUSED = 0, 1, 2
 FILTER_CHEBYSHEV, FILTER_RESIDUAL = 0, 1
@@ -385,8 +385,9 @@ def zgemm_cn_bf16x3(a_dev, lda, b_dev, ldb, m, n, k, c_dev, stream=0, shape=None
 
 def inject_fault(what, arg=0):
     """Host-side fault injection for error-path tests (INJECT_TC_NO_LOADS:
-    the next `arg` tensor-core GEMM launches issue no loads and time out;
-    INJECT_ALLOC_FAIL: the arg-th device allocation fails; INJECT_NONE clears)."""
+    the next `arg` BF16 tensor-core GEMM launches issue no loads and time out;
+    INJECT_I8_NO_LOADS: the arg-th INT8 GEMM launch does; INJECT_ALLOC_FAIL: the
+    arg-th device allocation fails; INJECT_NONE clears)."""
     _check(lib().chfsi_test_inject(what, arg))
 
 

@@ -1440,11 +1440,9 @@ chfsi_status finish_diag(chfsi_ctx* ctx, double* eig_out, bool have_rr) {
     if (ctx->d_tc_err)
         CK(cudaMemcpyAsync(&tc_err, ctx->d_tc_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
+    if (tc_err) CK(cudaMemsetAsync(ctx->d_tc_err, 0, sizeof(int), ctx->st));
     if (chfsi_status e = i8_status(ctx)) return e;
-    if (tc_err) {
-        CK(cudaMemsetAsync(ctx->d_tc_err, 0, sizeof(int), ctx->st));
-        return ctx->fail(CHFSI_ERR_TIMEOUT, "tensor-core GEMM pipeline wait timed out");
-    }
+    if (tc_err) return ctx->fail(CHFSI_ERR_TIMEOUT, "tensor-core GEMM pipeline wait timed out");
     std::memcpy(ctx->h_coef, h + n, sizeof(double) * 6);
     int flags[4];
     std::memcpy(flags, h + n + 6, sizeof(flags));
@@ -4063,6 +4061,7 @@ extern "C" chfsi_status chfsi_test_inject(int what, long long arg) {
     switch (what) {
         case CHFSI_INJECT_NONE:
             tc_inject_no_loads(0);
+            i8_inject_no_loads(-1);
             g_alloc_fail_in.store(-1);
             return CHFSI_OK;
         case CHFSI_INJECT_TC_NO_LOADS:
@@ -4071,6 +4070,9 @@ extern "C" chfsi_status chfsi_test_inject(int what, long long arg) {
             return CHFSI_OK;
         case CHFSI_INJECT_ALLOC_FAIL:
             g_alloc_fail_in.store(arg < 0 ? -1 : arg);
+            return CHFSI_OK;
+        case CHFSI_INJECT_I8_NO_LOADS:
+            i8_inject_no_loads(arg);
             return CHFSI_OK;
         default:
             return CHFSI_ERR_BAD_INPUT;

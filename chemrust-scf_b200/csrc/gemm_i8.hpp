@@ -59,4 +59,8 @@ bool gemm_tn_i8(const double2* W, int ldw, const double2* X, int ldx, const I8Op
                 double2* O, int ldo, int M, int N, int K, double alpha, double beta, void* scratch,
                 size_t bytes, int* err, cudaStream_t st);
 
+// Test hook: the launch that is `launches` from now (0: the next; negative:
+// none) copies no operands, so that its waits run out.
+void i8_inject_no_loads(long long launches);
+
 }  // namespace chfsi

@@ -517,14 +517,21 @@ chfsi_status chfsi_hegv_dev(const chfsi_c128* h_dev, const chfsi_c128* s_dev, in
 chfsi_status chfsi_hpsi_device_ptr(chfsi_ctx* ctx, chfsi_c128** out);
 
 /* ---- test hooks (host-side fault injection; no counterpart in the crate) --
- * CHFSI_INJECT_TC_NO_LOADS: the next `arg` tensor-core GEMM launches run with
- *   a producer that issues no loads; the consumer's wait runs out after 20 ms
+ * CHFSI_INJECT_TC_NO_LOADS: the next `arg` launches of the BF16 tensor-core GEMM
+ *   (mixed precision, chfsi_zgemm_cn_bf16x3) run with a producer that issues no loads; the consumer's wait runs out after 20 ms
  *   and the call returns CHFSI_ERR_TIMEOUT (no GPU fault, nothing in flight).
  * CHFSI_INJECT_ALLOC_FAIL: the arg-th device allocation of a context from now
  *   (0 = the next) fails as out of memory.  The INT8 scratch and the projector
  *   digits are counted too; a context works without them.
- * CHFSI_INJECT_NONE clears both. */
-enum { CHFSI_INJECT_NONE = 0, CHFSI_INJECT_TC_NO_LOADS = 1, CHFSI_INJECT_ALLOC_FAIL = 2 };
+ * CHFSI_INJECT_I8_NO_LOADS: the same for the arg-th launch from now (0 = the
+ *   next) of the INT8 tensor-core GEMM that FP64 products are computed with.
+ * CHFSI_INJECT_NONE clears all. */
+enum {
+    CHFSI_INJECT_NONE = 0,
+    CHFSI_INJECT_TC_NO_LOADS = 1,
+    CHFSI_INJECT_ALLOC_FAIL = 2,
+    CHFSI_INJECT_I8_NO_LOADS = 3
+};
 chfsi_status chfsi_test_inject(int what, long long arg);
 
 #ifdef __cplusplus

@@ -93,3 +93,35 @@ def test_context_without_the_scratch(chfsi, sys_kb):
     out = _apply_h(ctx, psi)
     assert _same(out, ref)
     assert not bool((out == ref).all())  # the other path did compute it
+
+
+def _operands(m, n, k):
+    g = torch.Generator(device="cuda").manual_seed(m)
+    a, b, o = [torch.view_as_complex(torch.randn(*shape, 2, generator=g, device="cuda", dtype=torch.float64))
+               for shape in ((m, k), (n, k), (m, n))]
+    torch.cuda.synchronize()
+    return a, b, o
+
+
+def test_products_report_a_wait_that_ran_out(chfsi):
+    m, n, k = 256, 160, 20000
+    a, b, c = _operands(m, n, k)
+    args = (a.data_ptr(), k, b.data_ptr(), k, m, n, k, c.data_ptr())
+    chfsi.zgemm_cn(*args)
+    ref = c.clone()
+    chfsi.inject_fault(chfsi.INJECT_I8_NO_LOADS, 0)
+    with pytest.raises(chfsi.Timeout, match="timed out"):
+        chfsi.zgemm_cn(*args)
+    chfsi.zgemm_cn(*args)
+    assert bool((c == ref).all())
+    m, n, k = 160, 20000, 256
+    w, x = _operands(k, 1, m)[0], _operands(k, 1, n)[0]
+    o = torch.empty(m, n, dtype=torch.complex128, device="cuda")
+    args = (w.data_ptr(), m, x.data_ptr(), n, o.data_ptr(), n, m, n, k)
+    chfsi.zgemm_tn(*args)
+    ref = o.clone()
+    chfsi.inject_fault(chfsi.INJECT_I8_NO_LOADS, 0)
+    with pytest.raises(chfsi.Timeout, match="timed out"):
+        chfsi.zgemm_tn(*args)
+    chfsi.zgemm_tn(*args)
+    assert bool((o == ref).all())
