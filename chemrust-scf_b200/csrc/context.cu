@@ -2155,6 +2155,7 @@ chfsi_status band_cg_dev(chfsi_ctx* ctx, int max_steps, double tol, double* eig,
     }
     CK(cudaStreamSynchronize(ctx->st));
     CK(cudaGetLastError());
+    if ((st = i8_status(ctx))) return st;
     if (n_conv) *n_conv = nconv;
     return CHFSI_OK;
 }
@@ -3111,6 +3112,7 @@ extern "C" chfsi_status chfsi_scf_run(chfsi_ctx* ctx, const chfsi_scf_params* p,
         double acc[3];
         CK(cudaMemcpyAsync(acc, ctx->d_acc, sizeof(acc), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
+        if ((s = i8_status(ctx))) { status = s; break; }  // the projections of the density
         double eband = 0.0;
         for (int b = 0; b < ctx->nb; ++b) eband += ctx->occ[b] * eig[b];
         const double etot = eband - acc[2] + acc[0] + acc[1] + ctx->e_ewald + e_ts;
