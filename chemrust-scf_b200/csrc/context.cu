@@ -556,6 +556,9 @@ struct chfsi_ctx {
     std::vector<double> ion_pos;  // ions with projectors, x 3 (bohr)
     double2* d_phase = nullptr;   // per ion e^{-i 2 pi f_d h}: [ion][fnx | fny | fnz]
     double2* d_dmat0 = nullptr;   // unscreened D
+    size_t n_dmat = 0;            // elements of d_dmat and d_dmat0
+    // counts the changes of buffers whose addresses a captured pass holds
+    unsigned layout = 0;
     double* d_cion = nullptr;     // per ion sum_n f_n C^H q C
     double* d_vion = nullptr;     // per ion int V_eff g(r - R_I)
     // learned density mixer (G-space residual history on the density grid)
@@ -658,10 +661,9 @@ void alloc_i8(chfsi_ctx* ctx) {
 }
 
 // Digits of beta (24 bytes per element and layout beside its 16), where the
-// projector products use them and the memory is there.
+// projector products use them and the memory is there.  New projectors of a
+// context are cut into the same place: a captured pass holds its address.
 void cut_beta(chfsi_ctx* ctx) {
-    if (ctx->d_i8_beta) cudaFree(ctx->d_i8_beta);
-    ctx->d_i8_beta = nullptr;
     ctx->i8_beta = ctx->i8_betaT = I8Operand{};
     const int np = ctx->np, nb = ctx->nb, npw = ctx->n_pw;
     if (!ctx->d_i8) return;
@@ -670,7 +672,7 @@ void cut_beta(chfsi_ctx* ctx) {
     const size_t ba = rows ? i8_operand_bytes(np, kI8RowTile, npw, spc) : 0;
     const size_t bt = cols ? i8_operand_bytes(npw, kI8RowTile, np, spcT) : 0;
     if (ba + bt == 0) return;
-    if (dalloc(&ctx->d_i8_beta, ba + bt) != cudaSuccess) {
+    if (!ctx->d_i8_beta && dalloc(&ctx->d_i8_beta, ba + bt) != cudaSuccess) {
         cudaGetLastError();
         ctx->d_i8_beta = nullptr;
         return;
@@ -2328,6 +2330,7 @@ chfsi_status chfsi_set_basis(chfsi_ctx* ctx, const int32_t* miller, const double
     for (int g = 0; g < n; ++g) kmax = std::max(kmax, kinetic[g]);
     // kinetic bound of the reference: 1/2 Gmax^2 (chebyshev.rs:232)
     ctx->kin_max = gmax > 0.0 ? 0.5 * gmax * gmax : kmax;
+    ++ctx->layout;
     if (ctx->d_col_start) cudaFree(ctx->d_col_start);
     if (ctx->d_col_pos) cudaFree(ctx->d_col_pos);
     if (ctx->d_xact) cudaFree(ctx->d_xact);
@@ -2413,11 +2416,15 @@ chfsi_status chfsi_set_projectors(chfsi_ctx* ctx, const chfsi_c128* beta,
         doff[i] = (int)dt;
         dt += (size_t)ne * ne;
     }
-    if (ctx->d_dmat) cudaFree(ctx->d_dmat);
-    if (ctx->d_dmat0) cudaFree(ctx->d_dmat0);
-    ctx->d_dmat = ctx->d_dmat0 = nullptr;
-    CK(dalloc(&ctx->d_dmat, dt));
-    CK(dalloc(&ctx->d_dmat0, dt));
+    if (!ctx->d_dmat0 || ctx->n_dmat != dt) {
+        ++ctx->layout;
+        if (ctx->d_dmat) cudaFree(ctx->d_dmat);
+        if (ctx->d_dmat0) cudaFree(ctx->d_dmat0);
+        ctx->d_dmat = ctx->d_dmat0 = nullptr;
+        CK(dalloc(&ctx->d_dmat, dt));
+        CK(dalloc(&ctx->d_dmat0, dt));
+        ctx->n_dmat = dt;
+    }
     CK(copy_sync(ctx->d_dmat, dmat, dt * sizeof(double2), cudaMemcpyHostToDevice, ctx->st));
     CK(cudaMemcpyAsync(ctx->d_dmat0, ctx->d_dmat, dt * sizeof(double2), cudaMemcpyDeviceToDevice,
                        ctx->st));
@@ -3582,6 +3589,7 @@ struct chfsi_batch {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     std::vector<cudaEvent_t> events;
+    std::vector<unsigned> layouts;  // chfsi_ctx::layout of the members at the capture
     int ndeg = 0;
     size_t nodes = 0;
     std::string err;
@@ -3666,6 +3674,8 @@ extern "C" chfsi_status chfsi_batch_capture(chfsi_batch* b, int ndeg) {
     cudaGraphGetNodes(g, nullptr, &nn);
     b->nodes = nn;
     b->ndeg = ndeg;
+    b->layouts.clear();
+    for (const chfsi_ctx* c : b->members) b->layouts.push_back(c->layout);
     return CHFSI_OK;
 }
 
@@ -3680,6 +3690,11 @@ extern "C" chfsi_status chfsi_batch_graph_nodes(chfsi_batch* b, size_t* nodes) {
 // status (filter divergence, failed Rayleigh-Ritz).
 extern "C" chfsi_status chfsi_batch_run(chfsi_batch* b, double* eig_out, int* status_out) {
     if (!b || !b->exec) return CHFSI_ERR_BAD_INPUT;
+    for (size_t i = 0; i < b->members.size(); ++i)
+        if (b->members[i]->layout != b->layouts[i]) {
+            set_last_error("a member's basis or projector blocks changed since the capture: capture again");
+            return CHFSI_ERR_BAD_INPUT;
+        }
     cudaSetDevice(b->members[0]->device);
     cudaError_t e = cudaGraphLaunch(b->exec, b->origin);
     if (e != cudaSuccess) return cuda_fail(e, "cudaGraphLaunch", __FILE__, __LINE__);

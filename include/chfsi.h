@@ -441,7 +441,9 @@ chfsi_status chfsi_band_cg(chfsi_ctx* ctx, int max_steps, double tol, double* ei
  * captured once into a CUDA graph, members on their own streams forked from
  * and joined to one origin stream; chfsi_batch_run replays it as a single
  * graph launch.  Members: contexts created with CHFSI_PREC_MIXED on one
- * device, each having run one chfsi_diagonalize before capture.  The
+ * device, each having run one chfsi_diagonalize before capture.  A replay takes
+ * new values from chfsi_set_projectors with the same blocks; a new basis or other
+ * blocks need a new capture (chfsi_batch_run: CHFSI_ERR_BAD_INPUT).  The
  * reference crate has no batched path (one context, one stream). */
 typedef struct chfsi_batch chfsi_batch;
 chfsi_status chfsi_batch_create(chfsi_ctx* const* ctxs, int n, chfsi_batch** out);

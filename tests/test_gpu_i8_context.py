@@ -161,3 +161,39 @@ def test_every_call_reports_its_own_time_out(chfsi, name):
         if not failed:
             break
     assert launches >= (2 if name.startswith("scf") else 1)
+
+
+def test_captured_pass_takes_new_projectors(chfsi):
+    """A captured pass holds the addresses of the projectors' digits and of D: new
+    values go to the same place, and a change of their layout is refused."""
+    s = chfsi.SyntheticSystem(config_index=0, n_shell=1, lmax=1, rc_proj=[1.2, 0, 0, 0],
+                              d_min=0.5, d_max=2.0)
+    beta, dmat, off = 0.9 * s.beta(), 1.1 * s.dmat(), s.proj_offsets()
+
+    def prepared():
+        ctx = _context(chfsi, s, precision=chfsi.PREC_MIXED)
+        ctx.set_tc_shapes(0, 0)
+        return ctx, ctx.diagonalize(8, ctx.diagonalize(8))
+
+    ref, w = prepared()
+    ref.set_projectors(beta, off, dmat)
+    ref = ref.diagonalize(8, w)
+    ctx, _ = prepared()
+    batch = chfsi.Batch([ctx])
+    batch.capture(8)
+    held = [torch.empty(1 << k, device="cuda") for k in range(10, 24)]  # takes what is given back
+    ctx.set_projectors(beta, off, dmat)
+    held += [torch.zeros(1 << k, device="cuda") for k in range(10, 24)]
+    torch.cuda.synchronize()
+    np.testing.assert_allclose(batch.run()[0], ref, atol=1e-12, rtol=0)
+    assert abs(ref - w).max() > 1e-6
+    # other blocks: D lies elsewhere
+    split = np.arange(0, s.n_proj + 1, s.n_proj // s.n_ions, dtype=np.int32)
+    merged = split.copy()
+    merged[1] += 1
+    sizes = np.diff(merged)
+    ctx.set_projectors(beta, merged, np.concatenate([1e-3 * np.eye(k).ravel() for k in sizes]))
+    with pytest.raises(chfsi.BadInput, match="capture again"):
+        batch.run()
+    batch.capture(8)
+    batch.run()
