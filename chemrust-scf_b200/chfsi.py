@@ -242,6 +242,8 @@ def lib():
     L.chfsi_mixer_destroy.restype = None
     L.chfsi_mixer_num_params.argtypes = []
     L.chfsi_mixer_num_params.restype = C.c_size_t
+    L.chfsi_release_scratch.argtypes = []
+    L.chfsi_release_scratch.restype = None
     L.chfsi_launch_count.argtypes = []
     L.chfsi_launch_count.restype = C.c_longlong
     L.chfsi_last_error.argtypes = [vp]
@@ -389,6 +391,11 @@ def inject_fault(what, arg=0):
     INJECT_I8_NO_LOADS: the arg-th INT8 GEMM launch does; INJECT_ALLOC_FAIL: the
     arg-th device allocation fails; INJECT_NONE clears)."""
     _check(lib().chfsi_test_inject(what, arg))
+
+
+def release_scratch():
+    """Gives back the device scratch that zgemm_* and hegv_dev keep between calls."""
+    lib().chfsi_release_scratch()
 
 
 def launch_count():

@@ -380,20 +380,6 @@ void digit_reversal(const AxisPlan& P, std::vector<int>& pos) {
 std::atomic<long long> g_alloc_fail_in{-1};
 std::atomic<int> g_contexts{0};  // live contexts
 
-template <typename T> cudaError_t dalloc(T** p, size_t n) {
-    *p = nullptr;
-    if (n == 0) return cudaSuccess;
-    if (g_alloc_fail_in.load() >= 0 && g_alloc_fail_in.fetch_sub(1) == 0)
-        return cudaErrorMemoryAllocation;
-    cudaError_t e = cudaMalloc((void**)p, n * sizeof(T));
-    if (e == cudaErrorMemoryAllocation) {
-        cudaGetLastError();
-        scratch_trim();  // the scratch kept between calls may be what is missing
-        e = cudaMalloc((void**)p, n * sizeof(T));
-    }
-    return e;
-}
-
 // The context stream is non-blocking, so a legacy-stream cudaMemcpy or
 // cudaMemset is not ordered with its kernels (a pageable host-to-device
 // cudaMemcpy may even return before its DMA lands).  Every set-up copy and
@@ -509,7 +495,7 @@ struct chfsi_ctx {
     bool mixed_active = false;   // current filter precision (SCF may switch to FP64)
     float2* d_psi32a = nullptr; float2* d_psi32b = nullptr; float2* d_psi32 = nullptr;
     float2* d_hpsi32 = nullptr; float2* d_nl32 = nullptr; float2* d_work32 = nullptr;
-    void* d_planes = nullptr;    // all bf16 plane storage
+    char* d_planes = nullptr;    // all bf16 plane storage
     TcPlanes tp_beta_a, tp_betaT_b, tp_psi_b, tp_small_a;
     float* d_tc_part = nullptr; int* d_tc_err = nullptr;
     // FP64 products on the INT8 tensor cores: digits of beta for the
@@ -589,6 +575,16 @@ struct chfsi_ctx {
     } while (0)
 
 namespace {
+
+// Device memory of a context; before it is refused the device gets back what is
+// kept between calls.
+template <typename T> cudaError_t dalloc(T** p, size_t n) {
+    *p = nullptr;
+    if (n == 0) return cudaSuccess;
+    const bool planned = g_alloc_fail_in.load() >= 0 && g_alloc_fail_in.fetch_sub(1) == 0;
+    if (planned) return cudaErrorMemoryAllocation;
+    return malloc_or_trim((void**)p, n * sizeof(T));
+}
 
 chfsi_status ensure_pinned(chfsi_ctx* ctx, size_t n) {
     if (ctx->h_pin_n >= n) return CHFSI_OK;
@@ -1018,9 +1014,9 @@ chfsi_status alloc_mixed(chfsi_ctx* ctx, int ncol) {
     }
     size_t total = 0;
     for (auto& s : specs) total += 3 * (size_t)s.rows_alloc * s.kp;
-    CK(cudaMalloc(&ctx->d_planes, total * 2));
+    CK(dalloc(&ctx->d_planes, total * 2));
     CK(cudaMemsetAsync(ctx->d_planes, 0, total * 2, ctx->st));
-    char* p = (char*)ctx->d_planes;
+    char* p = ctx->d_planes;
     for (auto& s : specs) {
         for (int i = 0; i < 3; ++i) {
             s.t->p[i] = p;
@@ -1992,9 +1988,9 @@ chfsi_status cg_prepare(chfsi_ctx* ctx) {
     if (ctx->uspp && np > 0) {
         // R = (-q^-1 - beta^H T beta)^-1 on the host (once per context)
         double2 *bt = nullptr, *part = nullptr, *cm = nullptr;
-        CK(cudaMalloc((void**)&bt, (size_t)np * n * sizeof(double2)));
-        cudaError_t e = cudaMalloc((void**)&part, splitk_partial_elems(np, np, (int)n) * sizeof(double2));
-        if (e == cudaSuccess) e = cudaMalloc((void**)&cm, (size_t)np * np * sizeof(double2));
+        CK(dalloc(&bt, (size_t)np * n));
+        cudaError_t e = dalloc(&part, splitk_partial_elems(np, np, (int)n));
+        if (e == cudaSuccess) e = dalloc(&cm, (size_t)np * np);
         if (e != cudaSuccess) {
             cudaFree(bt); cudaFree(part); cudaFree(cm);
             CK(e);
@@ -2242,7 +2238,7 @@ chfsi_status chfsi_create(const chfsi_dims* dims, const chfsi_config* cfg, chfsi
         const std::vector<int>& p = ctx->dr[d];
         std::vector<int> inv(p.size());
         for (size_t k = 0; k < p.size(); ++k) inv[p[k]] = (int)k;
-        if (cudaMalloc((void**)&ctx->d_idr[d], inv.size() * sizeof(int)) != cudaSuccess) return bail(CHFSI_ERR_OUT_OF_MEMORY);
+        if (malloc_or_trim((void**)&ctx->d_idr[d], inv.size() * sizeof(int)) != cudaSuccess) return bail(CHFSI_ERR_OUT_OF_MEMORY);
         if (copy_sync(ctx->d_idr[d], inv.data(), inv.size() * sizeof(int), cudaMemcpyHostToDevice,
                       ctx->st) != cudaSuccess)
             return bail(CHFSI_ERR_CUDA);
@@ -2437,7 +2433,7 @@ chfsi_status chfsi_set_projectors(chfsi_ctx* ctx, const chfsi_c128* beta,
     } else {
         // stage in the hpsi buffer when it is large enough, else in a temporary
         double2* stage = nullptr;
-        CK(cudaMalloc((void**)&stage, nbeta * sizeof(double2)));
+        CK(dalloc(&stage, nbeta));
         if (cudaError_t e = copy_sync(stage, beta, nbeta * sizeof(double2), cudaMemcpyHostToDevice,
                                       ctx->st)) {
             cudaFree(stage);
@@ -2469,8 +2465,11 @@ chfsi_status chfsi_set_qmat(chfsi_ctx* ctx, const chfsi_c128* qmat) {
     CK(copy_sync(ctx->d_qmat, qmat, dt * sizeof(double2), cudaMemcpyHostToDevice, ctx->st));
     // B = beta^H beta on the device
     double2 *part = nullptr, *dB = nullptr;
-    CK(cudaMalloc((void**)&part, splitk_partial_elems(np, np, ctx->n_pw) * sizeof(double2)));
-    CK(cudaMalloc((void**)&dB, (size_t)np * np * sizeof(double2)));
+    CK(dalloc(&part, splitk_partial_elems(np, np, ctx->n_pw)));
+    if (cudaError_t e = dalloc(&dB, (size_t)np * np)) {
+        cudaFree(part);
+        CK(e);
+    }
     gemm_cn(ctx->d_beta, ctx->n_pw, ctx->d_beta, ctx->n_pw, np, np, ctx->n_pw, part, dB, ctx->st);
     std::vector<std::complex<double>> B((size_t)np * np), Q((size_t)np * np, 0.0);
     cudaError_t e = cudaMemcpyAsync(B.data(), dB, B.size() * sizeof(double2), cudaMemcpyDeviceToHost, ctx->st);
@@ -2609,6 +2608,8 @@ chfsi_status chfsi_get_stream(chfsi_ctx* ctx, void** out) {
     *out = (void*)ctx->st;
     return CHFSI_OK;
 }
+
+void chfsi_release_scratch(void) { scratch_trim(); }
 
 long long chfsi_launch_count(void) { return g_launch_count.load(); }
 

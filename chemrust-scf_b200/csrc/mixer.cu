@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "launch_count.hpp"
+#include "scratch.hpp"
 
 namespace chfsi {
 namespace {
@@ -348,13 +349,13 @@ struct Rng {
 }  // namespace
 
 cudaError_t mlp_alloc(Mlp& M, int cap) {
-    auto fa = [](float** p, size_t n) { return cudaMalloc((void**)p, n * sizeof(float)); };
+    auto fa = [](float** p, size_t n) { return malloc_or_trim((void**)p, n * sizeof(float)); };
     cudaError_t e;
     if (!M.w) {
         if ((e = fa(&M.w, kMixParams)) || (e = fa(&M.g, kMixParams)) || (e = fa(&M.m, kMixParams)) ||
             (e = fa(&M.v, kMixParams)) || (e = fa(&M.loss, 1)))
             return e;
-        if ((e = cudaMalloc((void**)&M.wb, kMixParams * sizeof(__nv_bfloat16)))) return e;
+        if ((e = malloc_or_trim((void**)&M.wb, kMixParams * sizeof(__nv_bfloat16)))) return e;
         cudaMemsetAsync(M.m, 0, kMixParams * sizeof(float), M.st);
         cudaMemsetAsync(M.v, 0, kMixParams * sizeof(float), M.st);
     }

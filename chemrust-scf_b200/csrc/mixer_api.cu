@@ -9,6 +9,7 @@
 
 #include "chfsi.h"
 #include "mixer.hpp"
+#include "scratch.hpp"
 
 namespace chfsi {
 chfsi_status cuda_fail(cudaError_t e, const char* expr, const char* file, int line);
@@ -149,8 +150,8 @@ chfsi_status chfsi_mixer_train(chfsi_mixer* m, const float* x, const float* t, i
         cudaFree(M.data_t);
         M.data_x = M.data_t = nullptr;
         M.data_cap = 0;
-        MK(cudaMalloc((void**)&M.data_x, (size_t)n * kMixIn * sizeof(float)));
-        MK(cudaMalloc((void**)&M.data_t, (size_t)n * nt * sizeof(float)));
+        MK(malloc_or_trim((void**)&M.data_x, (size_t)n * kMixIn * sizeof(float)));
+        MK(malloc_or_trim((void**)&M.data_t, (size_t)n * nt * sizeof(float)));
         M.data_cap = n;
     }
     MK(cudaMemcpyAsync(M.data_x, x, (size_t)n * kMixIn * sizeof(float), cudaMemcpyHostToDevice, M.st));
@@ -159,13 +160,13 @@ chfsi_status chfsi_mixer_train(chfsi_mixer* m, const float* x, const float* t, i
     if ((size_t)nbatch * batch > M.idx_cap) {
         cudaFree(M.idx);
         M.idx = nullptr;
-        MK(cudaMalloc((void**)&M.idx, (size_t)nbatch * batch * sizeof(int)));
+        MK(malloc_or_trim((void**)&M.idx, (size_t)nbatch * batch * sizeof(int)));
         M.idx_cap = (size_t)nbatch * batch;
     }
     if (nbatch > m->loss_cap) {
         cudaFree(m->loss_hist);
         m->loss_hist = nullptr;
-        MK(cudaMalloc((void**)&m->loss_hist, nbatch * sizeof(float)));
+        MK(malloc_or_trim((void**)&m->loss_hist, nbatch * sizeof(float)));
         m->loss_cap = nbatch;
     }
     std::vector<int> perm(n);

@@ -46,6 +46,10 @@ cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t st) {
     cudaMemPool_t pool = nullptr;
     e = pool_of(dev, &pool);
     if (e != cudaSuccess) return e;
+    e = cudaMallocFromPoolAsync(p, bytes, pool, st);
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    scratch_trim();  // kept blocks of other sizes
     return cudaMallocFromPoolAsync(p, bytes, pool, st);
 }
 
@@ -54,10 +58,19 @@ void scratch_free(void* p, cudaStream_t st) {
 }
 
 void scratch_trim() {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
     std::lock_guard<std::mutex> lk(g_pool_mu);
-    if (g_pools[dev]) cudaMemPoolTrimTo(g_pools[dev], 0);
+    for (cudaMemPool_t pool : g_pools)
+        if (pool) cudaMemPoolTrimTo(pool, 0);
+}
+
+cudaError_t malloc_or_trim(void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    scratch_trim();
+    e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+    return e;
 }
 
 }  // namespace chfsi

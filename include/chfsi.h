@@ -277,6 +277,13 @@ chfsi_status chfsi_get_stream(chfsi_ctx* ctx, void** out);
 /* Kernels launched by this library since load (all contexts). */
 long long    chfsi_launch_count(void);
 
+/* The entry points below that take device pointers and no context keep their
+ * scratch between calls, at most 1 GiB per device.  It goes back when the last
+ * context is destroyed, when an allocation of this library would fail, and here
+ * (what calls in flight use stays); a process without contexts calls this when it
+ * has no more products or eigenproblems to solve. */
+void         chfsi_release_scratch(void);
+
 /* C[m][n] = sum_k conj(A[m][k]) B[n][k] on DEVICE pointers (row-major; C is
  * m x n dense), on `stream` (cudaStream_t, 0 = legacy default).  The op::C
  * ZGEMM of BlasHandle::gemm_c64 (src/device/blas.rs:79-102) that forms

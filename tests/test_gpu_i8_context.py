@@ -57,7 +57,7 @@ def _same(a, b):
 
 
 def test_context_without_the_scratch(chfsi, sys_kb):
-    """The scratch is the one allocation of a creation that may fail: what was
+    """The scratch is the one allocation of a creation that may fail first: what was
     asked for still runs, and its status does not come from memory that the
     process gave back before (the error word is mapped host memory)."""
     rt = ctypes.CDLL("libcudart.so.12")
@@ -73,20 +73,14 @@ def test_context_without_the_scratch(chfsi, sys_kb):
     ref = _apply_h(_context(chfsi, sys_kb), psi)
     dims = {"ngrid": list(sys_kb.ngrid), "n_pw": sys_kb.n_pw, "n_bands": sys_kb.n_bands,
             "n_proj": sys_kb.n_proj, "n_ions": sys_kb.n_ions}
-    made = []
     for nth in range(200):
         chfsi.inject_fault(chfsi.INJECT_ALLOC_FAIL, nth)
         try:
             chfsi.Context(dims=dims)
-            made.append(nth)
+            break
         except chfsi.OutOfMemory:
             pass
-        chfsi.inject_fault(chfsi.INJECT_NONE)
-        if made[-3:] == [nth - 2, nth - 1, nth]:
-            break  # past the last allocation
-    optional = [k for k in made if k < nth - 2]
-    assert len(optional) == 1
-    chfsi.inject_fault(chfsi.INJECT_ALLOC_FAIL, optional[0])
+    chfsi.inject_fault(chfsi.INJECT_ALLOC_FAIL, nth)
     ctx = chfsi.Context(sys_kb)
     chfsi.inject_fault(chfsi.INJECT_NONE)
     ctx.set_veff(ctx.get_vloc())
@@ -197,3 +191,15 @@ def test_captured_pass_takes_new_projectors(chfsi):
         batch.run()
     batch.capture(8)
     batch.run()
+
+
+def test_scratch_of_a_process_without_contexts(chfsi):
+    m, n, k = 256, 160, 20000
+    a, b, c = _operands(m, n, k)
+    chfsi.zgemm_cn(a.data_ptr(), k, b.data_ptr(), k, m, n, k, c.data_ptr())  # loads the kernels
+    chfsi.release_scratch()
+    free = torch.cuda.mem_get_info()[0]
+    chfsi.zgemm_cn(a.data_ptr(), k, b.data_ptr(), k, m, n, k, c.data_ptr())
+    assert torch.cuda.mem_get_info()[0] < free
+    chfsi.release_scratch()
+    assert torch.cuda.mem_get_info()[0] == free
