@@ -545,6 +545,7 @@ struct chfsi_ctx {
     size_t n_dmat = 0;            // elements of d_dmat and d_dmat0
     // counts the changes of buffers whose addresses a captured pass holds
     unsigned layout = 0;
+    bool in_graph = false;        // a captured pass holds the INT8 buffers
     double* d_cion = nullptr;     // per ion sum_n f_n C^H q C
     double* d_vion = nullptr;     // per ion int V_eff g(r - R_I)
     // learned density mixer (G-space residual history on the density grid)
@@ -576,13 +577,18 @@ struct chfsi_ctx {
 
 namespace {
 
-// Device memory of a context; before it is refused the device gets back what is
-// kept between calls.
-template <typename T> cudaError_t dalloc(T** p, size_t n) {
+// Memory of the INT8 products back to the device; false if there is none to give.
+bool give_back_i8(chfsi_ctx* ctx);
+
+// Device memory of a context.  Before it is refused the device gets back what is
+// kept between calls, and then what the context can do without: the scratch and
+// the digits of the INT8 products (ctx null: an allocation of those themselves).
+template <typename T> cudaError_t dalloc(chfsi_ctx* ctx, T** p, size_t n) {
     *p = nullptr;
     if (n == 0) return cudaSuccess;
     const bool planned = g_alloc_fail_in.load() >= 0 && g_alloc_fail_in.fetch_sub(1) == 0;
-    if (planned) return cudaErrorMemoryAllocation;
+    const cudaError_t e = planned ? cudaErrorMemoryAllocation : malloc_or_trim((void**)p, n * sizeof(T));
+    if (e != cudaErrorMemoryAllocation || !ctx || !give_back_i8(ctx)) return e;
     return malloc_or_trim((void**)p, n * sizeof(T));
 }
 
@@ -627,9 +633,28 @@ chfsi_status i8_status(chfsi_ctx* ctx) {
     return ctx->fail(CHFSI_ERR_TIMEOUT, "tensor-core GEMM pipeline wait timed out");
 }
 
+// Whether `bytes` are at most half of the device's free memory: what follows, of
+// this context or of others, is to fit as well.
+bool spare_memory(size_t bytes) {
+    size_t free_b = 0, total = 0;
+    return cudaMemGetInfo(&free_b, &total) == cudaSuccess && bytes <= free_b / 2;
+}
+
+bool give_back_i8(chfsi_ctx* ctx) {
+    if (ctx->in_graph || (!ctx->d_i8 && !ctx->d_i8_beta)) return false;
+    cudaStreamSynchronize(ctx->st);
+    cudaFree(ctx->d_i8);
+    cudaFree(ctx->d_i8_beta);
+    ctx->d_i8 = ctx->d_i8_beta = nullptr;
+    ctx->i8_bytes = 0;
+    ctx->i8_beta = ctx->i8_betaT = I8Operand{};
+    return true;
+}
+
 // Scratch for the INT8 products of this context's sizes, at most kI8Scratch
 // bytes (longer products run in groups).  Without it, as when the device is
-// short of memory, the FP64 tensor path computes the same products.
+// short of memory, then or later (give_back_i8), the FP64 tensor path computes
+// the same products.
 constexpr size_t kI8Scratch = (size_t)1 << 30;
 void alloc_i8(chfsi_ctx* ctx) {
     const int nb = ctx->nb + 1, np = ctx->np, npw = ctx->n_pw;
@@ -648,7 +673,7 @@ void alloc_i8(chfsi_ctx* ctx) {
         return;
     }
     *ctx->h_i8_err = 0;  // read after every synchronisation, scratch or not
-    if (dalloc(&ctx->d_i8, need) != cudaSuccess) {
+    if (!spare_memory(need) || dalloc(nullptr, &ctx->d_i8, need) != cudaSuccess) {
         cudaGetLastError();
         ctx->d_i8 = nullptr;
         return;
@@ -668,7 +693,8 @@ void cut_beta(chfsi_ctx* ctx) {
     const size_t ba = rows ? i8_operand_bytes(np, kI8RowTile, npw, spc) : 0;
     const size_t bt = cols ? i8_operand_bytes(npw, kI8RowTile, np, spcT) : 0;
     if (ba + bt == 0) return;
-    if (!ctx->d_i8_beta && dalloc(&ctx->d_i8_beta, ba + bt) != cudaSuccess) {
+    if (!ctx->d_i8_beta &&
+        (!spare_memory(ba + bt) || dalloc(nullptr, &ctx->d_i8_beta, ba + bt) != cudaSuccess)) {
         cudaGetLastError();
         ctx->d_i8_beta = nullptr;
         return;
@@ -997,11 +1023,11 @@ chfsi_status rr_dev(chfsi_ctx* ctx, bool fp32_block) {
 chfsi_status alloc_mixed(chfsi_ctx* ctx, int ncol) {
     const int nb = ctx->nb, np = ctx->np, npw = ctx->n_pw;
     const size_t nbpw = (size_t)nb * npw;
-    CK(dalloc(&ctx->d_psi32a, nbpw));
-    CK(dalloc(&ctx->d_psi32b, nbpw));
-    CK(dalloc(&ctx->d_hpsi32, nbpw));
-    if (np > 0) CK(dalloc(&ctx->d_nl32, nbpw));
-    CK(dalloc(&ctx->d_work32, (size_t)nb * ctx->nz * ncol));
+    CK(dalloc(ctx, &ctx->d_psi32a, nbpw));
+    CK(dalloc(ctx, &ctx->d_psi32b, nbpw));
+    CK(dalloc(ctx, &ctx->d_hpsi32, nbpw));
+    if (np > 0) CK(dalloc(ctx, &ctx->d_nl32, nbpw));
+    CK(dalloc(ctx, &ctx->d_work32, (size_t)nb * ctx->nz * ncol));
     struct Spec { TcPlanes* t; int rows_alloc; int kp; };
     const int kp_pw = tc_kpad(npw);
     std::vector<Spec> specs = {
@@ -1014,7 +1040,7 @@ chfsi_status alloc_mixed(chfsi_ctx* ctx, int ncol) {
     }
     size_t total = 0;
     for (auto& s : specs) total += 3 * (size_t)s.rows_alloc * s.kp;
-    CK(dalloc(&ctx->d_planes, total * 2));
+    CK(dalloc(ctx, &ctx->d_planes, total * 2));
     CK(cudaMemsetAsync(ctx->d_planes, 0, total * 2, ctx->st));
     char* p = ctx->d_planes;
     for (auto& s : specs) {
@@ -1029,8 +1055,8 @@ chfsi_status alloc_mixed(chfsi_ctx* ctx, int ncol) {
     // the K-split count depends on it: size for the largest
     size_t pf = 1;
     for (int b = 1; b <= nb && np > 0; ++b) pf = std::max(pf, tc_partial_floats(np, b, npw));
-    CK(dalloc(&ctx->d_tc_part, pf));
-    CK(dalloc(&ctx->d_tc_err, 4));
+    CK(dalloc(ctx, &ctx->d_tc_part, pf));
+    CK(dalloc(ctx, &ctx->d_tc_err, 4));
     CK(cudaMemsetAsync(ctx->d_tc_err, 0, 4 * sizeof(int), ctx->st));
     return CHFSI_OK;
 }
@@ -1273,15 +1299,15 @@ chfsi_status filter_dev32(chfsi_ctx* ctx, int ndeg, const double* eig_dev, int n
 // that follows gets the full H X_p in FP64.
 chfsi_status alloc_rchfsi(chfsi_ctx* ctx, bool fp32) {
     const size_t n = (size_t)ctx->nb * ctx->n_pw;
-    if (!ctx->d_rc_hx) CK(dalloc(&ctx->d_rc_hx, n));
-    if (!ctx->d_rc_y) CK(dalloc(&ctx->d_rc_y, n));
-    if (!ctx->d_rc_coef) CK(dalloc(&ctx->d_rc_coef, (size_t)3 * (ctx->max_deg + 1)));
-    if (!ctx->d_rc_lam) CK(dalloc(&ctx->d_rc_lam, (size_t)(ctx->max_deg + 1) * ctx->nb));
+    if (!ctx->d_rc_hx) CK(dalloc(ctx, &ctx->d_rc_hx, n));
+    if (!ctx->d_rc_y) CK(dalloc(ctx, &ctx->d_rc_y, n));
+    if (!ctx->d_rc_coef) CK(dalloc(ctx, &ctx->d_rc_coef, (size_t)3 * (ctx->max_deg + 1)));
+    if (!ctx->d_rc_lam) CK(dalloc(ctx, &ctx->d_rc_lam, (size_t)(ctx->max_deg + 1) * ctx->nb));
     if (fp32) {
-        if (!ctx->d_rc_y32) CK(dalloc(&ctx->d_rc_y32, n));
+        if (!ctx->d_rc_y32) CK(dalloc(ctx, &ctx->d_rc_y32, n));
     } else {
-        if (!ctx->d_rc_r0) CK(dalloc(&ctx->d_rc_r0, n));
-        if (!ctx->d_rc_r1) CK(dalloc(&ctx->d_rc_r1, n));
+        if (!ctx->d_rc_r0) CK(dalloc(ctx, &ctx->d_rc_r0, n));
+        if (!ctx->d_rc_r1) CK(dalloc(ctx, &ctx->d_rc_r1, n));
     }
     return CHFSI_OK;
 }
@@ -1629,12 +1655,12 @@ chfsi_status alloc_density(chfsi_ctx* ctx) {
     ctx->d_phase = nullptr;
     for (int d = 0; d < 3; ++d) ctx->d_fidr[d] = nullptr;
     const size_t ng = ctx->fng;
-    CK(dalloc(&ctx->d_veff_d, ng));
-    CK(dalloc(&ctx->d_vloc, ng));
-    CK(dalloc(&ctx->d_rho_in, ng)); CK(dalloc(&ctx->d_rho_out, ng));
-    CK(dalloc(&ctx->d_rho_next, ng));
-    CK(dalloc(&ctx->d_cgrid, ng));
-    CK(dalloc(&ctx->d_hist, 2 * (size_t)kPulayMax * ng));
+    CK(dalloc(ctx, &ctx->d_veff_d, ng));
+    CK(dalloc(ctx, &ctx->d_vloc, ng));
+    CK(dalloc(ctx, &ctx->d_rho_in, ng)); CK(dalloc(ctx, &ctx->d_rho_out, ng));
+    CK(dalloc(ctx, &ctx->d_rho_next, ng));
+    CK(dalloc(ctx, &ctx->d_cgrid, ng));
+    CK(dalloc(ctx, &ctx->d_hist, 2 * (size_t)kPulayMax * ng));
     std::vector<double*> hp(2 * kPulayMax);
     for (int i = 0; i < 2 * kPulayMax; ++i) hp[i] = ctx->d_hist + (size_t)i * ng;
     CK(copy_sync(ctx->d_hist_ptrs, hp.data(), hp.size() * sizeof(double*), cudaMemcpyHostToDevice,
@@ -1645,7 +1671,7 @@ chfsi_status alloc_density(chfsi_ctx* ctx) {
         const std::vector<int>& p = ctx->fdr[d];
         std::vector<int> inv(p.size());
         for (size_t k = 0; k < p.size(); ++k) inv[p[k]] = (int)k;
-        CK(dalloc(&ctx->d_fidr[d], (size_t)n3[d]));
+        CK(dalloc(ctx, &ctx->d_fidr[d], (size_t)n3[d]));
         CK(copy_sync(ctx->d_fidr[d], inv.data(), inv.size() * sizeof(int), cudaMemcpyHostToDevice,
                      ctx->st));
     }
@@ -1679,7 +1705,7 @@ chfsi_status upload_phases(chfsi_ctx* ctx) {
     }
     if (ctx->d_phase) cudaFree(ctx->d_phase);
     ctx->d_phase = nullptr;
-    CK(dalloc(&ctx->d_phase, ph.size()));
+    CK(dalloc(ctx, &ctx->d_phase, ph.size()));
     CK(copy_sync(ctx->d_phase, ph.data(), ph.size() * sizeof(double2), cudaMemcpyHostToDevice, ctx->st));
     return CHFSI_OK;
 }
@@ -1688,11 +1714,11 @@ chfsi_status upload_phases(chfsi_ctx* ctx) {
 chfsi_status alloc_mix(chfsi_ctx* ctx) {
     if (ctx->d_mix_c) return CHFSI_OK;
     const size_t ng = ctx->fng;
-    CK(dalloc(&ctx->d_shell, ng));
-    CK(dalloc(&ctx->d_mix_c, 7 * ng));
-    CK(dalloc(&ctx->d_mix_r, 4 * ng));
-    if (!ctx->d_mix_acc) CK(dalloc(&ctx->d_mix_acc, (size_t)kMixShells * kShellAcc));
-    if (!ctx->d_mix_x) CK(dalloc(&ctx->d_mix_x, (size_t)kMixIn + kMixShells * kMixTargets + kMixOut));
+    CK(dalloc(ctx, &ctx->d_shell, ng));
+    CK(dalloc(ctx, &ctx->d_mix_c, 7 * ng));
+    CK(dalloc(ctx, &ctx->d_mix_r, 4 * ng));
+    if (!ctx->d_mix_acc) CK(dalloc(ctx, &ctx->d_mix_acc, (size_t)kMixShells * kShellAcc));
+    if (!ctx->d_mix_x) CK(dalloc(ctx, &ctx->d_mix_x, (size_t)kMixIn + kMixShells * kMixTargets + kMixOut));
     launch_shell_index(grid_recip(ctx), ctx->d_shell, ctx->st);
     CK(cudaGetLastError());
     return CHFSI_OK;
@@ -1736,50 +1762,50 @@ chfsi_status alloc_all(chfsi_ctx* ctx) {
     // carries along as an extra column (CHFSI_BOUND_LANCZOS_FUSED)
     const int nbx = ctx->nb + 1;
     const size_t nbpw = (size_t)nbx * ctx->n_pw;
-    CK(dalloc(&ctx->d_kin, ctx->n_pw));
-    CK(dalloc(&ctx->d_perm, ctx->n_pw));
-    CK(dalloc(&ctx->d_pw_col, ctx->n_pw));
-    CK(dalloc(&ctx->d_pw_zpos, ctx->n_pw));
-    CK(dalloc(&ctx->d_veff, ctx->ng));
-    CK(dalloc(&ctx->d_rho_w, ctx->ng));
+    CK(dalloc(ctx, &ctx->d_kin, ctx->n_pw));
+    CK(dalloc(ctx, &ctx->d_perm, ctx->n_pw));
+    CK(dalloc(ctx, &ctx->d_pw_col, ctx->n_pw));
+    CK(dalloc(ctx, &ctx->d_pw_zpos, ctx->n_pw));
+    CK(dalloc(ctx, &ctx->d_veff, ctx->ng));
+    CK(dalloc(ctx, &ctx->d_rho_w, ctx->ng));
     {
         size_t groups = 1;
         for (int n = 1; n <= ctx->nb; ++n)
             groups = std::max(groups, (size_t)density_groups(ctx->nz, n));
-        CK(dalloc(&ctx->d_rho_part, groups * ctx->ng));
+        CK(dalloc(ctx, &ctx->d_rho_part, groups * ctx->ng));
     }
-    CK(dalloc(&ctx->d_wgrid, ctx->ng));
-    CK(dalloc(&ctx->d_minmax, 2));
-    CK(dalloc(&ctx->d_psi, nbpw));
-    CK(dalloc(&ctx->d_psi2, nbpw));
-    CK(dalloc(&ctx->d_hpsi, nbpw));
+    CK(dalloc(ctx, &ctx->d_wgrid, ctx->ng));
+    CK(dalloc(ctx, &ctx->d_minmax, 2));
+    CK(dalloc(ctx, &ctx->d_psi, nbpw));
+    CK(dalloc(ctx, &ctx->d_psi2, nbpw));
+    CK(dalloc(ctx, &ctx->d_hpsi, nbpw));
     if (ctx->np > 0) {
-        CK(dalloc(&ctx->d_nl, nbpw));
-        CK(dalloc(&ctx->d_beta, (size_t)ctx->np * ctx->n_pw));
-        CK(dalloc(&ctx->d_cp, (size_t)ctx->np * nbx));
-        CK(dalloc(&ctx->d_cd, (size_t)ctx->np * nbx));
-        CK(dalloc(&ctx->d_cq, (size_t)ctx->np * nbx));
-        CK(dalloc(&ctx->d_proj_ion, ctx->np));
-        CK(dalloc(&ctx->d_poff, ctx->nions + 1));
-        CK(dalloc(&ctx->d_doff, ctx->nions));
+        CK(dalloc(ctx, &ctx->d_nl, nbpw));
+        CK(dalloc(ctx, &ctx->d_beta, (size_t)ctx->np * ctx->n_pw));
+        CK(dalloc(ctx, &ctx->d_cp, (size_t)ctx->np * nbx));
+        CK(dalloc(ctx, &ctx->d_cd, (size_t)ctx->np * nbx));
+        CK(dalloc(ctx, &ctx->d_cq, (size_t)ctx->np * nbx));
+        CK(dalloc(ctx, &ctx->d_proj_ion, ctx->np));
+        CK(dalloc(ctx, &ctx->d_poff, ctx->nions + 1));
+        CK(dalloc(ctx, &ctx->d_doff, ctx->nions));
     }
     const size_t nn = (size_t)ctx->nb * ctx->nb;
-    CK(dalloc(&ctx->d_H, nn)); CK(dalloc(&ctx->d_S, nn)); CK(dalloc(&ctx->d_T1, nn));
-    CK(dalloc(&ctx->d_T2, nn)); CK(dalloc(&ctx->d_V, nn));
-    CK(dalloc(&ctx->d_eig, ctx->nb)); CK(dalloc(&ctx->d_eig_prev, ctx->nb));
-    CK(dalloc(&ctx->d_jac, heev_fits(ctx->nb) ? heev_scratch_doubles(ctx->nb)
+    CK(dalloc(ctx, &ctx->d_H, nn)); CK(dalloc(ctx, &ctx->d_S, nn)); CK(dalloc(ctx, &ctx->d_T1, nn));
+    CK(dalloc(ctx, &ctx->d_T2, nn)); CK(dalloc(ctx, &ctx->d_V, nn));
+    CK(dalloc(ctx, &ctx->d_eig, ctx->nb)); CK(dalloc(ctx, &ctx->d_eig_prev, ctx->nb));
+    CK(dalloc(ctx, &ctx->d_jac, heev_fits(ctx->nb) ? heev_scratch_doubles(ctx->nb)
                                               : jacobi_scratch_doubles(ctx->nb, ctx->jac_max_sweeps)));
-    CK(dalloc(&ctx->d_flags, 8));
+    CK(dalloc(ctx, &ctx->d_flags, 8));
     CK(cudaMemsetAsync(ctx->d_flags, 0, 8 * sizeof(int), ctx->st));
-    CK(dalloc(&ctx->d_coef, 8));
-    CK(dalloc(&ctx->d_nsq, ctx->max_deg + 2));
-    CK(dalloc(&ctx->d_lz_v, ctx->n_pw)); CK(dalloc(&ctx->d_lz_v0, ctx->n_pw));
-    CK(dalloc(&ctx->d_lz_f, ctx->n_pw)); CK(dalloc(&ctx->d_lz_start, ctx->n_pw));
-    CK(dalloc(&ctx->d_lz, 2 * 64));
-    CK(dalloc(&ctx->d_occ, ctx->nb));
-    CK(dalloc(&ctx->d_acc, 8));
-    CK(dalloc(&ctx->d_hist_ptrs, 2 * kPulayMax));
-    CK(dalloc(&ctx->d_dots, kPulayMax));
+    CK(dalloc(ctx, &ctx->d_coef, 8));
+    CK(dalloc(ctx, &ctx->d_nsq, ctx->max_deg + 2));
+    CK(dalloc(ctx, &ctx->d_lz_v, ctx->n_pw)); CK(dalloc(ctx, &ctx->d_lz_v0, ctx->n_pw));
+    CK(dalloc(ctx, &ctx->d_lz_f, ctx->n_pw)); CK(dalloc(ctx, &ctx->d_lz_start, ctx->n_pw));
+    CK(dalloc(ctx, &ctx->d_lz, 2 * 64));
+    CK(dalloc(ctx, &ctx->d_occ, ctx->nb));
+    CK(dalloc(ctx, &ctx->d_acc, 8));
+    CK(dalloc(ctx, &ctx->d_hist_ptrs, 2 * kPulayMax));
+    CK(dalloc(ctx, &ctx->d_dots, kPulayMax));
     // split-K partials: max over the GEMMs that use them
     // (any band count 1..nb may reach the projector GEMM through chfsi_apply_h)
     size_t pe = std::max(splitk_partial_elems(ctx->nb, ctx->nb, ctx->n_pw),
@@ -1789,7 +1815,7 @@ chfsi_status alloc_all(chfsi_ctx* ctx) {
         for (int n = 1; n <= nbx; ++n)
             pe = std::max(pe, splitk_partial_elems(ctx->np, n, ctx->n_pw));
     ctx->part_elems = pe;
-    CK(dalloc(&ctx->d_part, pe));
+    CK(dalloc(ctx, &ctx->d_part, pe));
     // Lanczos start vector: SplitMix64(0x5EED) uniform pairs in [-1/2, 1/2)
     {
         std::vector<double2> v(ctx->n_pw);
@@ -1966,12 +1992,12 @@ chfsi_status cg_prepare(chfsi_ctx* ctx) {
     if (ctx->cg_ready) return CHFSI_OK;
     const size_t n = ctx->n_pw;
     const int np = ctx->np, nb = ctx->nb;
-    if (!ctx->d_tpa) CK(dalloc(&ctx->d_tpa, n));
-    if (!ctx->d_cgv) CK(dalloc(&ctx->d_cgv, 10 * n));
-    if (!ctx->d_cgc) CK(dalloc(&ctx->d_cgc, (size_t)3 * std::max(np, 1)));
-    if (!ctx->d_cgov) CK(dalloc(&ctx->d_cgov, 2 * (size_t)nb));
-    if (!ctx->d_cgG) CK(dalloc(&ctx->d_cgG, (size_t)nb * nb));
-    if (!ctx->d_cgdot) CK(dalloc(&ctx->d_cgdot, 16));
+    if (!ctx->d_tpa) CK(dalloc(ctx, &ctx->d_tpa, n));
+    if (!ctx->d_cgv) CK(dalloc(ctx, &ctx->d_cgv, 10 * n));
+    if (!ctx->d_cgc) CK(dalloc(ctx, &ctx->d_cgc, (size_t)3 * std::max(np, 1)));
+    if (!ctx->d_cgov) CK(dalloc(ctx, &ctx->d_cgov, 2 * (size_t)nb));
+    if (!ctx->d_cgG) CK(dalloc(ctx, &ctx->d_cgG, (size_t)nb * nb));
+    if (!ctx->d_cgdot) CK(dalloc(ctx, &ctx->d_cgdot, 16));
     size_t pe = 0;
     for (int k = 1; k <= nb; ++k)
         pe = std::max({pe, splitk_partial_elems(k, 1, (int)n), splitk_partial_elems(1, k, (int)n)});
@@ -1979,7 +2005,7 @@ chfsi_status cg_prepare(chfsi_ctx* ctx) {
         pe = std::max(pe, splitk_partial_elems(np, 1, (int)n));
         pe = std::max(pe, splitk_partial_elems(np, 1, np));
     }
-    if (!ctx->d_cgpart) CK(dalloc(&ctx->d_cgpart, pe));
+    if (!ctx->d_cgpart) CK(dalloc(ctx, &ctx->d_cgpart, pe));
     double sum = 0.0;
     for (double k : ctx->kin_host) sum += k;
     const double mean = n ? sum / (double)n : 0.0;
@@ -1988,9 +2014,9 @@ chfsi_status cg_prepare(chfsi_ctx* ctx) {
     if (ctx->uspp && np > 0) {
         // R = (-q^-1 - beta^H T beta)^-1 on the host (once per context)
         double2 *bt = nullptr, *part = nullptr, *cm = nullptr;
-        CK(dalloc(&bt, (size_t)np * n));
-        cudaError_t e = dalloc(&part, splitk_partial_elems(np, np, (int)n));
-        if (e == cudaSuccess) e = dalloc(&cm, (size_t)np * np);
+        CK(dalloc(ctx, &bt, (size_t)np * n));
+        cudaError_t e = dalloc(ctx, &part, splitk_partial_elems(np, np, (int)n));
+        if (e == cudaSuccess) e = dalloc(ctx, &cm, (size_t)np * np);
         if (e != cudaSuccess) {
             cudaFree(bt); cudaFree(part); cudaFree(cm);
             CK(e);
@@ -2028,7 +2054,7 @@ chfsi_status cg_prepare(chfsi_ctx* ctx) {
         // gemm_cn conjugates its first operand: store conj(R)
         std::vector<double2> rc(Q.size());
         for (size_t i = 0; i < Q.size(); ++i) rc[i] = make_double2(Q[i].real(), -Q[i].imag());
-        if (!ctx->d_cgR) CK(dalloc(&ctx->d_cgR, (size_t)np * np));
+        if (!ctx->d_cgR) CK(dalloc(ctx, &ctx->d_cgR, (size_t)np * np));
         CK(copy_sync(ctx->d_cgR, rc.data(), rc.size() * sizeof(double2), cudaMemcpyHostToDevice, ctx->st));
     }
     CK(cudaGetLastError());
@@ -2336,14 +2362,14 @@ chfsi_status chfsi_set_basis(chfsi_ctx* ctx, const int32_t* miller, const double
     if (ctx->d_work) cudaFree(ctx->d_work);
     ctx->d_col_start = ctx->d_col_pos = ctx->d_xact = nullptr;
     ctx->d_work = nullptr;
-    CK(dalloc(&ctx->d_col_start, ncol + 1));
-    CK(dalloc(&ctx->d_col_pos, ncol));
-    CK(dalloc(&ctx->d_xact, xact.size()));
-    CK(dalloc(&ctx->d_xline, xline.size()));
+    CK(dalloc(ctx, &ctx->d_col_start, ncol + 1));
+    CK(dalloc(ctx, &ctx->d_col_pos, ncol));
+    CK(dalloc(ctx, &ctx->d_xact, xact.size()));
+    CK(dalloc(ctx, &ctx->d_xline, xline.size()));
     CK(copy_sync(ctx->d_xline, xline.data(), sizeof(int) * xline.size(), cudaMemcpyHostToDevice, ctx->st));
-    CK(dalloc(&ctx->d_colidx, colidx.size()));
+    CK(dalloc(ctx, &ctx->d_colidx, colidx.size()));
     CK(copy_sync(ctx->d_colidx, colidx.data(), sizeof(int) * colidx.size(), cudaMemcpyHostToDevice, ctx->st));
-    CK(dalloc(&ctx->d_work, (size_t)(ctx->nb + 1) * nz * ncol));
+    CK(dalloc(ctx, &ctx->d_work, (size_t)(ctx->nb + 1) * nz * ncol));
     CK(copy_sync(ctx->d_col_start, col_start.data(), sizeof(int) * (ncol + 1), cudaMemcpyHostToDevice, ctx->st));
     CK(copy_sync(ctx->d_col_pos, col_pos.data(), sizeof(int) * ncol, cudaMemcpyHostToDevice, ctx->st));
     CK(copy_sync(ctx->d_xact, xact.data(), sizeof(int) * xact.size(), cudaMemcpyHostToDevice, ctx->st));
@@ -2362,8 +2388,8 @@ chfsi_status chfsi_set_basis(chfsi_ctx* ctx, const int32_t* miller, const double
                 twd[o] = make_double2(std::cos(a), std::sin(a));
                 twf[o] = make_float2((float)twd[o].x, (float)twd[o].y);
             }
-        CK(dalloc(&ctx->d_twd, twd.size()));
-        CK(dalloc(&ctx->d_twf, twf.size()));
+        CK(dalloc(ctx, &ctx->d_twd, twd.size()));
+        CK(dalloc(ctx, &ctx->d_twf, twf.size()));
         CK(copy_sync(ctx->d_twd, twd.data(), twd.size() * sizeof(double2), cudaMemcpyHostToDevice, ctx->st));
         CK(copy_sync(ctx->d_twf, twf.data(), twf.size() * sizeof(float2), cudaMemcpyHostToDevice, ctx->st));
     }
@@ -2417,8 +2443,8 @@ chfsi_status chfsi_set_projectors(chfsi_ctx* ctx, const chfsi_c128* beta,
         if (ctx->d_dmat) cudaFree(ctx->d_dmat);
         if (ctx->d_dmat0) cudaFree(ctx->d_dmat0);
         ctx->d_dmat = ctx->d_dmat0 = nullptr;
-        CK(dalloc(&ctx->d_dmat, dt));
-        CK(dalloc(&ctx->d_dmat0, dt));
+        CK(dalloc(ctx, &ctx->d_dmat, dt));
+        CK(dalloc(ctx, &ctx->d_dmat0, dt));
         ctx->n_dmat = dt;
     }
     CK(copy_sync(ctx->d_dmat, dmat, dt * sizeof(double2), cudaMemcpyHostToDevice, ctx->st));
@@ -2433,7 +2459,7 @@ chfsi_status chfsi_set_projectors(chfsi_ctx* ctx, const chfsi_c128* beta,
     } else {
         // stage in the hpsi buffer when it is large enough, else in a temporary
         double2* stage = nullptr;
-        CK(dalloc(&stage, nbeta));
+        CK(dalloc(ctx, &stage, nbeta));
         if (cudaError_t e = copy_sync(stage, beta, nbeta * sizeof(double2), cudaMemcpyHostToDevice,
                                       ctx->st)) {
             cudaFree(stage);
@@ -2461,19 +2487,19 @@ chfsi_status chfsi_set_qmat(chfsi_ctx* ctx, const chfsi_c128* qmat) {
     CK(copy_sync(doff.data(), ctx->d_doff, sizeof(int) * ni, cudaMemcpyDeviceToHost, ctx->st));
     size_t dt = 0;
     for (int i = 0; i < ni; ++i) dt += (size_t)(poff[i + 1] - poff[i]) * (poff[i + 1] - poff[i]);
-    if (!ctx->d_qmat) CK(dalloc(&ctx->d_qmat, dt));
+    if (!ctx->d_qmat) CK(dalloc(ctx, &ctx->d_qmat, dt));
     CK(copy_sync(ctx->d_qmat, qmat, dt * sizeof(double2), cudaMemcpyHostToDevice, ctx->st));
     // B = beta^H beta on the device
     double2 *part = nullptr, *dB = nullptr;
-    CK(dalloc(&part, splitk_partial_elems(np, np, ctx->n_pw)));
-    if (cudaError_t e = dalloc(&dB, (size_t)np * np)) {
+    CK(dalloc(ctx, &part, splitk_partial_elems(np, np, ctx->n_pw)));
+    if (cudaError_t e = dalloc(ctx, &dB, (size_t)np * np)) {
         cudaFree(part);
         CK(e);
     }
     gemm_cn(ctx->d_beta, ctx->n_pw, ctx->d_beta, ctx->n_pw, np, np, ctx->n_pw, part, dB, ctx->st);
     std::vector<std::complex<double>> B((size_t)np * np), Q((size_t)np * np, 0.0);
     cudaError_t e = cudaMemcpyAsync(B.data(), dB, B.size() * sizeof(double2), cudaMemcpyDeviceToHost, ctx->st);
-    if (e == cudaSuccess && !ctx->d_bmatT) e = dalloc(&ctx->d_bmatT, (size_t)np * np);
+    if (e == cudaSuccess && !ctx->d_bmatT) e = dalloc(ctx, &ctx->d_bmatT, (size_t)np * np);
     if (e == cudaSuccess) {
         count_launch();
         k_conj<<<grid_for((size_t)np * np), 256, 0, ctx->st>>>(dB, ctx->d_bmatT, (size_t)np * np);
@@ -2516,9 +2542,9 @@ chfsi_status chfsi_set_qmat(chfsi_ctx* ctx, const chfsi_c128* qmat) {
             MT[(size_t)j * np + i] = m;
         }
     }
-    if (!ctx->d_sinvT) CK(dalloc(&ctx->d_sinvT, (size_t)np * np));
-    if (!ctx->d_cq) CK(dalloc(&ctx->d_cq, (size_t)np * ctx->nb));
-    if (!ctx->d_sx) CK(dalloc(&ctx->d_sx, (size_t)ctx->nb * ctx->n_pw));
+    if (!ctx->d_sinvT) CK(dalloc(ctx, &ctx->d_sinvT, (size_t)np * np));
+    if (!ctx->d_cq) CK(dalloc(ctx, &ctx->d_cq, (size_t)np * ctx->nb));
+    if (!ctx->d_sx) CK(dalloc(ctx, &ctx->d_sx, (size_t)ctx->nb * ctx->n_pw));
     CK(copy_sync(ctx->d_sinvT, MT.data(), MT.size() * sizeof(double2), cudaMemcpyHostToDevice, ctx->st));
     ctx->uspp = true;
     return CHFSI_OK;
@@ -3041,7 +3067,7 @@ extern "C" chfsi_status chfsi_scf_run(chfsi_ctx* ctx, const chfsi_scf_params* p,
             const size_t npsi = (size_t)ctx->nb * ctx->n_pw;
             if (mixed_pass) {
                 // psi and the eigenvalues the bounds come from, for an FP64 retry
-                if (!ctx->d_psi_save) CK(dalloc(&ctx->d_psi_save, npsi + (ctx->nb + 1) / 2));
+                if (!ctx->d_psi_save) CK(dalloc(ctx, &ctx->d_psi_save, npsi + (ctx->nb + 1) / 2));
                 CK(cudaMemcpyAsync(ctx->d_psi_save, ctx->d_psi, npsi * sizeof(double2),
                                    cudaMemcpyDeviceToDevice, st));
                 CK(cudaMemcpyAsync(ctx->d_psi_save + npsi, ctx->d_eig, ctx->nb * sizeof(double),
@@ -3382,8 +3408,8 @@ extern "C" chfsi_status chfsi_set_xc(chfsi_ctx* ctx, int functional) {
         return ctx->fail(CHFSI_ERR_BAD_INPUT, "unknown exchange-correlation functional");
     cudaSetDevice(ctx->device);
     if (functional == CHFSI_XC_PBE) {
-        if (!ctx->d_gga) CK(dalloc(&ctx->d_gga, 3 * ctx->fng));
-        if (!ctx->d_gga_v1) CK(dalloc(&ctx->d_gga_v1, ctx->fng));
+        if (!ctx->d_gga) CK(dalloc(ctx, &ctx->d_gga, 3 * ctx->fng));
+        if (!ctx->d_gga_v1) CK(dalloc(ctx, &ctx->d_gga_v1, ctx->fng));
     }
     ctx->xc = functional;
     return CHFSI_OK;
@@ -3405,7 +3431,7 @@ extern "C" chfsi_status chfsi_set_ions(chfsi_ctx* ctx, int n_atoms, const double
     if (ctx->d_atom_of_ion) cudaFree(ctx->d_atom_of_ion);
     ctx->d_ion = nullptr;
     ctx->d_atom_of_ion = nullptr;
-    CK(dalloc(&ctx->d_ion, 8 * (size_t)n_atoms));
+    CK(dalloc(ctx, &ctx->d_ion, 8 * (size_t)n_atoms));
     std::vector<double> h(5 * (size_t)n_atoms);
     std::memcpy(h.data(), positions, sizeof(double) * 3 * n_atoms);
     std::memcpy(h.data() + 3 * n_atoms, zion, sizeof(double) * n_atoms);
@@ -3414,7 +3440,7 @@ extern "C" chfsi_status chfsi_set_ions(chfsi_ctx* ctx, int n_atoms, const double
     if (ctx->nions > 0) {
         std::vector<int> map(ctx->nions);
         for (int i = 0; i < ctx->nions; ++i) map[i] = i;
-        CK(dalloc(&ctx->d_atom_of_ion, ctx->nions));
+        CK(dalloc(ctx, &ctx->d_atom_of_ion, ctx->nions));
         CK(copy_sync(ctx->d_atom_of_ion, map.data(), sizeof(int) * map.size(), cudaMemcpyHostToDevice,
                      ctx->st));
     }
@@ -3457,7 +3483,7 @@ extern "C" chfsi_status chfsi_forces(chfsi_ctx* ctx, double* forces) {
                     q[(size_t)d * npw + i] = m[0] * ctx->recip[d] + m[1] * ctx->recip[3 + d] +
                                              m[2] * ctx->recip[6 + d];
             }
-            CK(dalloc(&ctx->d_qvec, q.size()));
+            CK(dalloc(ctx, &ctx->d_qvec, q.size()));
             CK(copy_sync(ctx->d_qvec, q.data(), sizeof(double) * q.size(), cudaMemcpyHostToDevice, st));
         }
         cn_product(ctx, ctx->d_beta, &ctx->i8_beta, ctx->d_psi, np, nb, npw, ctx->d_cp);
@@ -3539,8 +3565,8 @@ extern "C" chfsi_status chfsi_set_density_grid(chfsi_ctx* ctx, const int* ngrid)
             }
         }
         ctx->n_gmap = (int)wp.size();
-        CK(dalloc(&ctx->d_gmap_w, wp.size()));
-        CK(dalloc(&ctx->d_gmap_f, fp.size()));
+        CK(dalloc(ctx, &ctx->d_gmap_w, wp.size()));
+        CK(dalloc(ctx, &ctx->d_gmap_f, fp.size()));
         CK(copy_sync(ctx->d_gmap_w, wp.data(), wp.size() * sizeof(int), cudaMemcpyHostToDevice, ctx->st));
         CK(copy_sync(ctx->d_gmap_f, fp.data(), fp.size() * sizeof(int), cudaMemcpyHostToDevice, ctx->st));
     }
@@ -3572,8 +3598,8 @@ extern "C" chfsi_status chfsi_set_augmentation(chfsi_ctx* ctx, const double* pos
     ctx->ion_pos.assign(positions, positions + 3 * (size_t)ctx->nions);
     ctx->aug_width = width;
     ctx->aug = true;
-    if (!ctx->d_cion) CK(dalloc(&ctx->d_cion, (size_t)ctx->nions));
-    if (!ctx->d_vion) CK(dalloc(&ctx->d_vion, (size_t)ctx->nions));
+    if (!ctx->d_cion) CK(dalloc(ctx, &ctx->d_cion, (size_t)ctx->nions));
+    if (!ctx->d_vion) CK(dalloc(ctx, &ctx->d_vion, (size_t)ctx->nions));
     return upload_phases(ctx);
 }
 
@@ -3641,6 +3667,7 @@ extern "C" chfsi_status chfsi_batch_capture(chfsi_batch* b, int ndeg) {
             return CHFSI_ERR_BAD_INPUT;
         }
         cudaStreamSynchronize(c->st);
+        c->in_graph = true;
     }
     cudaSetDevice(b->members[0]->device);
     if (b->exec) { cudaGraphExecDestroy(b->exec); b->exec = nullptr; }

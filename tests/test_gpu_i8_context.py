@@ -193,6 +193,45 @@ def test_captured_pass_takes_new_projectors(chfsi):
     batch.run()
 
 
+def test_int8_memory_is_given_back_before_an_allocation_is_refused(chfsi, sys_kb):
+    psi = _psi(sys_kb)
+    plain = _context(chfsi, sys_kb)
+    ref_f, ref_h = plain.forces(), _apply_h(plain, psi)
+    ctx = _context(chfsi, sys_kb)
+    free = torch.cuda.mem_get_info()[0]
+    chfsi.inject_fault(chfsi.INJECT_ALLOC_FAIL, 0)
+    f = ctx.forces()  # allocates at its first call
+    chfsi.inject_fault(chfsi.INJECT_NONE)
+    assert torch.cuda.mem_get_info()[0] > free
+    assert np.abs(f - ref_f).max() <= TOL * sys_kb.n_pw * np.abs(ref_f).max()  # sums that cancel
+    out = _apply_h(ctx, psi)
+    assert _same(out, ref_h) and not bool((out == ref_h).all())
+    ctx.set_projectors(sys_kb.beta(), sys_kb.proj_offsets(), sys_kb.dmat())
+    assert bool((_apply_h(ctx, psi) == out).all())
+    # nothing left to give: the failure is reported, and the context still works
+    chfsi.inject_fault(chfsi.INJECT_ALLOC_FAIL, 0)
+    with pytest.raises(chfsi.OutOfMemory):
+        ctx.band_cg(1)
+    chfsi.inject_fault(chfsi.INJECT_NONE)
+    assert bool((_apply_h(ctx, psi) == out).all())
+
+
+def test_memory_that_a_captured_pass_uses_is_kept(chfsi, sys_kb):
+    ctx = _context(chfsi, sys_kb, precision=chfsi.PREC_MIXED)
+    ctx.set_tc_shapes(0, 0)
+    ctx.diagonalize(4, ctx.diagonalize(4))
+    psi = ctx.get_psi()
+    batch = chfsi.Batch([ctx])
+    batch.capture(4)
+    w = batch.run()[0]
+    chfsi.inject_fault(chfsi.INJECT_ALLOC_FAIL, 0)
+    with pytest.raises(chfsi.OutOfMemory):
+        ctx.forces()
+    chfsi.inject_fault(chfsi.INJECT_NONE)
+    assert np.isfinite(batch.run()[0]).all()
+    assert np.isfinite(w).all() and np.isfinite(psi).all()
+
+
 def test_scratch_of_a_process_without_contexts(chfsi):
     m, n, k = 256, 160, 20000
     a, b, c = _operands(m, n, k)
