@@ -13,7 +13,8 @@ void symmetrize(const double2* in, double2* out, int n, cudaStream_t st);
 cudaError_t chol_inv(double2* A, double2* X, int n, int* info, cudaStream_t st);
 // A = U diag(w) U^H, w ascending, U row-major with the eigenvectors as columns
 // (heev.cu), for the sizes heev_fits() says; A is kept.  sweeps_out: Jacobi
-// sweeps of the leaf problems (huge when A is not finite)
+// sweeps of the leaf problems, huge when the solve did not converge or its result
+// is not finite
 bool heev_fits(int n);
 size_t heev_scratch_doubles(int n);
 cudaError_t heev(const double2* A, int n, double* w, double2* U, double* scratch, int* sweeps_out,

@@ -35,6 +35,9 @@ namespace chfsi {
 namespace {
 
 constexpr double kEps = 1.1102230246251565e-16;  // 2^-53
+// what the sweep count says of a solve that did not converge (above any limit
+// a caller has)
+constexpr int kNoConvergence = 1 << 20;
 
 __device__ __forceinline__ double2 c_mul(double2 a, double2 b) {
     return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
@@ -698,6 +701,7 @@ struct DcWork {
 // splits subtract |e| from the two diagonal entries beside them.  One warp per
 // rotated pair, a lane per column.
 constexpr int kLeafWarps = kLeaf / 2;
+constexpr int kLeafSweeps = 30;
 __global__ void __launch_bounds__(32 * kLeafWarps) k_dc_leaf(DcWork w, int level) {
     constexpr int LS = kLeaf + 1;
     __shared__ double a[kLeaf * LS], v[kLeaf * LS];
@@ -722,7 +726,8 @@ __global__ void __launch_bounds__(32 * kLeafWarps) k_dc_leaf(DcWork w, int level
     __syncthreads();
     const int m = N + (N & 1), np = m / 2;
     int sweep = 0;
-    for (; sweep < 30; ++sweep) {
+    bool bad = false;
+    for (;; ++sweep) {
         double f = 0.0, t = 0.0;
         for (int i = warp; i < N; i += kLeafWarps) {
             const double x = lane < N ? a[i * LS + lane] * a[i * LS + lane] : 0.0;
@@ -742,6 +747,10 @@ __global__ void __launch_bounds__(32 * kLeafWarps) k_dc_leaf(DcWork w, int level
         // rotated entries are set to zero, so the sum falls quadratically well
         // below rounding; also leaves on NaN
         if (!(f > 1e-34 * t)) break;
+        if (sweep == kLeafSweeps) {
+            bad = f > 1e-28 * t;  // short of working precision, not just of its last bits
+            break;
+        }
         for (int s = 0; s < m - 1; ++s) {
             if (tid < np) {  // circle method: pair tid of step s
                 int x = tid == 0 ? 0 : tid - 1 + s, y = m - 2 - tid + s;
@@ -802,7 +811,6 @@ __global__ void __launch_bounds__(32 * kLeafWarps) k_dc_leaf(DcWork w, int level
         }
     }
     __syncthreads();
-    bool bad = false;
     for (int i = tid; i < N; i += 32 * kLeafWarps) {
         const double x = a[i * LS + i];
         bad |= !isfinite(x);
@@ -814,7 +822,7 @@ __global__ void __launch_bounds__(32 * kLeafWarps) k_dc_leaf(DcWork w, int level
         w.D[0][o + r] = x;
         for (int k = 0; k < N; ++k) w.Zt[0][(size_t)(o + r) * n + o + k] = v[k * LS + i];
     }
-    if (bad) atomicMax(w.sweeps, 1 << 20);
+    if (bad) atomicMax(w.sweeps, kNoConvergence);
     else if (tid == 0) atomicMax(w.sweeps, sweep);
 }
 
@@ -977,6 +985,7 @@ __global__ void __launch_bounds__(256) k_dc_deflate(DcWork w, int level, int par
 
 // Root j of 1/rho + sum z_i^2 / (d_i - x): one warp per root, bracketed two-pole
 // iteration on the offset from the nearer pole.
+constexpr int kSecularSteps = 100;
 __global__ void __launch_bounds__(128) k_dc_secular(DcWork w, int level) {
     const int n = w.n, t = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (t >= n) return;
@@ -1035,9 +1044,15 @@ __global__ void __launch_bounds__(128) k_dc_secular(DcWork w, int level) {
     // the two poles of the interpolation
     const double pa = d[split] - d[q], pb = d[split + 1] - d[q];
     double width = hi - lo;
-    for (int it = 0; it < 100; ++it) {
+    bool bad = false;
+    for (int it = 0;; ++it) {
         const double err = 8.0 * (fabs(psi) + fabs(phi)) + ri + fabs(mu) * (dpsi + dphi);
-        if (!(fabs(f) > kEps * err)) break;  // also leaves on NaN
+        bad = !isfinite(f);
+        if (!(fabs(f) > kEps * err) || bad) break;
+        if (it == kSecularSteps) {
+            bad = fabs(f) > 0x1p20 * kEps * err;
+            break;
+        }
         if (f < 0.0) lo = fmax(lo, mu);
         else hi = fmin(hi, mu);
         if (hi - lo <= 2.0 * kEps * fmax(fabs(lo), fabs(hi))) break;
@@ -1073,6 +1088,7 @@ __global__ void __launch_bounds__(128) k_dc_secular(DcWork w, int level) {
         w.km[t] = mu;
         w.org[t] = q;
         w.kl[t] = d[q] + mu;
+        if (bad) atomicMax(w.sweeps, kNoConvergence);
     }
 }
 
@@ -1117,6 +1133,7 @@ __global__ void __launch_bounds__(128) k_dc_vectors(DcWork w, int level, int par
             s += u * u;
         }
         s = 1.0 / sqrt(warp_add(s));
+        if (lane == 0 && !(s > 0.0 && isfinite(s))) atomicMax(w.sweeps, kNoConvergence);
         for (int i = lane; i < K; i += 32) S[i] *= s;
         x = w.kl[t];
         for (int i = lane; i < nd; i += 32) r += w.dd[o + i] < x;
@@ -1185,14 +1202,17 @@ __global__ void __launch_bounds__(256) k_dc_update(DcWork w, int level, int par)
     }
 }
 
-__global__ void k_heev1(const double2* A, double* w, double2* U) {
+__global__ void k_heev1(const double2* A, double* w, double2* U, int* sweeps) {
     w[0] = A[0].x;
     U[0] = make_double2(1.0, 0.0);
+    *sweeps = isfinite(A[0].x) ? 0 : kNoConvergence;
 }
 
-__global__ void k_copy_eig(const double* __restrict__ D, int n, double* __restrict__ w) {
+__global__ void k_copy_eig(const double* __restrict__ D, int n, double* __restrict__ w, int* sweeps) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) w[i] = D[i];
+    if (i >= n) return;
+    w[i] = D[i];
+    if (!isfinite(D[i])) atomicMax(sweeps, kNoConvergence);
 }
 
 int dc_levels(int n) {
@@ -1248,8 +1268,8 @@ cudaError_t heev(const double2* A, int n, double* w, double2* U, double* scratch
     const size_t nn = (size_t)n * n;
     if (n == 1) {
         count_launch();
-        k_heev1<<<1, 1, 0, st>>>(A, w, U);
-        return cudaMemsetAsync(sweeps_out, 0, sizeof(int), st);
+        k_heev1<<<1, 1, 0, st>>>(A, w, U, sweeps_out);
+        return cudaGetLastError();
     }
     double* s = (double*)(((uintptr_t)scratch + 15) & ~(uintptr_t)15);
     double2* Vh = (double2*)s;
@@ -1320,7 +1340,7 @@ cudaError_t heev(const double2* A, int n, double* w, double2* U, double* scratch
         k_dc_vectors<<<(n + 3) / 4, 128, 0, st>>>(q, l, par);
         k_dc_update<<<dim3((most + 63) / 64, (most + 31) / 32, 1 << l), 256, 0, st>>>(q, l, par);
     }
-    k_copy_eig<<<(n + 255) / 256, 256, 0, st>>>(q.D[par], n, w);
+    k_copy_eig<<<(n + 255) / 256, 256, 0, st>>>(q.D[par], n, w, sweeps_out);
     // ---- U = Q Z
     k_wy<<<((n + kGrp - 1) / kGrp + 3) / 4, 128, 0, st>>>(Vh, tau, n, Tg);
     if (n <= 32) return launch_back<1>(Vh, Tg, q.Zt[par], n, U, st);

@@ -121,3 +121,16 @@ def test_errors(chfsi, n):
     h = (h + h.mH) / 2
     w, v = _solve(chfsi, h, s)
     _check(h, s, w, v, 1.0)
+
+
+@pytest.mark.parametrize("n", [1, 2, 24, 25, 160, 300])
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), -float("inf")])
+def test_non_finite_h_is_reported(chfsi, n, value):
+    """Whatever the solver makes of it, an eigenvalue that is not a number does not
+    come back as a success; n = 1 has no iteration that could notice."""
+    s = torch.eye(n, dtype=torch.complex128, device="cuda")
+    h = _gauss(n, 5)
+    h = (h + h.mH) / 2
+    h[n // 2, n // 2] = value
+    with pytest.raises(chfsi.RayleighRitzFailed, match="did not converge"):
+        _solve(chfsi, h, s)
