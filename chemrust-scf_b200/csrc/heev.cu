@@ -277,7 +277,21 @@ k_chol_inv(double2* A, double2* X, int n, int* info) {
 // thread-block cluster (n <= 256): a cheaper barrier (390 clocks, the grid's
 // takes 2,300), q and a pushed into every block's shared memory instead of the
 // round trip through L2.
-// Columns with |x|^2 < 1e-280 count as zero.
+// The rows are scaled by a power of two to a largest entry next to 1 (its top word
+// in *top, zero before the launch; the eigenvalues are scaled back at the end), and
+// columns with |x|^2 < 1e-140 then count as zero: sigma is about 1 / |x|^2, and its
+// square and beta |u|^2 leave the range of the exponents for |x| below 1e-77 and
+// above 1e77 otherwise.
+__device__ __forceinline__ unsigned tri_top(double2 v) {
+    const unsigned x = ((unsigned)__double2hiint(v.x) & 0x7fffffffu) | (__double2loint(v.x) != 0);
+    const unsigned y = ((unsigned)__double2hiint(v.y) & 0x7fffffffu) | (__double2loint(v.y) != 0);
+    return max(x, y);
+}
+__device__ __forceinline__ double tri_scale(unsigned top) {
+    const int f = (int)(top >> 20);
+    if (top == 0 || f == 2047) return 1.0;
+    return __longlong_as_double((long long)max(1, 2046 - f) << 52);
+}
 constexpr int kTriPer = 5;  // vector entries per thread (n <= 5 x 256)
 constexpr int kTriCluster = 256;  // largest n of the cluster form
 template <bool CL> struct TriCfg {
@@ -289,7 +303,7 @@ template <bool CL> struct TriCfg {
 template <bool CL>
 __global__ void __launch_bounds__(TriCfg<CL>::threads)
 k_tridiag(const double2* __restrict__ A, int n, int rows, double2* Vh, double2* tau, double* d,
-          double* e, double2* P) {
+          double* e, double2* P, unsigned* top) {
     constexpr int T = TriCfg<CL>::threads, W = T / 32, KP = TriCfg<CL>::per;
     extern __shared__ double2 tsm[];
     double2* M = tsm;                      // own rows
@@ -313,26 +327,41 @@ k_tridiag(const double2* __restrict__ A, int n, int rows, double2* Vh, double2* 
         rb ^= 1;
         return v;
     };
+    unsigned big = 0;
     for (int l = 0; l < rows; ++l) {
         const int i = rank + l * G;
         if (i < n)
-            for (int k = tid; k < n; k += T) M[(size_t)l * n + k] = A[(size_t)i * n + k];
+            for (int k = tid; k < n; k += T) {
+                const double2 v = A[(size_t)i * n + k];
+                M[(size_t)l * n + k] = v;
+                big = max(big, tri_top(v));
+            }
     }
+    big = __reduce_max_sync(0xffffffffu, big);
+    if (lane == 0) atomicMax(top, big);
+    __threadfence();
+    // also: a block's shared memory may be stored to only once the block runs
+    if constexpr (CL) cg::this_cluster().sync();
+    else cg::this_grid().sync();
+    const double scale = tri_scale(__ldcg(top));
+    for (int l = 0; l < rows; ++l)
+        if (rank + l * G < n)
+            for (int k = tid; k < n; k += T) {
+                M[(size_t)l * n + k].x *= scale;
+                M[(size_t)l * n + k].y *= scale;
+            }
     const int wpr = rows <= W ? W / rows : 1, rpp = W / wpr;  // warps per row, rows at a time
     double2 x[KP];
 #pragma unroll
     for (int q = 0; q < KP; ++q) {
         const int k = tid + q * T;
         x[q] = make_double2(0.0, 0.0);
-        if (k > 0 && k < n) { x[q] = A[k]; x[q].y = -x[q].y; }
+        if (k > 0 && k < n) x[q] = make_double2(A[k].x * scale, -A[k].y * scale);
         if (k < n) xc[k] = k > 1 ? x[q] : make_double2(0.0, 0.0);
     }
-    double2 alpha = A[1];  // x_{j+1}
-    alpha.y = -alpha.y;
-    double dj = A[0].x;
-    // a block's shared memory may be stored to only once the block runs
-    if constexpr (CL) cg::this_cluster().sync();
-    else __syncthreads();
+    double2 alpha = make_double2(A[1].x * scale, -A[1].y * scale);  // x_{j+1}
+    double dj = A[0].x * scale;
+    __syncthreads();
     for (int j = 0; j < n - 1; ++j) {
         double2* Pj = (CL ? pl : P) + (size_t)(j & 1) * 2 * n;
         for (int l0 = 0; l0 < rows; l0 += rpp) {
@@ -420,7 +449,7 @@ k_tridiag(const double2* __restrict__ A, int n, int rows, double2* Vh, double2* 
             }
             v = sum(v);
             const double s2 = alpha.x * alpha.x + alpha.y * alpha.y + v;
-            if ((v != 0.0 || alpha.y != 0.0) && !(s2 < 1e-280)) {
+            if ((v != 0.0 || alpha.y != 0.0) && !(s2 < 1e-140)) {
                 beta = -copysign(s2 * rsqrt(s2), alpha.x);
                 u0 = make_double2(alpha.x - beta, alpha.y);
                 const double q = -1.0 / (beta * (u0.x * u0.x + u0.y * u0.y));
@@ -1208,10 +1237,11 @@ __global__ void k_heev1(const double2* A, double* w, double2* U, int* sweeps) {
     *sweeps = isfinite(A[0].x) ? 0 : kNoConvergence;
 }
 
-__global__ void k_copy_eig(const double* __restrict__ D, int n, double* __restrict__ w, int* sweeps) {
+__global__ void k_copy_eig(const double* __restrict__ D, int n, const unsigned* __restrict__ top,
+                           double* __restrict__ w, int* sweeps) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    w[i] = D[i];
+    w[i] = D[i] / tri_scale(*top);
     if (!isfinite(D[i])) atomicMax(sweeps, kNoConvergence);
 }
 
@@ -1283,6 +1313,7 @@ cudaError_t heev(const double2* A, int n, double* w, double2* U, double* scratch
     auto take = [&](size_t k) { double* p = at; at += k; return p; };
     q.Zt[0] = take(nn);
     q.Zt[1] = take(nn);
+    unsigned* top = (unsigned*)take(1);
     q.S = take(nn);
     double** vecs[] = {&q.d, &q.e, &q.D[0], &q.D[1], &q.kd, &q.kz, &q.kl, &q.km, &q.zh, &q.dd, &q.rho};
     for (double** v : vecs) *v = take(n);
@@ -1290,7 +1321,7 @@ cudaError_t heev(const double2* A, int n, double* w, double2* U, double* scratch
     for (int** v : ints) *v = (int*)take(n);
     q.sweeps = sweeps_out;
     cudaError_t e = cudaMemsetAsync(sweeps_out, 0, sizeof(int), st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(q.Zt[0], 0, 2 * nn * sizeof(double), st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(q.Zt[0], 0, (2 * nn + 1) * sizeof(double), st);
     if (e != cudaSuccess) return e;
     // ---- A = Q T Q^H
     count_launch();
@@ -1314,13 +1345,13 @@ cudaError_t heev(const double2* A, int n, double* w, double2* U, double* scratch
         int clusters = 0;
         if (p.smem <= kTriSmem &&
             cudaOccupancyMaxActiveClusters(&clusters, k_tridiag<true>, &lc) == cudaSuccess && clusters >= 1)
-            done = cudaLaunchKernelEx(&lc, k_tridiag<true>, A, n, p.rows, Vh, tau, q.d, q.e, P) == cudaSuccess;
+            done = cudaLaunchKernelEx(&lc, k_tridiag<true>, A, n, p.rows, Vh, tau, q.d, q.e, P, top) == cudaSuccess;
         cudaGetLastError();  // a refused configuration: the grid version
     }
     if (!done) {
         TriPlan p = tri_plan(n, std::min(device_sms(), std::max(1, (n + 3) / 4)), TriCfg<false>::vectors);
         if ((e = raise_smem_limit(k_tridiag<false>, p.smem)) != cudaSuccess) return e;
-        void* args[] = {&A, &n, &p.rows, &Vh, &tau, &q.d, &q.e, &P};
+        void* args[] = {&A, &n, &p.rows, &Vh, &tau, &q.d, &q.e, &P, &top};
         e = cudaLaunchCooperativeKernel((const void*)k_tridiag<false>, dim3(p.blocks),
                                         dim3(TriCfg<false>::threads), args, p.smem, st);
         if (e != cudaSuccess) return e;
@@ -1340,7 +1371,7 @@ cudaError_t heev(const double2* A, int n, double* w, double2* U, double* scratch
         k_dc_vectors<<<(n + 3) / 4, 128, 0, st>>>(q, l, par);
         k_dc_update<<<dim3((most + 63) / 64, (most + 31) / 32, 1 << l), 256, 0, st>>>(q, l, par);
     }
-    k_copy_eig<<<(n + 255) / 256, 256, 0, st>>>(q.D[par], n, w, sweeps_out);
+    k_copy_eig<<<(n + 255) / 256, 256, 0, st>>>(q.D[par], n, top, w, sweeps_out);
     // ---- U = Q Z
     k_wy<<<((n + kGrp - 1) / kGrp + 3) / 4, 128, 0, st>>>(Vh, tau, n, Tg);
     if (n <= 32) return launch_back<1>(Vh, Tg, q.Zt[par], n, U, st);

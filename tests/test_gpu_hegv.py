@@ -134,3 +134,30 @@ def test_non_finite_h_is_reported(chfsi, n, value):
     h[n // 2, n // 2] = value
     with pytest.raises(chfsi.RayleighRitzFailed, match="did not converge"):
         _solve(chfsi, h, s)
+
+
+@pytest.mark.parametrize("n", [2, 5, 20, 60, 160, 300])
+@pytest.mark.parametrize("exponent", [-480, -300, -200, 200, 300, 480])
+def test_scaled_matrix(chfsi, n, exponent):
+    """A power of two on H goes through to the eigenvalues, whatever squares and
+    cubes of its entries do to the range of the exponents."""
+    h = _gauss(n, n + 3)
+    h = (h + h.mH) / 2
+    s = torch.eye(n, dtype=torch.complex128, device="cuda")
+    w0, v0 = _solve(chfsi, h, s)
+    _check(h, s, w0, v0, 1.0)
+    w, v = _solve(chfsi, h * 2.0 ** exponent, s)
+    assert float((w * 2.0 ** -exponent - w0).abs().max()) <= 40 * n * EPS * float(w0.abs().max())
+    _check(h, s, w * 2.0 ** -exponent, v, 1.0)
+
+
+@pytest.mark.parametrize("n", [20, 60, 160, 300])
+@pytest.mark.parametrize("size", [1e-60, 1e-80, 1e-100, 1e-130])
+def test_blocks_with_a_negligible_coupling(chfsi, n, size):
+    h = size * _gauss(n, 9)
+    for i in range(0, n, 7):
+        h[i:i + 7, i:i + 7] = _gauss(min(7, n - i), i + 1)
+    h = (h + h.mH) / 2
+    s = torch.eye(n, dtype=torch.complex128, device="cuda")
+    w, v = _solve(chfsi, h, s)
+    _check(h, s, w, v, 1.0)
