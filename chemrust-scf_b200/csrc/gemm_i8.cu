@@ -39,6 +39,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 
 namespace chfsi {
 
@@ -54,6 +55,8 @@ constexpr int kRing = 4;
 constexpr int kEpiThreads = 256, kThreads = 320;
 constexpr int kMaxSpc = kI8MaxK / kSlab;
 constexpr int kNonFinite = 1 << 20;           // exponent mark of a row with inf or NaN
+constexpr int kZeroRow = -2000;               // and of one of zeros
+constexpr int kPlainExp = 900;
 
 constexpr size_t kSmemBytes = 1024 + (size_t)kRing * kStageBytes + 128;
 
@@ -147,13 +150,24 @@ __device__ __forceinline__ void tmem_ld4(uint32_t taddr, int* r) {
                  : "r"(taddr));
 }
 
-// 2^p for -1022 <= p <= 1023
+// 2^p for -1022 <= p <= 1023, inf for 1024
 __device__ __forceinline__ double pow2(int p) { return __longlong_as_double((long long)(p + 1023) << 52); }
-// 2^(E - 33), or NaN for a row with an inf or NaN; E >= -1022, so the smallest
-// is a denormal, still a power of two
+// 2^(E - 33) for |E| <= kPlainExp; NaN for a row with an inf or NaN, and 1 for a
+// row of zeros
 __device__ __forceinline__ double side_scale(int e) {
     if (e == kNonFinite) return __longlong_as_double(0x7ff8000000000000LL);
-    return e > -900 ? pow2(e - 33) : pow2(e + 67) * pow2(-100);
+    return e == kZeroRow ? 1.0 : pow2(max(e - 33, -1022));
+}
+// rows whose scale is not multiplied on its own: it may leave the range of the
+// exponents where the product with another row's does not
+__device__ __forceinline__ bool far_row(int e) {
+    return e != kZeroRow && e != kNonFinite && (e > kPlainExp || e < -kPlainExp);
+}
+// 2^e v, |v| < 2^80, e the sum of two rows' exponents; 0 times inf, NaN, when one
+// is kNonFinite
+__device__ __forceinline__ double scale_by(double v, int e) {
+    const int h = min(max(e >> 1, -700), 1024);
+    return v * pow2(h) * pow2(min(max(e - h, -700), 1024));
 }
 
 // x as a double, |x| < 2^51: through the exponent bits of 2^52 + 2^51, one add
@@ -318,16 +332,17 @@ k_umma_i8(I8Side a, I8Side b, int M, int N, int mt, int per_chunk, int items, in
             i8_item(item, per_chunk, mt, b.tiles, herm, c, tm, tn);
             const int i = tm * kTM + lq * 32 + lane, j0 = tn * kTN + half * 32;
             // X = x 2^(61 - E) and the digits' 256^7: products carry 2^(EA + EB - 66)
-            const double fa = side_scale(a.exps[(size_t)(a.chunk0 + c) * a.rows_pad + i]);
-            const double fb_lane = side_scale(b.exps[(size_t)(b.chunk0 + c) * b.rows_pad + j0 + lane]);
+            const int ea = a.exps[(size_t)(a.chunk0 + c) * a.rows_pad + i];
+            const int eb_lane = b.exps[(size_t)(b.chunk0 + c) * b.rows_pad + j0 + lane];
+            const double fa = side_scale(ea), fb_lane = side_scale(eb_lane);
+            const bool far = __any_sync(0xffffffffu, far_row(ea) || far_row(eb_lane));
             double2* o = out + (long long)c * chunk_stride + (long long)j0 * ldo + i;
             const int cols = i < M ? N - j0 : 0;
-#pragma unroll 1
-            for (int part = 0; part < 3; ++part, ++pc) {
-                if (lane == 0) ok = mbar_wait_or(acc_full, pc & 1, wait_ns, abort_flag);
-                ok = __shfl_sync(0xffffffffu, ok, 0);  // tcgen05.ld is warp-collective
-                if (!ok) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            // the accumulators of one part; FAR: some row of the warp's is far_row (a
+            // loop of its own, as a branch per element keeps the compiler from
+            // interleaving them: 10 % of a launch)
+            auto convert = [&](auto is_far, int part) {
+                constexpr bool FAR = decltype(is_far)::value;
                 int I[2][kDig][4];
 #pragma unroll
                 for (int d = 0; d < kDig; ++d) tmem_ld4(tl + (uint32_t)(d * kTN), I[0][d]);
@@ -346,11 +361,12 @@ k_umma_i8(I8Side a, I8Side b, int M, int N, int mt, int per_chunk, int items, in
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
                         const int jj = g * 4 + q;
-                        const double fb = __shfl_sync(0xffffffffu, fb_lane, jj);
                         int v[kDig];
 #pragma unroll
                         for (int d = 0; d < kDig; ++d) v[d] = I[g & 1][d][q];
-                        const double t = i8_value(v) * fa * fb;
+                        double t = i8_value(v);
+                        if constexpr (FAR) t = scale_by(t, ea + __shfl_sync(0xffffffffu, eb_lane, jj) - 66);
+                        else t = t * fa * __shfl_sync(0xffffffffu, fb_lane, jj);
                         // conj: re = T1 + T2, im = T3 + (T2 - T1); else re = T1 - T2,
                         // im = T3 + (-T2 - T1)
                         const double r = fma(part == 1 ? sgn : 1.0, t, keep[jj]);
@@ -362,6 +378,15 @@ k_umma_i8(I8Side a, I8Side b, int M, int N, int mt, int per_chunk, int items, in
                         if (put) *e = fma(beta, old, alpha * r);
                     }
                 }
+            };
+#pragma unroll 1
+            for (int part = 0; part < 3; ++part, ++pc) {
+                if (lane == 0) ok = mbar_wait_or(acc_full, pc & 1, wait_ns, abort_flag);
+                ok = __shfl_sync(0xffffffffu, ok, 0);  // tcgen05.ld is warp-collective
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (far) convert(std::true_type{}, part);
+                else convert(std::false_type{}, part);
             }
         }
         if (!ok && lane == 0) {
@@ -413,13 +438,16 @@ __device__ __forceinline__ void store16(const long long* x, int8_t* dst, int pla
         *reinterpret_cast<uint4*>(dst + (size_t)p * plane_bytes) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
 }
 
+// high word without the sign; its last bit is set for any number but zero
 __device__ __forceinline__ unsigned int top_word(double2 v) {
-    return max((unsigned)__double2hiint(v.x) & 0x7fffffffu, (unsigned)__double2hiint(v.y) & 0x7fffffffu);
+    const unsigned x = ((unsigned)__double2hiint(v.x) & 0x7fffffffu) | (__double2loint(v.x) != 0);
+    const unsigned y = ((unsigned)__double2hiint(v.y) & 0x7fffffffu) | (__double2loint(v.y) != 0);
+    return max(x, y);
 }
 // largest top word of a row part -> exponent E with |x| < 2^E
 __device__ __forceinline__ int row_exponent(unsigned int top) {
     const int f = (int)(top >> 20);
-    return f == 2047 ? kNonFinite : f - 1022;
+    return f == 2047 ? kNonFinite : top == 0 ? kZeroRow : f - 1022;
 }
 
 // round to nearest of v, |v| < 2^61, in two 31-bit steps on the FP64 pipe

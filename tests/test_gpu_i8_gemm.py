@@ -106,3 +106,26 @@ def test_same_inputs_same_bits(chfsi):
     c, _ = _cn(chfsi, a, b)
     d, _ = _cn(chfsi, a, b)
     assert bool((c == d).all())
+
+
+def test_rows_at_both_ends_of_the_exponents(chfsi):
+    """A row near 2^1000 times one near 2^-1000 is an ordinary number."""
+    m, n, k = 256, 192, 20000
+    a, b = _gauss((m, k), 12), _gauss((n, k), 13)
+    ref, norm = a.conj() @ b.T, _norms(a, b)
+    ea = torch.zeros(m, dtype=torch.int64, device="cuda")
+    eb = torch.zeros(n, dtype=torch.int64, device="cuda")
+    ea[1:4] = torch.tensor([990, -1000, 970])
+    eb[1:4] = torch.tensor([-990, 1000, -1005])
+
+    def scaled(x, e):
+        two = torch.tensor(2.0, dtype=torch.float64, device="cuda")
+        return x * two ** (e // 2) * two ** (e - e // 2)
+
+    c, launches = _cn(chfsi, scaled(a, ea[:, None]), scaled(b, eb[None, :].T))
+    assert launches == 4
+    e = ea[:, None] + eb[None, :]
+    ordinary = e.abs() <= 1000
+    assert bool(ordinary[1, 1] and ordinary[2, 2] and ordinary[3, 3])
+    err = (scaled(c, torch.where(ordinary, -e, 0)) - ref).abs() / norm
+    assert float(err[ordinary].max()) < TOL
