@@ -3887,8 +3887,9 @@ extern "C" chfsi_status chfsi_mixer_samples(chfsi_ctx* ctx, const double* rho_in
 constexpr int kGemmMaxK = 1 << 30;
 
 // Runs an INT8-path product with scratch of its own on `st` and waits for it.
-// *done stays false, with nothing launched, where the scratch is not to be had
-// or too small: the caller then takes the FP64 tensor path.
+// *done stays false where the scratch is not to be had or too small, with nothing
+// launched, and where the product came back unresolved: the caller then takes the
+// FP64 tensor path.
 template <typename F>
 static chfsi_status with_i8_scratch(size_t want, cudaStream_t st, bool* done, F&& product) {
     const size_t bytes = std::min(want, kScratchKeep - 256);
@@ -3897,19 +3898,20 @@ static chfsi_status with_i8_scratch(size_t want, cudaStream_t st, bool* done, F&
         cudaGetLastError();
         return CHFSI_OK;
     }
-    int* err = (int*)(buf + bytes);
-    int herr = 0;
-    cudaError_t e = cudaMemsetAsync(err, 0, sizeof(int), st);
-    if (e == cudaSuccess) *done = product(buf, bytes, err);
+    int* words = (int*)(buf + bytes);  // time-out, unresolved
+    int h[2] = {0, 0};
+    cudaError_t e = cudaMemsetAsync(words, 0, sizeof(h), st);
+    if (e == cudaSuccess) *done = product(buf, bytes, words, words + 1);
     if (*done) e = cudaGetLastError();
-    if (*done && e == cudaSuccess) e = cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, st);
+    if (*done && e == cudaSuccess) e = cudaMemcpyAsync(h, words, sizeof(h), cudaMemcpyDeviceToHost, st);
     scratch_free(buf, st);
     if (*done && e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_fail(e, "INT8-path product", __FILE__, __LINE__);
-    if (herr) {
+    if (h[0]) {
         g_last_error = "tensor-core GEMM pipeline wait timed out";
         return CHFSI_ERR_TIMEOUT;
     }
+    if (h[1]) *done = false;
     return CHFSI_OK;
 }
 
@@ -3932,9 +3934,9 @@ extern "C" chfsi_status chfsi_zgemm_cn(const chfsi_c128* a_dev, int lda, const c
     double2* c = reinterpret_cast<double2*>(c_dev);
     if (i8_cn_pays(m, n, k, false, false)) {
         bool done = false;
-        chfsi_status s = with_i8_scratch(i8_cn_scratch_bytes(m, n, k, false), st, &done,
-                                         [&](void* buf, size_t bytes, int* err) {
-            return gemm_cn_i8(a, lda, nullptr, b, ldb, m, n, k, false, buf, bytes, c, err, st);
+        chfsi_status s = with_i8_scratch(i8_cn_scratch_bytes(m, n, k, false, true), st, &done,
+                                         [&](void* buf, size_t bytes, int* err, int* unresolved) {
+            return gemm_cn_i8(a, lda, nullptr, b, ldb, m, n, k, false, buf, bytes, c, err, st, unresolved);
         });
         if (s || done) return s;
     }
@@ -4022,9 +4024,10 @@ extern "C" chfsi_status chfsi_zgemm_tn(const chfsi_c128* w_dev, int ldw, const c
     double2* o = reinterpret_cast<double2*>(o_dev);
     if (i8_tn_pays(m, n, k, false)) {
         bool done = false;
-        chfsi_status s = with_i8_scratch(i8_tn_scratch_bytes(m, n, k, false), st, &done,
-                                         [&](void* buf, size_t bytes, int* err) {
-            return gemm_tn_i8(w, ldw, x, ldx, nullptr, o, ldo, m, n, k, alpha, beta, buf, bytes, err, st);
+        chfsi_status s = with_i8_scratch(i8_tn_scratch_bytes(m, n, k, false, true), st, &done,
+                                         [&](void* buf, size_t bytes, int* err, int* unresolved) {
+            return gemm_tn_i8(w, ldw, x, ldx, nullptr, o, ldo, m, n, k, alpha, beta, buf, bytes, err, st,
+                              unresolved);
         });
         if (s || done) return s;
     }

@@ -12,16 +12,26 @@
 //     digits, X = sum_i d_i 256^(7-i).  A row's own 53 bits survive for every
 //     element above 2^-8 of its largest.
 //   * X Y = sum_{i,j} d_i e_j 256^(14-i-j); the 36 products with i + j <= 7
-//     are kept (the first one left out is 2^-62 of the largest product), those
-//     of one i + j in one INT32 accumulator: eight accumulators of 64 columns
-//     fill the 512 TMEM columns of an SM.  8 products x 2^14 x 8192 terms < 2^31.
+//     are kept, those of one i + j in one INT32 accumulator: eight accumulators
+//     of 64 columns fill the 512 TMEM columns of an SM.  8 products x 2^14 x 8192
+//     terms < 2^31.
 //   * Complex products in the three-multiplication form of the DMMA kernels,
 //     the parts of (re, im, re -+ im) sliced as integers:
 //       conj(a) b: T1 = ar br, T2 = ai bi, T3 = (ar - ai)(br + bi)
 //       a b:       T1, T2 as above,        T3 = (ar + ai)(br + bi)
-//   * The sums over K inside a chunk are exact, so what rounding remains is
-//     that of the digits and of the final FP64 sums: smaller than the FP64
-//     accumulation it replaces (relative errors at i8_cn_pays).
+//   * The sums over K inside a chunk are exact.  What remains, in units of 2^(EA +
+//     EB): the products with i + j = 8, seven of at most 2^14 256^6, and the
+//     rounding of the digits, together at most 2^-57 per term of T1 and T2 and
+//     2^-55 of the complex product; over random digits about 2^-59 sqrt(K) in
+//     all.  That is below K 2^-53 |a||b| (2-norms of the rows) always, and measured
+//     below the FP64 accumulation it replaces (i8_cn_pays), but it is relative to
+//     the rows' largest parts: where the large elements of one row meet only small
+//     ones of the other, FP64 keeps more.  A caller whose result is to hold
+//     element by element has that looked at (`unresolved`): a fourth part
+//     multiplies the magnitudes, the top 7 bits of max(|re|, |im|), in one digit;
+//     sum |a||b| is at least that sum, so that from a quarter of 2^(EA + EB) on
+//     the error is at most K 2^-53 sum |a||b|, FP64's own bound.  Costs a
+//     twentieth of a launch.
 //
 // Kernel (one persistent CTA per SM, work items = 128 x 64 output tile x K
 // chunk, three parts each): warp 8 copies operand blocks, warp 9 issues the
@@ -60,8 +70,12 @@ constexpr int kPlainExp = 900;
 
 constexpr size_t kSmemBytes = 1024 + (size_t)kRing * kStageBytes + 128;
 
+// magnitudes: 2^7 per side, a quarter of the product of the two
+constexpr int kResolved = 1 << 12;
+constexpr int kParts = 3, kMagPart = 3;       // re, im, re -+ im; magnitudes
+
 struct I8Side {
-    const int8_t* data;
+    const int8_t *data, *mag;
     const int* exps;
     int tiles, rows_pad, nslab, slab0, chunk0;
 };
@@ -201,10 +215,13 @@ __device__ __forceinline__ void i8_item(int item, int per_chunk, int mt, int nt,
     tm = t;
 }
 
+// parts p0 .. p1 - 1 of every item; nothing when *gate is set
 __global__ void __launch_bounds__(kThreads, 1)
-k_umma_i8(I8Side a, I8Side b, int M, int N, int mt, int per_chunk, int items, int nslab, int spc,
+k_umma_i8(I8Side a, I8Side b, int p0, int p1, int M, int N, int mt, int per_chunk, int items, int nslab, int spc,
           int conj, int herm, double2* __restrict__ out, long long ldo, long long chunk_stride,
-          double alpha, double beta, int* err, unsigned long long wait_ns, int no_loads) {
+          double alpha, double beta, int* err, int* unresolved, const int* gate,
+          unsigned long long wait_ns, int no_loads) {
+    if (gate && *gate) return;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint64_t* full = (uint64_t*)(base + kRing * kStageBytes);
@@ -246,10 +263,16 @@ k_umma_i8(I8Side a, I8Side b, int M, int N, int mt, int per_chunk, int items, in
                 int c, tm, tn;
                 i8_item(item, per_chunk, mt, b.tiles, herm, c, tm, tn);
                 const int s0 = c * spc, s1 = min(nslab, s0 + spc);
-                for (int part = 0; part < 3 && ok; ++part) {
-                    const int8_t* pa = a.data + (((size_t)part * a.tiles + tm) * a.nslab + a.slab0 + s0) * kABytes;
-                    const int8_t* pb = b.data + (((size_t)part * b.tiles + tn) * b.nslab + b.slab0 + s0) * kBBytes;
-                    for (int s = s0; s < s1; ++s, ++issued, pa += kABytes, pb += kBBytes) {
+                for (int part = p0; part < p1 && ok; ++part) {
+                    // magnitudes: one digit, kDig slabs to a stage
+                    const bool mag = part == kMagPart;
+                    const int step = mag ? kDig : 1;
+                    const size_t ta = (size_t)tm * a.nslab + a.slab0 + s0, tb = (size_t)tn * b.nslab + b.slab0 + s0;
+                    const int8_t* pa = mag ? a.mag + ta * (kABytes / kDig)
+                                           : a.data + ((size_t)part * a.tiles * a.nslab + ta) * kABytes;
+                    const int8_t* pb = mag ? b.mag + tb * (kBBytes / kDig)
+                                           : b.data + ((size_t)part * b.tiles * b.nslab + tb) * kBBytes;
+                    for (int s = s0; s < s1; s += step, ++issued, pa += kABytes, pb += kBBytes) {
                         const int slot = issued % kRing;
                         if (!mbar_wait_or(&empty[slot], ((issued / kRing) & 1) ^ 1, wait_ns, abort_flag)) {
                             report(err, 1);
@@ -258,9 +281,10 @@ k_umma_i8(I8Side a, I8Side b, int M, int N, int mt, int per_chunk, int items, in
                             break;
                         }
                         unsigned char* dst = base + (size_t)slot * kStageBytes;
-                        mbar_expect_tx(&full[slot], kStageBytes);
-                        bulk_load(dst, pa, kABytes, &full[slot]);
-                        bulk_load(dst + kABytes, pb, kBBytes, &full[slot]);
+                        const int planes = mag ? min(kDig, s1 - s) : kDig;
+                        mbar_expect_tx(&full[slot], planes * (kStageBytes / kDig));
+                        bulk_load(dst, pa, planes * (kABytes / kDig), &full[slot]);
+                        bulk_load(dst + kABytes, pb, planes * (kBBytes / kDig), &full[slot]);
                     }
                 }
             }
@@ -279,7 +303,8 @@ k_umma_i8(I8Side a, I8Side b, int M, int N, int mt, int per_chunk, int items, in
         for (int item = blockIdx.x; item < items; item += gridDim.x) {
             int c, tm, tn;
             i8_item(item, per_chunk, mt, b.tiles, herm, c, tm, tn);
-            total += 3 * (min(nslab, (c + 1) * spc) - c * spc);
+            const int n = min(nslab, (c + 1) * spc) - c * spc;
+            total += max(0, min(p1, kParts) - p0) * n + (p1 > kMagPart ? (n + kDig - 1) / kDig : 0);
         }
         // the whole warp waits, and goes on or gives up together
         auto wait = [&](uint64_t* bar, uint32_t parity) {
@@ -291,9 +316,27 @@ k_umma_i8(I8Side a, I8Side b, int M, int N, int mt, int per_chunk, int items, in
             int c, tm, tn;
             i8_item(item, per_chunk, mt, b.tiles, herm, c, tm, tn);
             const int n = min(nslab, (c + 1) * spc) - c * spc;
-            for (int part = 0; part < 3 && ok; ++part, ++pc) {
+            for (int part = p0; part < p1 && ok; ++part, ++pc) {
                 if (!(ok = wait(acc_free, (pc & 1) ^ 1))) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (part == kMagPart) {
+                    for (int s = 0; s < n && ok; s += kDig, ++it) {
+                        const int slot = it % kRing;
+                        const uint32_t sa = smem_u32(base + (size_t)slot * kStageBytes);
+                        const uint64_t da = i8_desc(sa, kTM), db = i8_desc(sa + kABytes, kTN);
+                        const int planes = min(kDig, n - s);
+                        if (elect_one()) {
+                            for (int j = 0; j < planes; ++j)
+                                umma_i8<0>(tmem, da + (uint64_t)(j * (kTM * kSlab / 16)),
+                                           db + (uint64_t)(j * (kTN * kSlab / 16)), idesc_i8(kTM, kTN),
+                                           s + j > 0 ? 1u : 0u);
+                            umma_commit(&empty[slot]);
+                        }
+                        if (it + 1 < total) ok = wait(&full[(it + 1) % kRing], ((it + 1) / kRing) & 1);
+                    }
+                    if (ok && elect_one()) umma_commit(acc_full);
+                    continue;
+                }
                 for (int s = 0; s < n && ok; ++s, ++it) {
                     const int slot = it % kRing;
                     const uint32_t sa = smem_u32(base + (size_t)slot * kStageBytes);
@@ -380,12 +423,28 @@ k_umma_i8(I8Side a, I8Side b, int M, int N, int mt, int per_chunk, int items, in
                 }
             };
 #pragma unroll 1
-            for (int part = 0; part < 3; ++part, ++pc) {
+            for (int part = p0; part < p1; ++part, ++pc) {
                 if (lane == 0) ok = mbar_wait_or(acc_full, pc & 1, wait_ns, abort_flag);
                 ok = __shfl_sync(0xffffffffu, ok, 0);  // tcgen05.ld is warp-collective
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (far) convert(std::true_type{}, part);
+                if (part == kMagPart) {
+                    // rows of zeros give exact zeros, rows with an inf or NaN give NaN
+                    const bool row = i < M && ea != kZeroRow && ea != kNonFinite;
+                    const unsigned colm = __ballot_sync(0xffffffffu, j0 + lane < N && eb_lane != kZeroRow &&
+                                                                         eb_lane != kNonFinite);
+                    int L[8][4];
+#pragma unroll
+                    for (int g = 0; g < 8; ++g) tmem_ld4(tl + (uint32_t)(g * 4), L[g]);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(acc_free);
+                    bool low = false;
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) low |= L[j >> 2][j & 3] < kResolved && ((colm >> j) & 1u);
+                    if (__any_sync(0xffffffffu, row && low) && lane == 0) *(volatile int*)unresolved = 1;
+                } else if (far) convert(std::true_type{}, part);
                 else convert(std::false_type{}, part);
             }
         }
@@ -460,6 +519,11 @@ __device__ __forceinline__ long long round61(double v) {
            (__double_as_longlong(tl) - 0x4338000000000000LL);
 }
 
+// top 7 of the 61 bits of the larger part
+__device__ __forceinline__ uint32_t magnitude(long long xr, long long xi) {
+    return (uint32_t)(max(xr < 0 ? -xr : xr, xi < 0 ? -xi : xi) >> 54);
+}
+
 // One block cuts 8 rows (or 32 of a transposed source, whose rows lie side by
 // side) of one K chunk: a first read finds each row's exponent, the second,
 // from L2, writes the digits.  HBM-bound (16 bytes read, 24 written per
@@ -467,7 +531,7 @@ __device__ __forceinline__ long long round61(double v) {
 template <bool TRANS>
 __global__ void __launch_bounds__(256)
 k_i8_slice(const double2* __restrict__ x, long long ld, int sign, int rows, int K, int nslab, int spc,
-           int tile, int tiles, int8_t* __restrict__ data, int* __restrict__ exps) {
+           int tile, int tiles, int8_t* __restrict__ data, int8_t* __restrict__ mag, int* __restrict__ exps) {
     constexpr int R = TRANS ? 32 : 8;
     __shared__ unsigned int top[8][32];
     __shared__ int ex[32];
@@ -522,6 +586,16 @@ k_i8_slice(const double2* __restrict__ x, long long ld, int sign, int rows, int 
         const size_t part = (size_t)tiles * nslab * block_bytes;
         store16(xr, dst, plane_bytes);
         store16(xi, dst + part, plane_bytes);
+        if (mag) {
+            uint32_t w[4];
+#pragma unroll
+            for (int g = 0; g < 4; ++g)
+                w[g] = magnitude(xr[4 * g], xi[4 * g]) | magnitude(xr[4 * g + 1], xi[4 * g + 1]) << 8 |
+                       magnitude(xr[4 * g + 2], xi[4 * g + 2]) << 16 | magnitude(xr[4 * g + 3], xi[4 * g + 3]) << 24;
+            *reinterpret_cast<uint4*>(mag + ((size_t)(r / tile) * nslab + (kc >> 1)) * plane_bytes +
+                                      (size_t)(kc & 1) * tile * 16 + (size_t)(r % tile) * 16) =
+                make_uint4(w[0], w[1], w[2], w[3]);
+        }
 #pragma unroll
         for (int j = 0; j < 16; ++j) xr[j] += sign > 0 ? xi[j] : -xi[j];
         store16(xr, dst + 2 * part, plane_bytes);
@@ -605,13 +679,13 @@ struct CnPlan {
 
 size_t align256(size_t n) { return (n + 255) & ~(size_t)255; }
 
-size_t cn_bytes(const CnPlan& p, int M, int N, bool cached_a) {
+size_t cn_bytes(const CnPlan& p, int M, int N, bool cached_a, bool check) {
     const int K = p.slabs_per_group * kSlab;
-    return (cached_a ? 0 : i8_operand_bytes(M, kTM, K, p.spc)) + i8_operand_bytes(N, kTN, K, p.spc) +
+    return (cached_a ? 0 : i8_operand_bytes(M, kTM, K, p.spc, check)) + i8_operand_bytes(N, kTN, K, p.spc, check) +
            align256((size_t)ceil_div(p.slabs_per_group, p.spc) * M * N * sizeof(double2));
 }
 
-CnPlan cn_plan(int M, int N, int K, bool herm, int fixed_spc, size_t bytes) {
+CnPlan cn_plan(int M, int N, int K, bool herm, int fixed_spc, size_t bytes, bool check = false) {
     CnPlan p{};
     p.mt = ceil_div(M, kTM);
     p.nt = ceil_div(N, kTN);
@@ -629,7 +703,7 @@ CnPlan cn_plan(int M, int N, int K, bool herm, int fixed_spc, size_t bytes) {
         }
         const int chunks = ceil_div(p.slabs_per_group, p.spc);
         p.clk = p.groups * (launch_clk(p.tiles, chunks, p.spc) + chunks * (double)M * N * 32.0 / kHbmBytesPerClk);
-        if (cn_bytes(p, M, N, fixed_spc > 0) <= bytes) return p;
+        if (cn_bytes(p, M, N, fixed_spc > 0, check) <= bytes) return p;
         if (p.slabs_per_group <= std::max(8, fixed_spc)) break;
     }
     p.groups = 0;
@@ -646,20 +720,20 @@ Waits launch_waits() {
 }
 
 I8Side side_of(const I8Operand& op, int slab0) {
-    return {op.data, op.exps, op.tiles, op.tiles * op.tile, op.nslab, slab0, slab0 / op.spc};
+    return {op.data, op.mag, op.exps, op.tiles, op.tiles * op.tile, op.nslab, slab0, slab0 / op.spc};
 }
 
 }  // namespace
 
 void i8_inject_no_loads(long long launches) { g_no_loads_in.store(launches < 0 ? -1 : launches); }
 
-size_t i8_operand_bytes(int rows, int tile, int K, int spc) {
+size_t i8_operand_bytes(int rows, int tile, int K, int spc, bool mag) {
     const size_t tiles = ceil_div(rows, tile), nslab = ceil_div(K, kSlab);
-    return align256(3 * tiles * nslab * tile * kSlab * kDig) +
+    return align256(kParts * tiles * nslab * tile * kSlab * kDig) + (mag ? align256(tiles * nslab * tile * kSlab) : 0) +
            align256((size_t)ceil_div((int)nslab, spc) * tiles * tile * sizeof(int));
 }
 
-size_t i8_operand_place(I8Operand& op, void* buf, int rows, int tile, int K, int spc) {
+size_t i8_operand_place(I8Operand& op, void* buf, int rows, int tile, int K, int spc, bool mag) {
     op.rows = rows;
     op.tile = tile;
     op.tiles = ceil_div(rows, tile);
@@ -667,8 +741,11 @@ size_t i8_operand_place(I8Operand& op, void* buf, int rows, int tile, int K, int
     op.nslab = ceil_div(K, kSlab);
     op.spc = spc;
     op.data = (int8_t*)buf;
-    op.exps = (int*)((char*)buf + align256((size_t)3 * op.tiles * op.nslab * tile * kSlab * kDig));
-    return i8_operand_bytes(rows, tile, K, spc);
+    const size_t plane = (size_t)op.tiles * op.nslab * tile * kSlab;
+    char* at = (char*)buf + align256(kParts * plane * kDig);
+    op.mag = mag ? (int8_t*)at : nullptr;
+    op.exps = (int*)(at + (mag ? align256(plane) : 0));
+    return i8_operand_bytes(rows, tile, K, spc, mag);
 }
 
 void i8_slice(const double2* x, long long ld, bool transposed, int sign, const I8Operand& op,
@@ -678,24 +755,24 @@ void i8_slice(const double2* x, long long ld, bool transposed, int sign, const I
     const int rp = op.tiles * op.tile;
     if (transposed)
         k_i8_slice<true><<<dim3(rp / 32, op.chunks()), 256, 0, st>>>(
-            x, ld, sign, op.rows, op.K, op.nslab, op.spc, op.tile, op.tiles, op.data, op.exps);
+            x, ld, sign, op.rows, op.K, op.nslab, op.spc, op.tile, op.tiles, op.data, op.mag, op.exps);
     else
         k_i8_slice<false><<<dim3(rp / 8, op.chunks()), 256, 0, st>>>(
-            x, ld, sign, op.rows, op.K, op.nslab, op.spc, op.tile, op.tiles, op.data, op.exps);
+            x, ld, sign, op.rows, op.K, op.nslab, op.spc, op.tile, op.tiles, op.data, op.mag, op.exps);
 }
 
 int i8_cn_chunk_slabs(int M, int N, int K) {
     return best_spc(ceil_div(M, kTM) * ceil_div(N, kTN), ceil_div(K, kSlab), (double)M * N);
 }
 
-size_t i8_cn_scratch_bytes(int M, int N, int K, bool cached_a) {
+size_t i8_cn_scratch_bytes(int M, int N, int K, bool cached_a, bool check) {
     const CnPlan p = cn_plan(M, N, K, false, cached_a ? i8_cn_chunk_slabs(M, N, K) : 0, (size_t)-1);
-    return cn_bytes(p, M, N, cached_a);
+    return cn_bytes(p, M, N, cached_a, check);
 }
 
-size_t i8_tn_scratch_bytes(int M, int N, int K, bool cached_x) {
+size_t i8_tn_scratch_bytes(int M, int N, int K, bool cached_x, bool check) {
     const int spc = ceil_div(K, kSlab);
-    return i8_operand_bytes(M, kTN, K, spc) + (cached_x ? 0 : i8_operand_bytes(N, kTM, K, spc));
+    return i8_operand_bytes(M, kTN, K, spc, check) + (cached_x ? 0 : i8_operand_bytes(N, kTM, K, spc, check));
 }
 
 // The DMMA kernels: one 64 x 64 tile per SM at 264 clocks per 1 K; the INT8
@@ -728,8 +805,9 @@ bool i8_tn_pays(int M, int N, int K, bool cached_x) {
 
 bool gemm_cn_i8(const double2* A, int lda, const I8Operand* pre, const double2* B, int ldb, int M,
                 int N, int K, bool herm, void* scratch, size_t bytes, double2* out, int* err,
-                cudaStream_t st) {
-    const CnPlan p = cn_plan(M, N, K, herm, pre ? pre->spc : 0, bytes);
+                cudaStream_t st, int* unresolved) {
+    const bool check = unresolved != nullptr;  // not with digits cut before or herm
+    const CnPlan p = cn_plan(M, N, K, herm, pre ? pre->spc : 0, bytes, check);
     if (p.groups == 0 || raise_smem_limit(k_umma_i8, kSmemBytes) != cudaSuccess) return false;
     for (int g = 0; g < p.groups; ++g) {
         const int slab0 = g * p.slabs_per_group, k0 = slab0 * kSlab;
@@ -740,18 +818,18 @@ bool gemm_cn_i8(const double2* A, int lda, const I8Operand* pre, const double2* 
         if (pre) {
             oa = *pre;
         } else {
-            at += i8_operand_place(oa, at, M, kTM, kg, p.spc);
+            at += i8_operand_place(oa, at, M, kTM, kg, p.spc, check);
             i8_slice(A + k0, lda, false, -1, oa, st);
         }
-        at += i8_operand_place(ob, at, N, kTN, kg, p.spc);
+        at += i8_operand_place(ob, at, N, kTN, kg, p.spc, check);
         i8_slice(B + k0, ldb, false, 1, ob, st);
         double2* part = (double2*)at;
         const int chunks = ob.chunks(), items = p.tiles * chunks;
         const Waits w = launch_waits();
         count_launch(2);
         k_umma_i8<<<std::min(items, kSms), kThreads, kSmemBytes, st>>>(
-            side_of(oa, pre ? slab0 : 0), side_of(ob, 0), M, N, p.mt, p.tiles, items, ob.nslab, p.spc, 1,
-            herm ? 1 : 0, part, M, (long long)M * N, 1.0, 0.0, err, w.ns, w.no_loads);
+            side_of(oa, pre ? slab0 : 0), side_of(ob, 0), 0, check ? kParts + 1 : kParts, M, N, p.mt, p.tiles, items, ob.nslab, p.spc, 1,
+            herm ? 1 : 0, part, M, (long long)M * N, 1.0, 0.0, err, unresolved, nullptr, w.ns, w.no_loads);
         k_i8_reduce<<<dim3(ceil_div(M, 16), ceil_div(N, 16)), 256, 0, st>>>(part, chunks, M, N,
                                                                             herm ? 1 : 0, g > 0, out);
     }
@@ -760,15 +838,16 @@ bool gemm_cn_i8(const double2* A, int lda, const I8Operand* pre, const double2* 
 
 bool gemm_tn_i8(const double2* W, int ldw, const double2* X, int ldx, const I8Operand* pre,
                 double2* O, int ldo, int M, int N, int K, double alpha, double beta, void* scratch,
-                size_t bytes, int* err, cudaStream_t st) {
+                size_t bytes, int* err, cudaStream_t st, int* unresolved) {
     if (K > kI8MaxK || raise_smem_limit(k_umma_i8, kSmemBytes) != cudaSuccess) return false;
+    const bool check = unresolved != nullptr;  // not with digits cut before
     const int spc = ceil_div(K, kSlab), mt = ceil_div(M, kTN);
-    const size_t wb = i8_operand_bytes(M, kTN, K, spc);
+    const size_t wb = i8_operand_bytes(M, kTN, K, spc, check);
     // rows of X^T per group: what the rest of the scratch holds
     int rows = N;
     if (bytes < wb) return false;
-    if (!pre && wb + i8_operand_bytes(N, kTM, K, spc) > bytes) {
-        const size_t one = i8_operand_bytes(kTM, kTM, K, spc);
+    if (!pre && wb + i8_operand_bytes(N, kTM, K, spc, check) > bytes) {
+        const size_t one = i8_operand_bytes(kTM, kTM, K, spc, check);
         const size_t fit = (bytes - wb) / one;
         if (fit < 1) return false;
         const int groups = ceil_div(ceil_div(N, kTM), (int)std::min<size_t>(fit, 1 << 20));
@@ -776,23 +855,29 @@ bool gemm_tn_i8(const double2* W, int ldw, const double2* X, int ldx, const I8Op
     }
     I8Operand ow, ox;
     char* at = (char*)scratch;
-    at += i8_operand_place(ow, at, M, kTN, K, spc);
+    at += i8_operand_place(ow, at, M, kTN, K, spc, check);
     i8_slice(W, ldw, true, 1, ow, st);
-    for (int n0 = 0; n0 < N; n0 += rows) {
-        const int n = std::min(rows, N - n0);
-        if (pre) {
-            ox = *pre;
-        } else {
-            i8_operand_place(ox, at, n, kTM, K, spc);
-            i8_slice(X + n0, ldx, true, 1, ox, st);
+    // O += ... cannot be taken back: everything is looked at before any of it is
+    // added, and added only if `unresolved` stayed clear
+    const bool first_look = check && beta != 0.0;
+    for (int pass = first_look ? 0 : 1; pass < 2; ++pass)
+        for (int n0 = 0; n0 < N; n0 += rows) {
+            const int n = std::min(rows, N - n0);
+            if (pre) {
+                ox = *pre;
+            } else if (pass == 0 || !first_look || rows < N) {
+                i8_operand_place(ox, at, n, kTM, K, spc, check);
+                i8_slice(X + n0, ldx, true, 1, ox, st);
+            }
+            const int nt = ceil_div(n, kTM), items = nt * mt;
+            const Waits w = launch_waits();
+            count_launch();
+            k_umma_i8<<<std::min(items, kSms), kThreads, kSmemBytes, st>>>(
+                side_of(ox, 0), side_of(ow, 0), pass == 0 ? kMagPart : 0,
+                pass == 0 || (check && !first_look) ? kParts + 1 : kParts, n, M, nt, items, items, ox.nslab,
+                spc, 0, 0, O + n0, ldo, 0, alpha, beta, err, unresolved,
+                pass == 1 && first_look ? unresolved : nullptr, w.ns, w.no_loads);
         }
-        const int nt = ceil_div(n, kTM), items = nt * mt;
-        const Waits w = launch_waits();
-        count_launch();
-        k_umma_i8<<<std::min(items, kSms), kThreads, kSmemBytes, st>>>(
-            side_of(ox, 0), side_of(ow, 0), n, M, nt, items, items, ox.nslab, spc, 0, 0, O + n0, ldo, 0,
-            alpha, beta, err, w.ns, w.no_loads);
-    }
     return true;
 }
 

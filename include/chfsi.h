@@ -287,7 +287,12 @@ void         chfsi_release_scratch(void);
 /* C[m][n] = sum_k conj(A[m][k]) B[n][k] on DEVICE pointers (row-major; C is
  * m x n dense), on `stream` (cudaStream_t, 0 = legacy default).  The op::C
  * ZGEMM of BlasHandle::gemm_c64 (src/device/blas.rs:79-102) that forms
- * beta^H psi, psi^H psi and psi^H H psi.  Blocks until done. */
+ * beta^H psi, psi^H psi and psi^H H psi.  Blocks until done.
+ * Larger products run on the INT8 tensor cores with their elements cut to a fixed
+ * point of 2^-61 of their row's largest part, and are done again on the FP64
+ * tensor path where that could cost an element of C more than FP64 sums do (their
+ * bound: k 2^-53 sum |a||b|).  A row of A or B with an inf or NaN makes its row or
+ * column of C NaN. */
 chfsi_status chfsi_zgemm_cn(const chfsi_c128* a_dev, int lda, const chfsi_c128* b_dev, int ldb,
                             int m, int n, int k, chfsi_c128* c_dev, void* stream);
 /* Same product with no device allocation, for callers that cannot call

@@ -129,3 +129,64 @@ def test_rows_at_both_ends_of_the_exponents(chfsi):
     assert bool(ordinary[1, 1] and ordinary[2, 2] and ordinary[3, 3])
     err = (scaled(c, torch.where(ordinary, -e, 0)) - ref).abs() / norm
     assert float(err[ordinary].max()) < TOL
+
+
+# ---- element by element: |error| <= c K 2^-53 sum |a||b|, the bound of FP64 sums.
+# The digits alone are relative to the rows' largest parts (at most 2^-55 of their
+# product per term, 2^-59 sqrt(K) of it over random digits); products whose terms
+# are smaller than that go to the FP64 tensor path.  c = 8: the reference's sums,
+# the three-multiplication form there (3) and its own.
+def _spread(kind, rows, k, seed):
+    a = _gauss((rows, k), seed)
+    i = torch.arange(k, device="cuda", dtype=torch.float64)
+    if kind == "pairs":  # one large element that meets a small one, one ordinary
+        a[:] = 0
+        a[:, 100] = 1.0 if seed % 2 else 2.0 ** -60
+        a[:, 200] = 1.23 * 2.0 ** -40 if seed % 2 else 1.0
+    elif kind == "underflow":  # 2^-63 against 1, where the row's largest meets zero
+        a[:] = 0
+        a[:, 100] = 1.0 if seed % 2 else 0.0
+        a[:, 200] = 2.0 ** -63 if seed % 2 else 1.0
+    elif kind == "dominant":  # one element of 1, the rest near 2^-20 with full digits
+        a *= 2.0 ** -20
+        a[:, 7 if seed % 2 else 9] = 1.0
+    elif kind == "slope":  # 2^-30 from one end of the row to the other, in opposite directions
+        a *= 2.0 ** (-30.0 * (i if seed % 2 else k - 1 - i) / k)
+    elif kind == "shuffled slope":
+        a *= 2.0 ** (-30.0 * ((i * (7919 if seed % 2 else 104729)) % k) / k)
+    elif kind == "apart":  # no common support: exact zeros
+        a *= (i < k // 2) if seed % 2 else (i >= k // 2)
+    elif kind == "one row":  # a single element of the result that the digits do not hold
+        a[3] = 0
+        a[3, 100] = 1.0 if seed % 2 else 2.0 ** -50
+        a[3, 200] = 2.0 ** -50 if seed % 2 else 1.0
+    return a
+
+
+KINDS = ["pairs", "underflow", "dominant", "slope", "shuffled slope", "apart", "one row", "plain"]
+
+
+def _elementwise(c, ref, terms, k):
+    assert bool(((c - ref).abs() <= 8 * k * 2.0 ** -53 * terms).all())
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("m,n,k", [(256, 160, 20000), (130, 65, 60000)])
+def test_projection_element_by_element(chfsi, kind, m, n, k):
+    a, b = _spread(kind, m, k, 1), _spread(kind, n, k, 2)
+    c, launches = _cn(chfsi, a, b)
+    _elementwise(c, a.conj() @ b.T, a.abs() @ b.abs().T, k)
+    assert launches == (4 if kind == "plain" else launches)
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("m,n,k,alpha,beta", [(160, 20000, 512, 1.0, 0.0), (160, 20000, 512, 0.5, -2.0),
+                                              (576, 100000, 576, 1.0, 1.0)])
+def test_expansion_element_by_element(chfsi, kind, m, n, k, alpha, beta):
+    w, x = _spread(kind, m, k, 3).T.contiguous(), _spread(kind, n, k, 4).T.contiguous()
+    o0 = _gauss((m, n), 5)
+    o = o0.clone()
+    torch.cuda.synchronize()
+    chfsi.zgemm_tn(w.data_ptr(), m, x.data_ptr(), n, o.data_ptr(), n, m, n, k, alpha, beta)
+    ref = alpha * (w.T @ x) + beta * o0
+    _elementwise(o, ref, abs(alpha) * (w.abs().T @ x.abs()) + abs(beta) * o0.abs() * 4 / k, k)
