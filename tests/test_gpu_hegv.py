@@ -161,3 +161,15 @@ def test_blocks_with_a_negligible_coupling(chfsi, n, size):
     s = torch.eye(n, dtype=torch.complex128, device="cuda")
     w, v = _solve(chfsi, h, s)
     _check(h, s, w, v, 1.0)
+
+
+@pytest.mark.parametrize("n", [768, 769, 1025, 1163, 1164])
+def test_largest_sizes(chfsi, n):
+    """Past 768 rows the back transformation holds 40 entries per lane, past 1,024
+    the reduction a fifth entry per thread and the deflation over 48 KB; 1,163 is the
+    last size whose rows fit the grid's shared memory, 1,164 goes to the Jacobi."""
+    h = _gauss(n, n)
+    h = (h + h.mH) / 2
+    s = torch.eye(n, dtype=torch.complex128, device="cuda")
+    w, v = _solve(chfsi, h, s)
+    _check(h, s, w, v, 1.0)

@@ -242,3 +242,35 @@ def test_scratch_of_a_process_without_contexts(chfsi):
     assert torch.cuda.mem_get_info()[0] < free
     chfsi.release_scratch()
     assert torch.cuda.mem_get_info()[0] == free
+
+
+def test_products_in_groups_with_cut_projectors(chfsi):
+    """A projection whose second operand and partial sums are past the 1 GiB of
+    scratch runs in groups along the plane waves, against digits cut once for all
+    of them."""
+    n, radius, np_, nb = 108, 28.8, 256, 400
+    r = np.arange(-28, 29)
+    y, x, z = np.meshgrid(r, r, r, indexing="ij")
+    on = x * x + y * y + z * z <= radius * radius
+    m = np.stack([x[on], y[on], z[on]], axis=1).astype(np.int32)
+    m = np.ascontiguousarray(m[np.lexsort((m[:, 2], m[:, 0] % n, m[:, 1] % n))])
+    npw = len(m)
+    assert 7 * 64 * npw * 24 > 2 ** 30  # the digits of the bands alone
+    g = torch.Generator(device="cuda").manual_seed(1)
+    beta, psi = [torch.view_as_complex(torch.randn(rows, npw, 2, generator=g, device="cuda",
+                                                   dtype=torch.float64)) / npw ** 0.5 for rows in (np_, nb)]
+    d = torch.randn(np_, generator=g, device="cuda", dtype=torch.float64)
+    ctx = chfsi.Context(dims={"ngrid": [n] * 3, "n_pw": npw, "n_bands": nb, "n_proj": np_, "n_ions": np_})
+    ctx.set_basis(m, np.zeros(npw), 1.0)
+    ctx.set_veff(np.zeros((n, n, n)))
+    ctx.set_projectors(beta.cpu().numpy(), np.arange(np_ + 1), d.cpu().numpy().astype(complex))
+    before = chfsi.launch_count()
+    out = _apply_h(ctx, psi)
+    # cuts, products and sums of two groups, D, the expansion's two, three passes
+    assert chfsi.launch_count() - before == 2 * 3 + 1 + 2 + 3
+    c = beta.conj() @ psi.T
+    ref = (d[:, None] * c).T @ beta
+    # sums of K products of unit rows, then of np_ of them: TOL covers one each
+    bound = TOL * float(d.abs().max()) * torch.linalg.vector_norm(beta, dim=0)[None, :]
+    bound = bound * torch.linalg.vector_norm(c, dim=0)[:, None] + TOL * np_ ** 0.5 * float(d.abs().max()) * 0.1
+    assert bool(((out - ref).abs() <= bound).all())
