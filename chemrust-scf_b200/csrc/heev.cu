@@ -1304,11 +1304,10 @@ cudaError_t heev(const double2* A, int n, double* w, double2* U, double* scratch
     double* s = (double*)(((uintptr_t)scratch + 15) & ~(uintptr_t)15);
     double2* Vh = (double2*)s;
     double2* tau = Vh + nn;
-    double2* P = tau + n;
-    double2* Rw = P + 2 * n;
+    double2* P = tau + n;      // q and a of two steps in turn
     DcWork q{};
     q.n = n;
-    double2* Tg = Rw + 2 * n;  // T of each reflector group, 16 entries per 4 columns
+    double2* Tg = P + 4 * n;   // T of each reflector group, 16 entries per 4 columns
     double* at = (double*)(Tg + 4 * n + 16);
     auto take = [&](size_t k) { double* p = at; at += k; return p; };
     q.Zt[0] = take(nn);

@@ -932,14 +932,14 @@ k_zsticks_forward2(const C* __restrict__ work, const C* __restrict__ psi, int ld
 }
 
 // ------------------------------------------------------ density (pass 2')
-template <typename C, int MAXPT>
+template <int MAXPT>
 __global__ void __launch_bounds__(512)
-k_planes_density(const C* __restrict__ work, const double* __restrict__ occ, int nb, int bpg,
+k_planes_density(const double2* __restrict__ work, const double* __restrict__ occ, int nb, int bpg,
                  double scale, double* part, HGeom g) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    C* twx = reinterpret_cast<C*>(smem_raw);
-    C* twy = reinterpret_cast<C*>(smem_raw + align16<C>(g.nx));
-    C* plane = reinterpret_cast<C*>(smem_raw + align16<C>(g.nx) + align16<C>(g.ny));
+    double2* twx = reinterpret_cast<double2*>(smem_raw);
+    double2* twy = reinterpret_cast<double2*>(smem_raw + align16<double2>(g.nx));
+    double2* plane = reinterpret_cast<double2*>(smem_raw + align16<double2>(g.nx) + align16<double2>(g.ny));
     int* xl = reinterpret_cast<int*>(plane + (size_t)g.ny * g.lsx);
     const int z = blockIdx.x;
     const int b0 = blockIdx.y * bpg, b1 = min(b0 + bpg, nb);
@@ -953,9 +953,9 @@ k_planes_density(const C* __restrict__ work, const double* __restrict__ occ, int
     for (int b = b0; b < b1; ++b) {
         const double f = occ[b] * scale;
         if (f == 0.0) continue;
-        for (int i = threadIdx.x; i < g.ny * g.lsx; i += blockDim.x) plane[i] = czero<C>();
+        for (int i = threadIdx.x; i < g.ny * g.lsx; i += blockDim.x) plane[i] = czero<double2>();
         __syncthreads();
-        const C* wp = work + ((size_t)b * g.nz + z) * g.ncol;
+        const double2* wp = work + ((size_t)b * g.nz + z) * g.ncol;
         for (int c = threadIdx.x; c < g.ncol; c += blockDim.x) plane[g.col_pos[c]] = wp[c];
         __syncthreads();
         fft_lines_grouped<false>(plane, g.nxact, LinesListed{xl}, g.lsx, g.ay, twy);
@@ -965,8 +965,8 @@ k_planes_density(const C* __restrict__ work, const double* __restrict__ occ, int
             const int i = threadIdx.x + k * blockDim.x;
             if (i < npl) {
                 const int y = i / g.nx, x = i - y * g.nx;
-                const C v = plane[swz(y, g.ny) * g.lsx + swz(x, g.nx)];
-                acc[k] += f * ((double)v.x * v.x + (double)v.y * v.y);
+                const double2 v = plane[swz(y, g.ny) * g.lsx + swz(x, g.nx)];
+                acc[k] += f * (v.x * v.x + v.y * v.y);
             }
         }
         __syncthreads();
@@ -1353,10 +1353,11 @@ void planes_vloc2_launch(C* work, const double* veff, int nb, const HGeom& g, cu
         case 2: planes_vloc_x2<2, R0, R1>(work, veff, nb, g, st); return;
         default: planes_vloc_x2<0, R0, R1>(work, veff, nb, g, st); return;
         }
+    } else {
+        dim3 grid(g.nz, (nb + NB - 1) / NB);
+        raise_smem_limit(k_planes_vloc2<C, NB, R0, R1>, P::bytes);
+        k_planes_vloc2<C, NB, R0, R1><<<grid, P::threads, P::bytes, st>>>(work, veff, nb, g);
     }
-    dim3 grid(g.nz, (nb + NB - 1) / NB);
-    raise_smem_limit(k_planes_vloc2<C, NB, R0, R1>, P::bytes);
-    k_planes_vloc2<C, NB, R0, R1><<<grid, P::threads, P::bytes, st>>>(work, veff, nb, g);
 }
 
 // Square planes on a plan that is compiled in
@@ -1467,8 +1468,8 @@ void launch_planes_density(const double2* work, const double* occ, int nb, doubl
 #undef CHFSI_PD
     default: {
         const size_t sm = planes_smem_bytes(g, sizeof(double2));
-        raise_smem_limit(k_planes_density<double2, 24>, sm);
-        k_planes_density<double2, 24><<<dim3(g.nz, groups), 512, sm, st>>>(work, occ, nb, bpg, scale, part, g);
+        raise_smem_limit(k_planes_density<24>, sm);
+        k_planes_density<24><<<dim3(g.nz, groups), 512, sm, st>>>(work, occ, nb, bpg, scale, part, g);
     }
     }
     const size_t n = (size_t)g.nx * g.ny * g.nz;
