@@ -542,7 +542,7 @@ struct chfsi_ctx {
     std::vector<double> ion_pos;  // ions with projectors, x 3 (bohr)
     double2* d_phase = nullptr;   // per ion e^{-i 2 pi f_d h}: [ion][fnx | fny | fnz]
     double2* d_dmat0 = nullptr;   // unscreened D
-    size_t n_dmat = 0;            // elements of d_dmat and d_dmat0
+    size_t n_dmat = 0, n_qmat = 0;  // elements of d_dmat and d_dmat0, of d_qmat
     // counts the changes of buffers whose addresses a captured pass holds
     unsigned layout = 0;
     bool in_graph = false;        // a captured pass holds the INT8 buffers
@@ -2487,7 +2487,13 @@ chfsi_status chfsi_set_qmat(chfsi_ctx* ctx, const chfsi_c128* qmat) {
     CK(copy_sync(doff.data(), ctx->d_doff, sizeof(int) * ni, cudaMemcpyDeviceToHost, ctx->st));
     size_t dt = 0;
     for (int i = 0; i < ni; ++i) dt += (size_t)(poff[i + 1] - poff[i]) * (poff[i + 1] - poff[i]);
-    if (!ctx->d_qmat) CK(dalloc(ctx, &ctx->d_qmat, dt));
+    if (!ctx->d_qmat || ctx->n_qmat != dt) {
+        ++ctx->layout;
+        cudaFree(ctx->d_qmat);
+        ctx->d_qmat = nullptr;
+        CK(dalloc(ctx, &ctx->d_qmat, dt));
+        ctx->n_qmat = dt;
+    }
     CK(copy_sync(ctx->d_qmat, qmat, dt * sizeof(double2), cudaMemcpyHostToDevice, ctx->st));
     // B = beta^H beta on the device
     double2 *part = nullptr, *dB = nullptr;

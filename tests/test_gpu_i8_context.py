@@ -274,3 +274,30 @@ def test_products_in_groups_with_cut_projectors(chfsi):
     bound = TOL * float(d.abs().max()) * torch.linalg.vector_norm(beta, dim=0)[None, :]
     bound = bound * torch.linalg.vector_norm(c, dim=0)[:, None] + TOL * np_ ** 0.5 * float(d.abs().max()) * 0.1
     assert bool(((out - ref).abs() <= bound).all())
+
+
+def test_overlap_of_larger_blocks(chfsi):
+    """Projectors set anew with other blocks, and then q of that larger size."""
+    s = chfsi.SyntheticSystem(config_index=2, n_rep=1, ecut=8.0, ngrid=[0, 0, 0], n_bands=24)
+    off = np.zeros(s.n_ions + 1, dtype=np.int32)
+    off[1:] = np.arange(1, s.n_ions + 1)
+    off[-1] = s.n_proj  # one large block
+    rng = np.random.default_rng(8)
+    sizes = np.diff(off)
+    d = [np.diag(rng.standard_normal(k)).astype(complex) for k in sizes]
+    q = [np.diag(0.1 + 0.1 * rng.random(k)).astype(complex) for k in sizes]
+    assert sum(k * k for k in sizes) > len(s.dmat())
+    ctx = _context(chfsi, s)
+    ctx.set_projectors(s.beta(), off, np.concatenate([x.ravel() for x in d]))
+    ctx.set_qmat(np.concatenate([x.ravel() for x in q]))
+    psi = _psi(s)
+    out, local = torch.empty_like(psi), torch.empty_like(psi)
+    torch.cuda.synchronize()
+    ctx.apply_sinv_h(psi.data_ptr(), out.data_ptr(), len(psi))
+    ctx.apply_h_local(psi.data_ptr(), local.data_ptr(), len(psi))
+    beta = torch.from_numpy(s.beta()).cuda()
+    diag = [torch.from_numpy(np.concatenate([np.diag(x) for x in m])).cuda() for m in (d, q)]
+    h = local + (diag[0][:, None] * (beta.conj() @ psi.T)).T @ beta
+    back = out + (diag[1][:, None] * (beta.conj() @ out.T)).T @ beta  # S S^-1 H psi
+    # a solve with S on either side of the products: cond(S) is below 1e3 here
+    assert float((back - h).abs().max()) <= 1e3 * TOL * float(h.abs().max())
