@@ -215,13 +215,17 @@ __device__ __forceinline__ void i8_item(int item, int per_chunk, int mt, int nt,
     tm = t;
 }
 
-// parts p0 .. p1 - 1 of every item; nothing when *gate is set
+// The parts of every item, with CHECK the magnitudes behind them (their loads are
+// in flight while the third part is converted: in front of the others 1 % slower);
+// only_mag: the magnitudes alone.  Nothing when *gate is set.
+template <bool CHECK>
 __global__ void __launch_bounds__(kThreads, 1)
-k_umma_i8(I8Side a, I8Side b, int p0, int p1, int M, int N, int mt, int per_chunk, int items, int nslab, int spc,
+k_umma_i8(I8Side a, I8Side b, bool only_mag, int M, int N, int mt, int per_chunk, int items, int nslab, int spc,
           int conj, int herm, double2* __restrict__ out, long long ldo, long long chunk_stride,
           double alpha, double beta, int* err, int* unresolved, const int* gate,
           unsigned long long wait_ns, int no_loads) {
     if (gate && *gate) return;
+    const int p0 = CHECK && only_mag ? kMagPart : 0, p1 = CHECK ? kMagPart + 1 : kParts;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint64_t* full = (uint64_t*)(base + kRing * kStageBytes);
@@ -265,7 +269,7 @@ k_umma_i8(I8Side a, I8Side b, int p0, int p1, int M, int N, int mt, int per_chun
                 const int s0 = c * spc, s1 = min(nslab, s0 + spc);
                 for (int part = p0; part < p1 && ok; ++part) {
                     // magnitudes: one digit, kDig slabs to a stage
-                    const bool mag = part == kMagPart;
+                    const bool mag = CHECK && part == kMagPart;
                     const int step = mag ? kDig : 1;
                     const size_t ta = (size_t)tm * a.nslab + a.slab0 + s0, tb = (size_t)tn * b.nslab + b.slab0 + s0;
                     const int8_t* pa = mag ? a.mag + ta * (kABytes / kDig)
@@ -304,7 +308,7 @@ k_umma_i8(I8Side a, I8Side b, int p0, int p1, int M, int N, int mt, int per_chun
             int c, tm, tn;
             i8_item(item, per_chunk, mt, b.tiles, herm, c, tm, tn);
             const int n = min(nslab, (c + 1) * spc) - c * spc;
-            total += max(0, min(p1, kParts) - p0) * n + (p1 > kMagPart ? (n + kDig - 1) / kDig : 0);
+            total += (kParts - p0) * n + (CHECK ? (n + kDig - 1) / kDig : 0);
         }
         // the whole warp waits, and goes on or gives up together
         auto wait = [&](uint64_t* bar, uint32_t parity) {
@@ -319,17 +323,19 @@ k_umma_i8(I8Side a, I8Side b, int p0, int p1, int M, int N, int mt, int per_chun
             for (int part = p0; part < p1 && ok; ++part, ++pc) {
                 if (!(ok = wait(acc_free, (pc & 1) ^ 1))) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (part == kMagPart) {
+                if (CHECK && part == kMagPart) {
                     for (int s = 0; s < n && ok; s += kDig, ++it) {
                         const int slot = it % kRing;
                         const uint32_t sa = smem_u32(base + (size_t)slot * kStageBytes);
                         const uint64_t da = i8_desc(sa, kTM), db = i8_desc(sa + kABytes, kTN);
                         const int planes = min(kDig, n - s);
                         if (elect_one()) {
-                            for (int j = 0; j < planes; ++j)
-                                umma_i8<0>(tmem, da + (uint64_t)(j * (kTM * kSlab / 16)),
-                                           db + (uint64_t)(j * (kTN * kSlab / 16)), idesc_i8(kTM, kTN),
-                                           s + j > 0 ? 1u : 0u);
+#pragma unroll
+                            for (int j = 0; j < kDig; ++j)
+                                if (j < planes)
+                                    umma_i8<0>(tmem, da + (uint64_t)(j * (kTM * kSlab / 16)),
+                                               db + (uint64_t)(j * (kTN * kSlab / 16)), idesc_i8(kTM, kTN),
+                                               s + j > 0 ? 1u : 0u);
                             umma_commit(&empty[slot]);
                         }
                         if (it + 1 < total) ok = wait(&full[(it + 1) % kRing], ((it + 1) / kRing) & 1);
@@ -428,7 +434,7 @@ k_umma_i8(I8Side a, I8Side b, int p0, int p1, int M, int N, int mt, int per_chun
                 ok = __shfl_sync(0xffffffffu, ok, 0);  // tcgen05.ld is warp-collective
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (part == kMagPart) {
+                if (CHECK && part == kMagPart) {
                     // rows of zeros give exact zeros, rows with an inf or NaN give NaN
                     const bool row = i < M && ea != kZeroRow && ea != kNonFinite;
                     const unsigned colm = __ballot_sync(0xffffffffu, j0 + lane < N && eb_lane != kZeroRow &&
@@ -519,16 +525,18 @@ __device__ __forceinline__ long long round61(double v) {
            (__double_as_longlong(tl) - 0x4338000000000000LL);
 }
 
-// top 7 of the 61 bits of the larger part
+// top 7 of the 61 bits of the larger part, rounded down (the complement of a
+// negative part's high word is at most its magnitude's)
 __device__ __forceinline__ uint32_t magnitude(long long xr, long long xi) {
-    return (uint32_t)(max(xr < 0 ? -xr : xr, xi < 0 ? -xi : xi) >> 54);
+    const int r = (int)(xr >> 32), i = (int)(xi >> 32);
+    return (uint32_t)max(r ^ (r >> 31), i ^ (i >> 31)) >> 22;
 }
 
 // One block cuts 8 rows (or 32 of a transposed source, whose rows lie side by
 // side) of one K chunk: a first read finds each row's exponent, the second,
 // from L2, writes the digits.  HBM-bound (16 bytes read, 24 written per
 // complex element).
-template <bool TRANS>
+template <bool TRANS, bool MAG>
 __global__ void __launch_bounds__(256)
 k_i8_slice(const double2* __restrict__ x, long long ld, int sign, int rows, int K, int nslab, int spc,
            int tile, int tiles, int8_t* __restrict__ data, int8_t* __restrict__ mag, int* __restrict__ exps) {
@@ -586,7 +594,7 @@ k_i8_slice(const double2* __restrict__ x, long long ld, int sign, int rows, int 
         const size_t part = (size_t)tiles * nslab * block_bytes;
         store16(xr, dst, plane_bytes);
         store16(xi, dst + part, plane_bytes);
-        if (mag) {
+        if constexpr (MAG) {
             uint32_t w[4];
 #pragma unroll
             for (int g = 0; g < 4; ++g)
@@ -753,12 +761,12 @@ void i8_slice(const double2* x, long long ld, bool transposed, int sign, const I
     count_launch();
     // whole tiles are cut: the rows past the matrix as zeros
     const int rp = op.tiles * op.tile;
-    if (transposed)
-        k_i8_slice<true><<<dim3(rp / 32, op.chunks()), 256, 0, st>>>(
+    auto cut = [&](auto kernel, int rows_per_block) {
+        kernel<<<dim3(rp / rows_per_block, op.chunks()), 256, 0, st>>>(
             x, ld, sign, op.rows, op.K, op.nslab, op.spc, op.tile, op.tiles, op.data, op.mag, op.exps);
-    else
-        k_i8_slice<false><<<dim3(rp / 8, op.chunks()), 256, 0, st>>>(
-            x, ld, sign, op.rows, op.K, op.nslab, op.spc, op.tile, op.tiles, op.data, op.mag, op.exps);
+    };
+    if (transposed) cut(op.mag ? k_i8_slice<true, true> : k_i8_slice<true, false>, 32);
+    else cut(op.mag ? k_i8_slice<false, true> : k_i8_slice<false, false>, 8);
 }
 
 int i8_cn_chunk_slabs(int M, int N, int K) {
@@ -808,7 +816,8 @@ bool gemm_cn_i8(const double2* A, int lda, const I8Operand* pre, const double2* 
                 cudaStream_t st, int* unresolved) {
     const bool check = unresolved != nullptr;  // not with digits cut before or herm
     const CnPlan p = cn_plan(M, N, K, herm, pre ? pre->spc : 0, bytes, check);
-    if (p.groups == 0 || raise_smem_limit(k_umma_i8, kSmemBytes) != cudaSuccess) return false;
+    const auto umma = check ? k_umma_i8<true> : k_umma_i8<false>;
+    if (p.groups == 0 || raise_smem_limit(umma, kSmemBytes) != cudaSuccess) return false;
     for (int g = 0; g < p.groups; ++g) {
         const int slab0 = g * p.slabs_per_group, k0 = slab0 * kSlab;
         if (slab0 >= p.nslab) break;
@@ -827,8 +836,8 @@ bool gemm_cn_i8(const double2* A, int lda, const I8Operand* pre, const double2* 
         const int chunks = ob.chunks(), items = p.tiles * chunks;
         const Waits w = launch_waits();
         count_launch(2);
-        k_umma_i8<<<std::min(items, kSms), kThreads, kSmemBytes, st>>>(
-            side_of(oa, pre ? slab0 : 0), side_of(ob, 0), 0, check ? kParts + 1 : kParts, M, N, p.mt, p.tiles, items, ob.nslab, p.spc, 1,
+        umma<<<std::min(items, kSms), kThreads, kSmemBytes, st>>>(
+            side_of(oa, pre ? slab0 : 0), side_of(ob, 0), false, M, N, p.mt, p.tiles, items, ob.nslab, p.spc, 1,
             herm ? 1 : 0, part, M, (long long)M * N, 1.0, 0.0, err, unresolved, nullptr, w.ns, w.no_loads);
         k_i8_reduce<<<dim3(ceil_div(M, 16), ceil_div(N, 16)), 256, 0, st>>>(part, chunks, M, N,
                                                                             herm ? 1 : 0, g > 0, out);
@@ -839,8 +848,14 @@ bool gemm_cn_i8(const double2* A, int lda, const I8Operand* pre, const double2* 
 bool gemm_tn_i8(const double2* W, int ldw, const double2* X, int ldx, const I8Operand* pre,
                 double2* O, int ldo, int M, int N, int K, double alpha, double beta, void* scratch,
                 size_t bytes, int* err, cudaStream_t st, int* unresolved) {
-    if (K > kI8MaxK || raise_smem_limit(k_umma_i8, kSmemBytes) != cudaSuccess) return false;
     const bool check = unresolved != nullptr;  // not with digits cut before
+    // O += ... cannot be taken back: everything is looked at before any of it is
+    // added, and added only if `unresolved` stayed clear
+    const bool first_look = check && beta != 0.0;
+    if (K > kI8MaxK ||
+        (check && raise_smem_limit(k_umma_i8<true>, kSmemBytes) != cudaSuccess) ||
+        raise_smem_limit(k_umma_i8<false>, kSmemBytes) != cudaSuccess)
+        return false;
     const int spc = ceil_div(K, kSlab), mt = ceil_div(M, kTN);
     const size_t wb = i8_operand_bytes(M, kTN, K, spc, check);
     // rows of X^T per group: what the rest of the scratch holds
@@ -857,9 +872,6 @@ bool gemm_tn_i8(const double2* W, int ldw, const double2* X, int ldx, const I8Op
     char* at = (char*)scratch;
     at += i8_operand_place(ow, at, M, kTN, K, spc, check);
     i8_slice(W, ldw, true, 1, ow, st);
-    // O += ... cannot be taken back: everything is looked at before any of it is
-    // added, and added only if `unresolved` stayed clear
-    const bool first_look = check && beta != 0.0;
     for (int pass = first_look ? 0 : 1; pass < 2; ++pass)
         for (int n0 = 0; n0 < N; n0 += rows) {
             const int n = std::min(rows, N - n0);
@@ -872,11 +884,11 @@ bool gemm_tn_i8(const double2* W, int ldw, const double2* X, int ldx, const I8Op
             const int nt = ceil_div(n, kTM), items = nt * mt;
             const Waits w = launch_waits();
             count_launch();
-            k_umma_i8<<<std::min(items, kSms), kThreads, kSmemBytes, st>>>(
-                side_of(ox, 0), side_of(ow, 0), pass == 0 ? kMagPart : 0,
-                pass == 0 || (check && !first_look) ? kParts + 1 : kParts, n, M, nt, items, items, ox.nslab,
-                spc, 0, 0, O + n0, ldo, 0, alpha, beta, err, unresolved,
-                pass == 1 && first_look ? unresolved : nullptr, w.ns, w.no_loads);
+            const auto umma = check && !(first_look && pass == 1) ? k_umma_i8<true> : k_umma_i8<false>;
+            umma<<<std::min(items, kSms), kThreads, kSmemBytes, st>>>(
+                side_of(ox, 0), side_of(ow, 0), pass == 0, n, M, nt, items, items, ox.nslab, spc,
+                0, 0, O + n0, ldo, 0, alpha, beta, err, unresolved,
+                first_look && pass == 1 ? unresolved : nullptr, w.ns, w.no_loads);
         }
     return true;
 }
