@@ -30,8 +30,8 @@
 //     element by element has that looked at (`unresolved`): a fourth part
 //     multiplies the magnitudes, the top 7 bits of max(|re|, |im|), in one digit;
 //     sum |a||b| is at least that sum, so that from a quarter of 2^(EA + EB) on
-//     the error is at most K 2^-53 sum |a||b|, FP64's own bound.  Costs a
-//     twentieth of a launch.
+//     the error is at most K 2^-53 sum |a||b|, FP64's own bound.  Costs 7 %
+//     of a launch (rotation, 576 x 173,925 x 576: 4.88 -> 5.21 ms).
 //
 // Kernel (one persistent CTA per SM, work items = 128 x 64 output tile x K
 // chunk, three parts each): warp 8 copies operand blocks, warp 9 issues the
@@ -787,7 +787,9 @@ size_t i8_tn_scratch_bytes(int M, int N, int K, bool cached_x, bool check) {
 // path is taken when its clocks, cutting included, are 5 % fewer.  Measured
 // (us, INT8 / DMMA): beta^H psi 256 x 160 x 37,073 with beta cut once 213 / 426,
 // 1,728 x 576 x 173,925 both cut 17,400 / 38,800; psi V 160 x 37,073 x 160
-// 202 / 282, 576 x 173,925 x 576 5,720 / 12,770; below the line 20 x 20 x 2,945
+// 202 / 282, 576 x 173,925 x 576 5,720 / 12,770 (with the check of single elements
+// 2-5 % more: 6,550, 19,500 and 232 us a call against 6,340, 19,000 and 220 for 576 x
+// 173,925 x 576, 1,728 x 576 x 173,925 and 261 x 77 x 23,847); below the line 20 x 20 x 2,945
 // 55 / 47, 160 x 160 x 8,000 94 / 75, 20 x 37,073 x 64 65 / 39.
 // Relative error (2-norm over the result) against 64-bit sums of the same
 // inputs, INT8 / DMMA: 1,728 x 576 x 173,925 1.1e-14 / 1.5e-14, 261 x 77 x 23,847

@@ -10,9 +10,9 @@
 // steps, each ending in a barrier over the grid; the reduction to tridiagonal
 // form takes one pass of n steps with one barrier each, and what follows has
 // no chain longer than the tree's depth.  Measured (us, here / parallel Jacobi
-// with its serial Cholesky): 160 rows, nearly diagonal: eigenproblem 710 / 2,670,
-// factor and inverse 163 / 826; 576 rows, dense: 3,430 / 132,600 and 620 / 25,900;
-// 20 rows: 160 / 206 and 18 / 35.  Of the 3,430: reduction 2,420, back
+// with its serial Cholesky): 160 rows, nearly diagonal: eigenproblem 715 / 2,670,
+// factor and inverse 163 / 826; 576 rows, dense: 3,450 / 132,600 and 620 / 25,900;
+// 20 rows: 160 / 206 and 18 / 35.  Of the 3,450: reduction 2,440, back
 // transformation 380, merges 505, leaves 80.
 //
 // Divide and conquer follows Cuppen (Numer. Math. 36 (1981) 177) with the
@@ -272,11 +272,12 @@ k_chol_inv(double2* A, double2* X, int n, int* info) {
 // sigma; past it, with u_{j+1} = x_{j+1} - beta,
 //   A u = q + a u_{j+1},   w = sigma A u - (|sigma|^2 / 2) (u^H A u) u,
 //   a <- a - u w_{j+1}^* - w u_{j+1}^*
-// and the new a is the next x.  What bounds it is that chain, one barrier and one
-// reduction behind it, about 2 us a step, not the 16 n^3 / 3 flops.  CL: one
-// thread-block cluster (n <= 256): a cheaper barrier (390 clocks, the grid's
-// takes 2,300), q and a pushed into every block's shared memory instead of the
-// round trip through L2.
+// and the new a is the next x.  What bounds it is that chain, not the 16 n^3 / 3
+// flops: 2.5 us a step at 160 rows and 4.2 at 576, of which the barrier takes 0.2
+// and 1.2 and the rest is two block-wide sums read back from shared memory and the
+// sweep over the rows.  CL: one thread-block cluster (n <= 256): a cheaper barrier
+// (390 clocks, the grid's takes 2,300), q and a pushed into every block's shared
+// memory instead of the round trip through L2.
 // The rows are scaled by a power of two to a largest entry next to 1 (its top word
 // in *top, zero before the launch; the eigenvalues are scaled back at the end), and
 // columns with |x|^2 < 1e-140 then count as zero: sigma is about 1 / |x|^2, and its
@@ -1371,7 +1372,9 @@ cudaError_t heev(const double2* A, int n, double* w, double2* U, double* scratch
         k_dc_update<<<dim3((most + 63) / 64, (most + 31) / 32, 1 << l), 256, 0, st>>>(q, l, par);
     }
     k_copy_eig<<<(n + 255) / 256, 256, 0, st>>>(q.D[par], n, top, w, sweeps_out);
-    // ---- U = Q Z
+    // ---- U = Q Z.  A size takes the next rung up, with the entries past it idle; 5
+    // and 18 are those of the 64- and 216-atom cells' 160 and 576 bands, the others
+    // keep the steps between sizes below a factor of two from 96 rows on.
     k_wy<<<((n + kGrp - 1) / kGrp + 3) / 4, 128, 0, st>>>(Vh, tau, n, Tg);
     if (n <= 32) return launch_back<1>(Vh, Tg, q.Zt[par], n, U, st);
     if (n <= 96) return launch_back<3>(Vh, Tg, q.Zt[par], n, U, st);

@@ -311,6 +311,9 @@ template <int R0, int R1> struct PlaneTwo {
     // stages, without block barriers between them
     static constexpr bool own = fit >= 5;
     static constexpr int shared_warps = pick(), warps = own ? G : shared_warps, threads = 32 * warps;
+    // 96 registers: what 9 x 8 and 8 x 5 need.  Not fitted plan by plan: -Xptxas -v
+    // shows 336 bytes of spill stores for 15 x 5 and (at 80 registers) 10 x 5, 68 for
+    // 9 x 5, 28 for 10 x 8, 16 or less for the others
     static constexpr int by_regs = 65536 / (threads * 96);
     static constexpr int min_blocks = fit < by_regs ? fit : by_regs > 0 ? by_regs : 1;
     // place of x position p in a row
