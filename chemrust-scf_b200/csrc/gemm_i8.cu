@@ -31,7 +31,7 @@
 //     multiplies the magnitudes, the top 7 bits of max(|re|, |im|), in one digit;
 //     sum |a||b| is at least that sum, so that from a quarter of 2^(EA + EB) on
 //     the error is at most K 2^-53 sum |a||b|, FP64's own bound.  Costs 7 %
-//     of a launch (rotation, 576 x 173,925 x 576: 4.88 -> 5.21 ms).
+//     of a launch (rotation, 576 x 173,925 x 576: 4.89 -> 5.25 ms).
 //
 // Kernel (one persistent CTA per SM, work items = 128 x 64 output tile x K
 // chunk, three parts each): warp 8 copies operand blocks, warp 9 issues the
@@ -49,7 +49,6 @@
 
 #include <algorithm>
 #include <atomic>
-#include <type_traits>
 
 namespace chfsi {
 
@@ -66,7 +65,6 @@ constexpr int kEpiThreads = 256, kThreads = 320;
 constexpr int kMaxSpc = kI8MaxK / kSlab;
 constexpr int kNonFinite = 1 << 20;           // exponent mark of a row with inf or NaN
 constexpr int kZeroRow = -2000;               // and of one of zeros
-constexpr int kPlainExp = 900;
 
 constexpr size_t kSmemBytes = 1024 + (size_t)kRing * kStageBytes + 128;
 
@@ -164,24 +162,23 @@ __device__ __forceinline__ void tmem_ld4(uint32_t taddr, int* r) {
                  : "r"(taddr));
 }
 
-// 2^p for -1022 <= p <= 1023, inf for 1024
+// 2^p for -1022 <= p <= 1023
 __device__ __forceinline__ double pow2(int p) { return __longlong_as_double((long long)(p + 1023) << 52); }
-// 2^(E - 33) for |E| <= kPlainExp; NaN for a row with an inf or NaN, and 1 for a
-// row of zeros
-__device__ __forceinline__ double side_scale(int e) {
+// Scales of a sum v, |v| < 2^80: 2^(EA + EB - 66) v = v side.x fb side.y, in that
+// order.  A's exponent goes in two halves where it is large, so that no step leaves
+// the range of the exponents where the product does not, whatever the other row's:
+// with |a| <= 400 the second half is 1, beyond it the half still to come would have
+// to be outweighed by an EB past 2^1024 or 2^-1074.  NaN for a row with an inf or
+// NaN, 1 for a row of zeros.
+__device__ __forceinline__ double2 side_a(int e) {
+    if (e == kNonFinite) return make_double2(__longlong_as_double(0x7ff8000000000000LL), 1.0);
+    if (e == kZeroRow) return make_double2(1.0, 1.0);
+    const int a = e - 65, h = a > 400 || a < -400 ? a >> 1 : a;
+    return make_double2(pow2(h), pow2(a - h));
+}
+__device__ __forceinline__ double side_b(int e) {
     if (e == kNonFinite) return __longlong_as_double(0x7ff8000000000000LL);
-    return e == kZeroRow ? 1.0 : pow2(max(e - 33, -1022));
-}
-// rows whose scale is not multiplied on its own: it may leave the range of the
-// exponents where the product with another row's does not
-__device__ __forceinline__ bool far_row(int e) {
-    return e != kZeroRow && e != kNonFinite && (e > kPlainExp || e < -kPlainExp);
-}
-// 2^e v, |v| < 2^80, e the sum of two rows' exponents; 0 times inf, NaN, when one
-// is kNonFinite
-__device__ __forceinline__ double scale_by(double v, int e) {
-    const int h = min(max(e >> 1, -700), 1024);
-    return v * pow2(h) * pow2(min(max(e - h, -700), 1024));
+    return e == kZeroRow ? 1.0 : pow2(e - 1);
 }
 
 // x as a double, |x| < 2^51: through the exponent bits of 2^52 + 2^51, one add
@@ -383,51 +380,10 @@ k_umma_i8(I8Side a, I8Side b, bool only_mag, int M, int N, int mt, int per_chunk
             // X = x 2^(61 - E) and the digits' 256^7: products carry 2^(EA + EB - 66)
             const int ea = a.exps[(size_t)(a.chunk0 + c) * a.rows_pad + i];
             const int eb_lane = b.exps[(size_t)(b.chunk0 + c) * b.rows_pad + j0 + lane];
-            const double fa = side_scale(ea), fb_lane = side_scale(eb_lane);
-            const bool far = __any_sync(0xffffffffu, far_row(ea) || far_row(eb_lane));
+            const double2 fa = side_a(ea);
+            const double fb_lane = side_b(eb_lane);
             double2* o = out + (long long)c * chunk_stride + (long long)j0 * ldo + i;
             const int cols = i < M ? N - j0 : 0;
-            // the accumulators of one part; FAR: some row of the warp's is far_row (a
-            // loop of its own, as a branch per element keeps the compiler from
-            // interleaving them: 10 % of a launch)
-            auto convert = [&](auto is_far, int part) {
-                constexpr bool FAR = decltype(is_far)::value;
-                int I[2][kDig][4];
-#pragma unroll
-                for (int d = 0; d < kDig; ++d) tmem_ld4(tl + (uint32_t)(d * kTN), I[0][d]);
-#pragma unroll
-                for (int g = 0; g < 8; ++g) {
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    if (g < 7) {
-#pragma unroll
-                        for (int d = 0; d < kDig; ++d)
-                            tmem_ld4(tl + (uint32_t)(d * kTN + (g + 1) * 4), I[(g + 1) & 1][d]);
-                    } else {
-                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(acc_free);
-                    }
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const int jj = g * 4 + q;
-                        int v[kDig];
-#pragma unroll
-                        for (int d = 0; d < kDig; ++d) v[d] = I[g & 1][d][q];
-                        double t = i8_value(v);
-                        if constexpr (FAR) t = scale_by(t, ea + __shfl_sync(0xffffffffu, eb_lane, jj) - 66);
-                        else t = t * fa * __shfl_sync(0xffffffffu, fb_lane, jj);
-                        // conj: re = T1 + T2, im = T3 + (T2 - T1); else re = T1 - T2,
-                        // im = T3 + (-T2 - T1)
-                        const double r = fma(part == 1 ? sgn : 1.0, t, keep[jj]);
-                        keep[jj] = part == 0 ? t : fma(sgn, t, -keep[jj]);
-                        double* e = reinterpret_cast<double*>(o + (long long)jj * ldo) + (part - 1);
-                        const bool put = part > 0 && jj < cols;
-                        double old = 0.0;
-                        if (put && beta != 0.0) old = *e;
-                        if (put) *e = fma(beta, old, alpha * r);
-                    }
-                }
-            };
 #pragma unroll 1
             for (int part = p0; part < p1; ++part, ++pc) {
                 if (lane == 0) ok = mbar_wait_or(acc_full, pc & 1, wait_ns, abort_flag);
@@ -450,8 +406,41 @@ k_umma_i8(I8Side a, I8Side b, bool only_mag, int M, int N, int mt, int per_chunk
 #pragma unroll
                     for (int j = 0; j < 32; ++j) low |= L[j >> 2][j & 3] < kResolved && ((colm >> j) & 1u);
                     if (__any_sync(0xffffffffu, row && low) && lane == 0) *(volatile int*)unresolved = 1;
-                } else if (far) convert(std::true_type{}, part);
-                else convert(std::false_type{}, part);
+                    continue;
+                }
+                int I[2][kDig][4];
+#pragma unroll
+                for (int d = 0; d < kDig; ++d) tmem_ld4(tl + (uint32_t)(d * kTN), I[0][d]);
+#pragma unroll
+                for (int g = 0; g < 8; ++g) {
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (g < 7) {
+#pragma unroll
+                        for (int d = 0; d < kDig; ++d)
+                            tmem_ld4(tl + (uint32_t)(d * kTN + (g + 1) * 4), I[(g + 1) & 1][d]);
+                    } else {
+                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(acc_free);
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int jj = g * 4 + q;
+                        int v[kDig];
+#pragma unroll
+                        for (int d = 0; d < kDig; ++d) v[d] = I[g & 1][d][q];
+                        const double t = i8_value(v) * fa.x * __shfl_sync(0xffffffffu, fb_lane, jj) * fa.y;
+                        // conj: re = T1 + T2, im = T3 + (T2 - T1); else re = T1 - T2,
+                        // im = T3 + (-T2 - T1)
+                        const double r = fma(part == 1 ? sgn : 1.0, t, keep[jj]);
+                        keep[jj] = part == 0 ? t : fma(sgn, t, -keep[jj]);
+                        double* e = reinterpret_cast<double*>(o + (long long)jj * ldo) + (part - 1);
+                        const bool put = part > 0 && jj < cols;
+                        double old = 0.0;
+                        if (put && beta != 0.0) old = *e;
+                        if (put) *e = fma(beta, old, alpha * r);
+                    }
+                }
             }
         }
         if (!ok && lane == 0) {
@@ -512,7 +501,7 @@ __device__ __forceinline__ unsigned int top_word(double2 v) {
 // largest top word of a row part -> exponent E with |x| < 2^E
 __device__ __forceinline__ int row_exponent(unsigned int top) {
     const int f = (int)(top >> 20);
-    return f == 2047 ? kNonFinite : top == 0 ? kZeroRow : f - 1022;
+    return f == 2047 ? kNonFinite : top == 0 ? kZeroRow : max(f, 1) - 1022;
 }
 
 // round to nearest of v, |v| < 2^61, in two 31-bit steps on the FP64 pipe
